@@ -642,11 +642,13 @@ __global__ void to_float_kernel(const double* in, float* out, int64_t n)
 // Mapped-leaf preconditioner: gather each leaf's dense (3L x 3L) block of A'
 // and invert it by full-pivot Gauss-Jordan (inv_mat, DBEM1/lin_comp.cpp:83-183,
 // pivot = first largest |a| in row-major scan, singular if <= 1e-10).
-// One CTA per leaf; the matrix lives in shared memory.
+// One CTA per leaf; the matrix lives in shared memory.  Written besides: the
+// dense blocks themselves, both also by columns, and the largest norm of an
+// inverse.
 __global__ void __launch_bounds__(256) leaf_inverse_kernel(int n_leaves, const int32_t* leaf_begin,
                                                            const int32_t* leaf_count, const int64_t* leaf_off,
                                                            const int32_t* a_rp, const int32_t* a_col,
-                                                           const double* a_val, double* pinv, int* singular)
+                                                           const double* a_val, LeafBlocks out, int* singular)
 {
     extern __shared__ double sa[];
     __shared__ int piv_i[1], piv_j[1];
@@ -669,6 +671,10 @@ __global__ void __launch_bounds__(256) leaf_inverse_kernel(int n_leaves, const i
         }
     }
     __syncthreads();
+    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
+        out.mat[leaf_off[L] + t] = sa[t];
+        out.mat_c[leaf_off[L] + (int64_t)(t % n) * n + t / n] = sa[t];
+    }
 #define AA(i, j) sa[((i)-1) * n + ((j)-1)]
     bool bad = false;
     for (int k = 1; k <= n; ++k) {
@@ -768,7 +774,24 @@ __global__ void __launch_bounds__(256) leaf_inverse_kernel(int n_leaves, const i
         }
     }
 #undef AA
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) pinv[leaf_off[L] + t] = sa[t];
+    double norm2 = 0.0;
+    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
+        const double v = sa[t];
+        out.inv[leaf_off[L] + t] = v;
+        out.inv_c[leaf_off[L] + (int64_t)(t % n) * n + t / n] = v;
+        norm2 += v * v;
+    }
+    // the largest Frobenius norm of an inverse (non-negative doubles order like
+    // their bit patterns)
+    norm2 = ws(norm2);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) wv[threadIdx.x >> 5] = norm2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += wv[w];
+        atomicMax(reinterpret_cast<unsigned long long*>(out.norm), (unsigned long long)__double_as_longlong(sqrt(s)));
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -56,6 +56,16 @@ struct GradState {
     const int64_t* col_h;
 };
 
+// The preconditioner leaves' dense blocks and their inverses, row-major and
+// column-major (_c), and the largest Frobenius norm of an inverse.
+struct LeafBlocks {
+    double* mat;
+    double* mat_c;
+    double* inv;
+    double* inv_c;
+    double* norm;
+};
+
 cudaError_t upload_materials(const DynaMat* mats, int n, cudaStream_t s);
 cudaError_t upload_materials_dual(const DynaMatD* mats, int n, cudaStream_t s);
 
@@ -84,6 +94,6 @@ __global__ void grad_history_kernel(PairSpace ps, const QuadRules* rules, ElemGe
 __global__ void to_float_kernel(const double* in, float* out, int64_t n);
 __global__ void leaf_inverse_kernel(int n_leaves, const int32_t* leaf_begin, const int32_t* leaf_count,
                                     const int64_t* leaf_off, const int32_t* a_rp, const int32_t* a_col,
-                                    const double* a_val, double* pinv, int* singular);
+                                    const double* a_val, LeafBlocks out, int* singular);
 
 }  // namespace tdbem

@@ -344,13 +344,48 @@ void tree_split(const std::vector<double>& node, const Cube& cb, std::vector<int
 }  // namespace
 
 // ---------------------------------------------------------------------------
+// A matrix in the tile form the GMRES clusters read, on the device.
+struct GmresTiles {
+    DevBuf cta_row, cs, sp, srows, halo, send_ptr, send, col, colg, val, val32;
+    int own_rows = 0, halo_rows = 0, leaf_max = 0;  // leaf_max: values of the largest CTA's leaf inverses
+    // tiles of the matrix rp, col (host) with row-major blocks d_val9 (device)
+    cudaError_t build(const std::vector<int32_t>& rows, int64_t leaf_values, const std::vector<int32_t>& rp,
+                      const std::vector<int32_t>& mcol, const double* d_val9, bool mixed, cudaStream_t s);
+    // for Rg load cases per cluster.  TDBEM_GMRES_DSM=0 forces the kernel's
+    // global-memory form, for tuning.
+    void fill(MarchData& d, int Rg, bool mixed) const
+    {
+        d.cta_row = cta_row.as<int32_t>();
+        d.g_cs = cs.as<int32_t>();
+        d.g_sp = sp.as<int2>();
+        d.g_rows = srows.as<int32_t>();
+        d.g_halo = halo.as<int32_t>();
+        d.g_send_ptr = send_ptr.as<int32_t>();
+        d.g_send = send.as<int2>();
+        d.g_col = col.as<int32_t>();
+        d.g_colg = colg.as<int32_t>();
+        d.g_val = val.as<double>();
+        d.g_val32 = val32.as<float>();
+        const int cap = gmres_row_capacity(own_rows);
+        const char* off = std::getenv("TDBEM_GMRES_DSM");
+        const bool fits = gmres_dsm_fits(cap, halo_rows, Rg, mixed) && !(off && std::atoi(off) == 0);
+        d.own_rows = own_rows;
+        d.leaf_max = leaf_max;
+        d.dsm_rows = fits ? cap : 0;
+        d.halo_rows = fits ? halo_rows : 0;
+    }
+};
+
 // Transposed operators and scratch of the adjoint march (built by the first
 // tdbem_md_march_vjp of a handle).
 struct AdjointState {
-    DevBuf at_rp, at_col, at_val, pinvT;            // A'^T (perm space) and its leaf inverses
+    std::vector<int32_t> at_rp, at_col;             // A'^T (perm space; its leaf blocks are the row-major ones)
+    DevBuf at_val;
+    GmresTiles tiles;                               // A'^T for the GMRES cluster of cta_row
+    std::vector<int32_t> cta_row;
     DevBuf tptr, trow, tval;                        // history blocks by (type, column), then k
-    DevBuf lam, adj, g, gp;                         // adjoint right-hand sides, state adjoint, solve rhs
-    DevBuf b, bp, x, rv, u, V, W, AW, givens, status, flags, audit, xring, wring, known, out_lu, out_lt;
+    DevBuf lam, adj, gp;                            // adjoint right-hand sides, state adjoint, solve rhs
+    DevBuf x, rv, aw, u, V, givens, status, flags;
     DevBuf unk_of, perm_of_row;
     DevBuf unk_src, kt_ptr, kt_row, kt_blk;         // write-back sources per unknown; KnownM by columns
     DevBuf cot_u, cot_t, gk, contrib, flags_all;    // per-call cotangents, gradient, scratch, per-step flags
@@ -423,24 +458,26 @@ struct tdbem_handle {
     bool saved_forward = false;  // the last march was tdbem_md_march_forward (states kept)
     bool diag_ready = false;     // the last march was a recorded host march (rhs diagnostics)
     int cluster = 1;
-    int dsm_rows = 0;   // GMRES Krylov copies in shared memory for owned ranges of this many rows (0: off)
+    std::vector<int32_t> cta_row;  // perm rows of each GMRES CTA
+    int64_t leaf_values = 0;       // values of the largest CTA's leaf inverses
     int groups = 1;
     int rhs_cpt = 0;              // history pass: load cases per thread (0 = the default for R)
-    std::vector<int32_t> ap_col;  // A' columns (perm space), for re-laying the GMRES clusters
+    std::vector<int32_t> ap_rp, ap_col;  // A' structure (perm space), for re-laying the GMRES clusters
     // device buffers
     DevBuf d_rules, d_secpw_pos, d_secpw_val, d_points, d_elements;
     DevBuf g_cc, g_center, g_radius, g_rpw, g_rcen, g_node, g_trans, g_u1, g_t1, g_t2, g_bcid, g_domain, g_surface;
     DevBuf d_uref_sign, d_tref_sign, d_hu_sign, d_ht_sign, d_itf_trans, d_uref_block, d_tref_block, d_hist_block;
-    DevBuf d_uref_known, d_tref_known, d_hist_owner, d_known_elem, d_known_sign, d_itf_pairs, d_itf_sign;
+    DevBuf d_uref_known, d_tref_known, d_hist_owner, d_known_elem, d_known_sign, d_itf_a, d_itf_asign;
     DevBuf d_h_kptr, d_h_col, d_h_val, d_h_val32;
     DevBuf d_r_ptr, d_r_meta, d_r_off, d_r_val;  // run layout of steps k >= run_k (T-step history pass)
     int64_t r_nb = 0, r_runs = 0;
     int run_k = 0;
     DevBuf d_k_rp, d_k_col, d_k_val, d_k_elem, d_k_sgn;
-    DevBuf d_a_rp, d_a_col, d_a_val, d_a_val32, d_row_of, d_unk_of, d_perm_of_unk;
-    DevBuf d_leaf_begin, d_leaf_count, d_leaf_of_perm, d_leaf_off, d_pinv, d_pinv32, d_cta_leaf, d_a_colx;
-    DevBuf d_xring, d_wring, d_bulk, d_b, d_bp, d_x, d_rv, d_u, d_V, d_W, d_AW, d_givens, d_status,
-        d_flags, d_audit;
+    DevBuf d_a_rp, d_a_col, d_a_val, d_row_of, d_unk_of, d_perm_of_unk;
+    DevBuf d_leaf_begin, d_leaf_count, d_leaf_off, d_row_leaf;
+    DevBuf d_pmat, d_pmat_c, d_pinv, d_pinv_c, d_pinv32, d_minv;  // leaf blocks and inverses (LeafBlocks)
+    GmresTiles tiles;                                             // A' for the GMRES clusters
+    DevBuf d_xring, d_wring, d_bulk, d_b, d_x, d_rv, d_aw, d_u, d_V, d_givens, d_status, d_flags, d_audit;
     DevBuf d_known, d_out_lu, d_out_lt, d_rec_rhs, d_rec_x, d_xold;
     std::unique_ptr<AdjointState> adjoint;
 
@@ -695,15 +732,14 @@ tdbem_status tdbem_md_create(const tdbem_problem* pr, int32_t device, tdbem_hand
                 h->itf_trans[9 * bb + si * 3 + r] = dot;
             }
     }
-    std::vector<int32_t> pairs;
-    std::vector<double> isign;
+    std::vector<int32_t> itf_a((size_t)E, -1);
+    std::vector<double> isign((size_t)E, 0.0);
     for (int64_t k = 0; k < h->I; ++k) {
-        pairs.push_back((int32_t)h->itf[5 * k + 1]);
-        pairs.push_back((int32_t)h->itf[5 * k + 3]);
-        isign.push_back((double)h->itf[5 * k + 4]);
+        itf_a[h->itf[5 * k + 3]] = (int32_t)h->itf[5 * k + 1];
+        isign[h->itf[5 * k + 3]] = (double)h->itf[5 * k + 4];
     }
-    CUDA_TRY(up(h->d_itf_pairs, pairs, s));
-    CUDA_TRY(up(h->d_itf_sign, isign, s));
+    CUDA_TRY(up(h->d_itf_a, itf_a, s));
+    CUDA_TRY(up(h->d_itf_asign, isign, s));
     CUDA_TRY(up(h->d_uref_sign, h->uref_sign, s));
     CUDA_TRY(up(h->d_tref_sign, h->tref_sign, s));
     CUDA_TRY(up(h->d_hu_sign, h->hu_sign, s));
@@ -914,12 +950,45 @@ tdbem_status history_step_bound(tdbem_handle* h, cudaStream_t s, int& kb)
     return TDBEM_OK;
 }
 
+}  // namespace
+
+cudaError_t GmresTiles::build(const std::vector<int32_t>& rows, int64_t leaf_values, const std::vector<int32_t>& rp,
+                              const std::vector<int32_t>& mcol, const double* d_val9, bool mixed, cudaStream_t s)
+{
+    GmresTileIndex ix;
+    own_rows = 0;
+    leaf_max = (int)std::min<int64_t>(leaf_values, 1 << 24);
+    for (size_t c = 0; c + 1 < rows.size(); ++c) own_rows = std::max(own_rows, rows[c + 1] - rows[c]);
+    gmres_tile_index(rows, gmres_row_capacity(own_rows), rp, mcol, ix);
+    halo_rows = ix.halo_max;
+    DevBuf src;
+    cudaError_t e = up(cta_row, rows, s);
+    if (e == cudaSuccess) e = up(cs, ix.cs, s);
+    if (e == cudaSuccess) e = up(sp, ix.sp, s);
+    if (e == cudaSuccess) e = up(srows, ix.rows, s);
+    if (e == cudaSuccess) e = up(halo, ix.halo, s);
+    if (e == cudaSuccess) e = up(send_ptr, ix.send_ptr, s);
+    if (e == cudaSuccess) e = up(send, ix.send, s);
+    if (e == cudaSuccess) e = up(col, ix.col, s);
+    if (e == cudaSuccess) e = up(colg, ix.colg, s);
+    if (e == cudaSuccess) e = up(src, ix.src, s);
+    const int64_t tiles = (int64_t)(ix.col.size() / 32);
+    if (e == cudaSuccess) e = val.alloc(sizeof(double) * 288 * (size_t)std::max<int64_t>(tiles, 1));
+    if (e == cudaSuccess && mixed) e = val32.alloc(sizeof(float) * 288 * (size_t)std::max<int64_t>(tiles, 1));
+    if (e == cudaSuccess)
+        e = gather_tiles(tiles, src.as<int32_t>(), d_val9, val.as<double>(), mixed ? val32.as<float>() : nullptr, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // src is freed here
+    return e;
+}
+
+namespace {
+
 // Permuted system matrix A', leaf inverses, GMRES partition and march state.
 // GMRES launch layout: G clusters (load-case groups) of C CTAs; within a
 // cluster every CTA owns a contiguous range of leaves of about equal point
-// count, and the A' columns are tagged with their owner CTA and row within
-// it so the products read Krylov vectors from the owners' shared memory
-// when the per-CTA copies fit.
+// count, and A' is laid out in tiles whose columns are tagged with their owner
+// CTA and row within it, so the products read Krylov vectors from the owners'
+// shared memory when they fit there.
 tdbem_status gmres_layout(tdbem_handle* h, int G, int C, cudaStream_t s)
 {
     const int64_t E = h->E;
@@ -940,30 +1009,20 @@ tdbem_status gmres_layout(tdbem_handle* h, int G, int C, cudaStream_t s)
         cta[C] = nl;
     }
     h->cluster = C;
-    CUDA_TRY(up(h->d_cta_leaf, cta, s));
-    {
-        std::vector<int32_t> owner((size_t)E, 0), local((size_t)E, 0);
-        int rows_max = 0;
-        for (int c = 0; c < C; ++c) {
-            if (cta[c] >= cta[c + 1]) continue;
-            const int lo = (int)h->leaf_begin[cta[c]];
-            const int hi = (int)(h->leaf_begin[cta[c + 1] - 1] + h->leaf_count[cta[c + 1] - 1]);
-            rows_max = std::max(rows_max, hi - lo);
-            for (int p = lo; p < hi; ++p) {
-                owner[p] = c;
-                local[p] = p - lo;
-            }
-        }
-        std::vector<int32_t> colx(h->ap_col.size());
-        for (size_t j = 0; j < h->ap_col.size(); ++j) colx[j] = (owner[h->ap_col[j]] << 24) | local[h->ap_col[j]];
-        CUDA_TRY(up(h->d_a_colx, colx, s));
-        h->dsm_rows = gmres_dsm_bytes(rows_max, R / G, h->precision == TDBEM_PRECISION_MIXED) <= kGmresDsmMax
-                          ? rows_max
-                          : 0;
-        if (const char* off = std::getenv("TDBEM_GMRES_DSM"))
-            if (std::atoi(off) == 0) h->dsm_rows = 0;  // tuning override: vectors from global memory
+    // a CTA without leaves (fewer leaves than the rounding above leaves) owns
+    // an empty range
+    h->cta_row.assign((size_t)C + 1, (int32_t)E);
+    for (int c = C - 1; c >= 0; --c)
+        h->cta_row[c] = cta[c] < cta[c + 1] ? (int32_t)h->leaf_begin[cta[c]] : h->cta_row[c + 1];
+    h->leaf_values = 0;
+    for (int c = 0; c < C; ++c) {
+        int64_t v = 0;
+        for (int L = cta[c]; L < cta[c + 1]; ++L) v += 9 * h->leaf_count[L] * h->leaf_count[L];
+        h->leaf_values = std::max(h->leaf_values, v);
     }
-    CUDA_TRY(h->d_givens.alloc(sizeof(double) * (size_t)C * R * kGivensArrays * (h->restart + 2)));
+    CUDA_TRY(h->tiles.build(h->cta_row, h->leaf_values, h->ap_rp, h->ap_col, h->d_a_val.as<double>(),
+                            h->precision == TDBEM_PRECISION_MIXED, s));
+    CUDA_TRY(h->d_givens.alloc(sizeof(double) * (size_t)C * R * gmres_givens_doubles(h->restart)));
     return TDBEM_OK;
 }
 
@@ -988,6 +1047,7 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     }
     CUDA_TRY(up(h->d_a_rp, arp, s));
     CUDA_TRY(up(h->d_a_col, acol, s));
+    h->ap_rp = arp;
     h->ap_col = acol;
     CUDA_TRY(up(h->d_a_val, aval, s));
     CUDA_TRY(up(h->d_row_of, row_of, s));
@@ -1005,12 +1065,15 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     }
     CUDA_TRY(up(h->d_leaf_begin, lb, s));
     CUDA_TRY(up(h->d_leaf_count, lc, s));
-    std::vector<int32_t> lop(E, 0);
+    std::vector<RowLeaf> lop((size_t)E);
     for (int l = 0; l < nl; ++l)
-        for (int q = 0; q < lc[l]; ++q) lop[lb[l] + q] = l;
-    CUDA_TRY(up(h->d_leaf_of_perm, lop, s));
+        for (int q = 0; q < lc[l]; ++q) lop[lb[l] + q] = RowLeaf{loff[l], lb[l], 3 * lc[l]};
+    CUDA_TRY(up(h->d_row_leaf, lop, s));
     CUDA_TRY(up(h->d_leaf_off, loff, s));
-    CUDA_TRY(h->d_pinv.alloc(sizeof(double) * std::max<int64_t>(loff[nl], 1)));
+    for (DevBuf* b : {&h->d_pmat, &h->d_pmat_c, &h->d_pinv, &h->d_pinv_c})
+        CUDA_TRY(b->alloc(sizeof(double) * std::max<int64_t>(loff[nl], 1)));
+    CUDA_TRY(h->d_minv.alloc(sizeof(double)));
+    CUDA_TRY(cudaMemsetAsync(h->d_minv.p, 0, sizeof(double), s));
     DevBuf sing;
     CUDA_TRY(sing.alloc(sizeof(int)));
     CUDA_TRY(cudaMemsetAsync(sing.p, 0, sizeof(int), s));
@@ -1020,7 +1083,10 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     leaf_inverse_kernel<<<nl, 256, smem, s>>>(nl, h->d_leaf_begin.as<int32_t>(), h->d_leaf_count.as<int32_t>(),
                                              h->d_leaf_off.as<int64_t>(), h->d_a_rp.as<int32_t>(),
                                              h->d_a_col.as<int32_t>(), h->d_a_val.as<double>(),
-                                             h->d_pinv.as<double>(), sing.as<int>());
+                                             LeafBlocks{h->d_pmat.as<double>(), h->d_pmat_c.as<double>(),
+                                                        h->d_pinv.as<double>(), h->d_pinv_c.as<double>(),
+                                                        h->d_minv.as<double>()},
+                                             sing.as<int>());
     CUDA_TRY(cudaGetLastError());
     int singular = 0;
     CUDA_TRY(cudaMemcpyAsync(&singular, sing.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1030,9 +1096,7 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
                                               " has a pivot <= 1e-10");
     if (h->precision == TDBEM_PRECISION_MIXED) {
         CUDA_TRY(h->d_pinv32.alloc(sizeof(float) * std::max<int64_t>(loff[nl], 1)));
-        to_float_kernel<<<148, 256, 0, s>>>(h->d_pinv.as<double>(), h->d_pinv32.as<float>(), loff[nl]);
-        CUDA_TRY(h->d_a_val32.alloc(sizeof(float) * std::max<size_t>(aval.size(), 1)));
-        to_float_kernel<<<148, 256, 0, s>>>(h->d_a_val.as<double>(), h->d_a_val32.as<float>(), (int64_t)aval.size());
+        to_float_kernel<<<148, 256, 0, s>>>(h->d_pinv_c.as<double>(), h->d_pinv32.as<float>(), loff[nl]);
         CUDA_TRY(cudaGetLastError());
     }
     // GMRES: `groups` clusters of C CTAs, each solving R / groups load cases;
@@ -1081,13 +1145,11 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     const int rs = h->restart;
     const size_t vec = sizeof(double) * 3 * (size_t)E * R;
     CUDA_TRY(h->d_V.alloc(vec * (rs + 1)));
-    CUDA_TRY(h->d_W.alloc(vec * (rs + 1)));
-    CUDA_TRY(h->d_AW.alloc(vec * (rs + 1)));
     CUDA_TRY(h->d_b.alloc(vec));
-    CUDA_TRY(h->d_bp.alloc(vec));
     CUDA_TRY(h->d_x.alloc(vec));
     if (h->precision == TDBEM_PRECISION_MIXED) CUDA_TRY(h->d_xold.alloc(vec));
     CUDA_TRY(h->d_rv.alloc(vec));
+    CUDA_TRY(h->d_aw.alloc(vec));
     CUDA_TRY(h->d_u.alloc(vec));
     CUDA_TRY(h->d_bulk.alloc(8 * vec));
     CUDA_TRY(h->d_status.alloc(sizeof(int) * 4));
@@ -1236,21 +1298,14 @@ struct MarchRun {
         d.k_sgn = h->d_k_sgn.as<double>();
         d.known_elem = h->d_known_elem.as<int32_t>();
         d.known_sign = h->d_known_sign.as<double>();
-        d.a_rp = h->d_a_rp.as<int32_t>();
-        d.a_col = h->d_a_col.as<int32_t>();
-        d.a_val = h->d_a_val.as<double>();
-        d.a_val32 = h->d_a_val32.as<float>();
+        h->tiles.fill(d, R / h->groups, d.mixed != 0);
         d.row_of = h->d_row_of.as<int32_t>();
         d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
-        d.leaf_begin = h->d_leaf_begin.as<int32_t>();
-        d.leaf_count = h->d_leaf_count.as<int32_t>();
-        d.leaf_of_perm = h->d_leaf_of_perm.as<int32_t>();
-        d.leaf_off = h->d_leaf_off.as<int64_t>();
-        d.pinv = h->d_pinv.as<double>();
+        d.row_leaf = h->d_row_leaf.as<RowLeaf>();
+        d.pinv = h->d_pinv_c.as<double>();
         d.pinv32 = h->d_pinv32.as<float>();
-        d.cta_leaf = h->d_cta_leaf.as<int32_t>();
-        d.a_colx = h->d_a_colx.as<int32_t>();
-        d.dsm_rows = h->dsm_rows;
+        d.pmat = h->d_pmat_c.as<double>();
+        d.minv = h->d_minv.as<double>();
         d.uref_block = h->d_uref_block.as<int64_t>();
         d.uref_sign = h->d_uref_sign.as<double>();
         d.uref_known = h->d_uref_known.as<int32_t>();
@@ -1264,22 +1319,19 @@ struct MarchRun {
         d.itf_trans = h->d_itf_trans.as<double>();
         d.trans = h->g_trans.as<double>();
         d.bcid = h->g_bcid.as<int32_t>();
-        d.itf_pairs = h->d_itf_pairs.as<int32_t>();
-        d.itf_sign = h->d_itf_sign.as<double>();
-        d.n_itf = (int)h->I;
+        d.itf_a = h->d_itf_a.as<int32_t>();
+        d.itf_asign = h->d_itf_asign.as<double>();
         d.xring = h->d_xring.as<double>();
         d.wring = h->d_wring.as<double>();
         d.bulk = h->d_bulk.as<double>();
         d.b = h->d_b.as<double>();
         d.groups = h->groups;
-        d.bp = h->d_bp.as<double>();
         d.x = h->d_x.as<double>();
         d.xold = h->d_xold.as<double>();
         d.rv = h->d_rv.as<double>();
+        d.aw = h->d_aw.as<double>();
         d.u = h->d_u.as<double>();
         d.V = h->d_V.as<double>();
-        d.W = h->d_W.as<double>();
-        d.AW = h->d_AW.as<double>();
         d.givens = h->d_givens.as<double>();
         d.status = h->d_status.as<int>();
         d.step_flags = h->d_flags.as<int>();
@@ -1293,7 +1345,7 @@ struct MarchRun {
         d.tol = h->tol;
         d.cluster = h->cluster;
         d.rhs_cpt = h->rhs_cpt;
-        d.givens_stride = (int64_t)kGivensArrays * (h->restart + 2);
+        d.givens_stride = gmres_givens_doubles(h->restart);
 
         overlap = h->K >= 3;
         if (const char* v = std::getenv("TDBEM_OVERLAP")) serial_history = std::atoi(v) == 0;
@@ -1734,12 +1786,16 @@ tdbem_status tdbem_md_march_many(tdbem_handle* const* handles, int32_t n, const 
         std::vector<int32_t> row_off((size_t)n + 1, 0);
         size_t dsm = 0;
         int max_K = 0;
+        bool local = true;  // one form of the kernel for all models
+        for (int i = 0; i < n; ++i) local = local && runs[i].d.dsm_rows > 0;
         for (int i = 0; i < n; ++i) {
             ds[i] = runs[i].d;
+            if (!local) ds[i].dsm_rows = ds[i].halo_rows = 0;
             ds[i].k_lo = 1;
             ds[i].k_hi = 0;
             row_off[i + 1] = row_off[i] + runs[i].d.E;
-            dsm = std::max(dsm, gmres_dsm_bytes(runs[i].d.dsm_rows, h0->R, h0->precision == TDBEM_PRECISION_MIXED));
+            dsm = std::max(dsm, gmres_dsm_bytes(ds[i].dsm_rows, ds[i].halo_rows, h0->R,
+                                                h0->precision == TDBEM_PRECISION_MIXED));
             max_K = std::max(max_K, runs[i].d.K);
         }
         DevBuf d_ds, d_off;
@@ -1764,7 +1820,7 @@ tdbem_status tdbem_md_march_many(tdbem_handle* const* handles, int32_t n, const 
         tdbem_status st = TDBEM_OK;
         auto launch = [&](int step, int phase, cudaStream_t on) {
             const cudaError_t e = march_models_step(d_ds.as<MarchData>(), d_off.as<int32_t>(), n, row_off[n], h0->R,
-                                                    mixed, gC, dsm, max_K, step, phase, on);
+                                                    mixed, gC, dsm, local, max_K, step, phase, on);
             if (e != cudaSuccess && st == TDBEM_OK)
                 st = fail(TDBEM_CUDA_ERROR, std::string("grouped march: ") + cudaGetErrorString(e));
         };
@@ -2049,10 +2105,12 @@ tdbem_status tdbem_md_precond_layout(tdbem_handle* h, int64_t* repid, int64_t* l
 // and (optionally) a copy of three flags.
 namespace {
 
-// Capacity of the static scratch.  One solve needs, in doubles,
+// Capacity of the static scratch, and what a solve is charged for, in doubles:
 //   (15 + 9 (restart + 1)) E + 5 C (restart + 2) + 32
 // plus 256-byte alignment of each region (C = GMRES cluster CTAs): at
-// restart 30 about 2.35 KB per element, so roughly 14,000 elements.
+// restart 30 about 2.35 KB per element, so roughly 14,000 elements.  The
+// solve uses less: its basis, 3 (restart + 1) E, and at most 16 x 115,921
+// doubles of small arrays (restart 480), which fit whenever the charge does.
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -2070,7 +2128,8 @@ std::mutex g_noalloc_mutex;
 // solve_only set, so the march's write-back targets (boundary values,
 // history states, audit) need no storage here.
 struct NoAllocLayout {
-    size_t head = 0, b = 0, bp = 0, x = 0, rv = 0, u = 0, V = 0, W = 0, AW = 0, givens = 0, zero_bytes = 0, total = 0;
+    size_t head = 0, b = 0, x = 0, rv = 0, aw = 0, u = 0, V = 0, givens = 0, zero_bytes = 0;
+    size_t used = 0, charge = 0;
 };
 
 NoAllocLayout noalloc_layout(int64_t E, int rs, int C)
@@ -2086,15 +2145,18 @@ NoAllocLayout noalloc_layout(int64_t E, int rs, int C)
     L.head = take(32);
     L.zero_bytes = at;
     L.b = take(e3);
-    L.bp = take(e3);
     L.x = take(e3);
     L.rv = take(e3);
+    L.aw = take(e3);
     L.u = take(e3);
     L.V = take((size_t)(rs + 1) * e3);
-    L.W = take((size_t)(rs + 1) * e3);
-    L.AW = take((size_t)(rs + 1) * e3);
-    L.givens = take((size_t)C * kGivensArrays * (rs + 2));
-    L.total = at;
+    L.givens = take((size_t)C * gmres_givens_doubles(rs));
+    L.used = at;
+    at = L.zero_bytes;
+    for (int i = 0; i < 5; ++i) take(e3);
+    for (int i = 0; i < 3; ++i) take((size_t)(rs + 1) * e3);
+    take((size_t)C * 5 * (rs + 2));
+    L.charge = at;
     return L;
 }
 
@@ -2153,8 +2215,8 @@ tdbem_status tdbem_md_solve_noalloc(tdbem_handle* h, const double* d_rhs, double
                                              " CTAs exceeds the " + std::to_string(nd->max_cluster) +
                                              " the single-load solver can be scheduled with");
     const NoAllocLayout L = noalloc_layout(E, rs, C);
-    if (L.total > kNoAllocScratchBytes)
-        return fail(TDBEM_INVALID_INPUT, "tdbem_md_solve_noalloc needs " + std::to_string(L.total) +
+    if (std::max(L.charge, L.used) > kNoAllocScratchBytes)
+        return fail(TDBEM_INVALID_INPUT, "tdbem_md_solve_noalloc needs " + std::to_string(std::max(L.charge, L.used)) +
                                              " bytes of scratch for " + std::to_string(E) +
                                              " elements at restart " + std::to_string(rs) +
                                              "; its static scratch holds " +
@@ -2169,52 +2231,28 @@ tdbem_status tdbem_md_solve_noalloc(tdbem_handle* h, const double* d_rhs, double
     d.nstep = 1;
     d.SW = 1;
     d.mixed = 0;
-    d.a_rp = h->d_a_rp.as<int32_t>();
-    d.a_col = h->d_a_col.as<int32_t>();
-    d.a_val = h->d_a_val.as<double>();
+    h->tiles.fill(d, 1, false);
     d.row_of = h->d_row_of.as<int32_t>();
     d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
-    d.leaf_begin = h->d_leaf_begin.as<int32_t>();
-    d.leaf_count = h->d_leaf_count.as<int32_t>();
-    d.leaf_of_perm = h->d_leaf_of_perm.as<int32_t>();
-    d.leaf_off = h->d_leaf_off.as<int64_t>();
-    d.pinv = h->d_pinv.as<double>();
-    d.cta_leaf = h->d_cta_leaf.as<int32_t>();
-    d.a_colx = h->d_a_colx.as<int32_t>();
-    d.dsm_rows = h->dsm_rows;
-    d.uref_block = h->d_uref_block.as<int64_t>();
-    d.uref_sign = h->d_uref_sign.as<double>();
-    d.uref_known = h->d_uref_known.as<int32_t>();
-    d.tref_block = h->d_tref_block.as<int64_t>();
-    d.tref_sign = h->d_tref_sign.as<double>();
-    d.tref_known = h->d_tref_known.as<int32_t>();
-    d.hist_block = h->d_hist_block.as<int64_t>();
-    d.hu_sign = h->d_hu_sign.as<double>();
-    d.ht_sign = h->d_ht_sign.as<double>();
-    d.hist_owner = h->d_hist_owner.as<int32_t>();
-    d.itf_trans = h->d_itf_trans.as<double>();
-    d.trans = h->g_trans.as<double>();
-    d.bcid = h->g_bcid.as<int32_t>();
-    d.itf_pairs = h->d_itf_pairs.as<int32_t>();
-    d.itf_sign = h->d_itf_sign.as<double>();
-    d.n_itf = (int)h->I;
+    d.row_leaf = h->d_row_leaf.as<RowLeaf>();
+    d.pinv = h->d_pinv_c.as<double>();
+    d.pmat = h->d_pmat_c.as<double>();
+    d.minv = h->d_minv.as<double>();
     d.status = reinterpret_cast<int*>(base + L.head);
     d.step_flags = reinterpret_cast<int*>(base + L.head + 16);
     d.solve_only = 1;
     d.b = dbl(L.b);
     d.groups = 1;
-    d.bp = dbl(L.bp);
     d.x = dbl(L.x);
     d.rv = dbl(L.rv);
+    d.aw = dbl(L.aw);
     d.u = dbl(L.u);
     d.V = dbl(L.V);
-    d.W = dbl(L.W);
-    d.AW = dbl(L.AW);
     d.givens = dbl(L.givens);
     d.restart = rs;
     d.tol = h->tol;
     d.cluster = C;
-    d.givens_stride = (int64_t)kGivensArrays * (rs + 2);
+    d.givens_stride = gmres_givens_doubles(rs);
     const int grid = (int)std::min<int64_t>(ceil_div(3 * E, 256), 4 * 148);
     CUDA_TRY(cudaMemsetAsync(base, 0, L.zero_bytes, s));
     noalloc_rows_to_perm<<<grid, 256, 0, s>>>((int)E, d.row_of, d_rhs, d.b);
@@ -2769,25 +2807,10 @@ tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
         }
         rp[q + 1] = (int32_t)col.size();
     }
-    CUDA_TRY(up(A->at_rp, rp, s));
-    CUDA_TRY(up(A->at_col, col, s));
     CUDA_TRY(up(A->at_val, val, s));
-    // transposed leaf inverses
-    const int nl = (int)h->leaf_begin.size();
-    int64_t total = 0;
-    for (int l = 0; l < nl; ++l) total += 9 * h->leaf_count[l] * h->leaf_count[l];
-    std::vector<double> pinv;
-    CUDA_TRY(download(pinv, h->d_pinv, (size_t)total, s));
     CUDA_TRY(cudaStreamSynchronize(s));
-    std::vector<double> pinvT(pinv.size());
-    int64_t off = 0;
-    for (int l = 0; l < nl; ++l) {
-        const int64_t n3 = 3 * h->leaf_count[l];
-        for (int64_t i = 0; i < n3; ++i)
-            for (int64_t j = 0; j < n3; ++j) pinvT[off + i * n3 + j] = pinv[off + j * n3 + i];
-        off += n3 * n3;
-    }
-    CUDA_TRY(up(A->pinvT, pinvT, s));
+    A->at_rp = std::move(rp);
+    A->at_col = std::move(col);
     // history blocks by (type, column) and k, regrouped on the device
     const int64_t hn = std::max<int64_t>(h->h_nnz, 1);
     CUDA_TRY(A->tptr.alloc(sizeof(int64_t) * 2 * (size_t)nh * (K + 1)));
@@ -2837,16 +2860,11 @@ tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
     // GMRES storage for one load case
     const size_t vec = sizeof(double) * 3 * (size_t)E;
     const int rs = h->restart;
-    for (DevBuf* b : {&A->b, &A->bp, &A->x, &A->rv, &A->u, &A->g, &A->gp}) CUDA_TRY(b->alloc(vec));
-    for (DevBuf* b : {&A->V, &A->W, &A->AW}) CUDA_TRY(b->alloc(vec * (rs + 1)));
-    CUDA_TRY(A->givens.alloc(sizeof(double) * (size_t)h->cluster * kGivensArrays * (rs + 2)));
+    for (DevBuf* b : {&A->x, &A->rv, &A->aw, &A->u, &A->gp}) CUDA_TRY(b->alloc(vec));
+    CUDA_TRY(A->V.alloc(vec * (rs + 1)));
+    CUDA_TRY(A->givens.alloc(sizeof(double) * (size_t)kGmresClusterMax * gmres_givens_doubles(rs)));
     CUDA_TRY(A->status.alloc(sizeof(int) * 4));
     CUDA_TRY(A->flags.alloc(sizeof(int) * 4));
-    CUDA_TRY(A->audit.alloc(sizeof(double) * 2));
-    CUDA_TRY(A->xring.alloc(sizeof(double) * 18 * nh));
-    CUDA_TRY(A->wring.alloc(sizeof(double) * 6 * nh));
-    for (DevBuf* b : {&A->known, &A->out_lu, &A->out_lt}) CUDA_TRY(b->alloc(2 * vec));
-    CUDA_TRY(cudaMemsetAsync(A->known.p, 0, 2 * vec, s));
     CUDA_TRY(A->lam.alloc(sizeof(double) * 3 * (size_t)E * (h->nstep + 2)));
     CUDA_TRY(A->adj.alloc(sizeof(double) * 6 * (size_t)nh));
     CUDA_TRY(cudaStreamSynchronize(s));
@@ -2881,56 +2899,33 @@ tdbem_status tdbem_md_march_vjp(tdbem_handle* h, const double* cot_lu, const dou
     d.R = 1;
     d.nstep = 1;
     d.SW = 1;
-    d.a_rp = A.at_rp.as<int32_t>();
-    d.a_col = A.at_col.as<int32_t>();
-    d.a_val = A.at_val.as<double>();
-    d.pinv = A.pinvT.as<double>();
+    if (A.cta_row != h->cta_row) {  // first call, or another GMRES layout since
+        CUDA_TRY(A.tiles.build(h->cta_row, h->leaf_values, A.at_rp, A.at_col, A.at_val.as<double>(), false, s));
+        A.cta_row = h->cta_row;
+    }
+    A.tiles.fill(d, 1, false);
+    // the transposed leaf blocks by columns are the row-major blocks
+    d.pinv = h->d_pinv.as<double>();
+    d.pmat = h->d_pmat.as<double>();
+    d.minv = h->d_minv.as<double>();
     d.row_of = h->d_row_of.as<int32_t>();
     d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
-    d.leaf_begin = h->d_leaf_begin.as<int32_t>();
-    d.leaf_count = h->d_leaf_count.as<int32_t>();
-    d.leaf_of_perm = h->d_leaf_of_perm.as<int32_t>();
-    d.leaf_off = h->d_leaf_off.as<int64_t>();
-    d.cta_leaf = h->d_cta_leaf.as<int32_t>();
-    d.dsm_rows = 0;
-    d.uref_block = h->d_uref_block.as<int64_t>();
-    d.uref_sign = h->d_uref_sign.as<double>();
-    d.uref_known = h->d_uref_known.as<int32_t>();
-    d.tref_block = h->d_tref_block.as<int64_t>();
-    d.tref_sign = h->d_tref_sign.as<double>();
-    d.tref_known = h->d_tref_known.as<int32_t>();
-    d.hist_block = h->d_hist_block.as<int64_t>();
-    d.hu_sign = h->d_hu_sign.as<double>();
-    d.ht_sign = h->d_ht_sign.as<double>();
-    d.hist_owner = h->d_hist_owner.as<int32_t>();
-    d.itf_trans = h->d_itf_trans.as<double>();
-    d.trans = h->g_trans.as<double>();
-    d.bcid = h->g_bcid.as<int32_t>();
-    d.itf_pairs = h->d_itf_pairs.as<int32_t>();
-    d.itf_sign = h->d_itf_sign.as<double>();
-    d.n_itf = (int)h->I;
+    d.row_leaf = h->d_row_leaf.as<RowLeaf>();
+    d.solve_only = 1;
     d.status = A.status.as<int>();
     d.step_flags = A.flags.as<int>();
-    d.audit = A.audit.as<double>();
-    d.xring = A.xring.as<double>();
-    d.wring = A.wring.as<double>();
-    d.known_lu = A.known.as<double>();
-    d.out_lu = A.out_lu.as<double>();
-    d.out_lt = A.out_lt.as<double>();
     d.b = A.gp.as<double>();
     d.groups = 1;
-    d.bp = A.bp.as<double>();
     d.x = A.x.as<double>();
     d.rv = A.rv.as<double>();
+    d.aw = A.aw.as<double>();
     d.u = A.u.as<double>();
     d.V = A.V.as<double>();
-    d.W = A.W.as<double>();
-    d.AW = A.AW.as<double>();
     d.givens = A.givens.as<double>();
     d.restart = h->restart;
     d.tol = h->tol;
     d.cluster = h->cluster;
-    d.givens_stride = (int64_t)kGivensArrays * (h->restart + 2);
+    d.givens_stride = gmres_givens_doubles(h->restart);
     CUDA_TRY(cudaMemsetAsync(A.lam.p, 0, A.lam.bytes, s));
     // the reverse march runs on the device without host round trips:
     // cotangents in, transposed write-back, A'^T solve, KnownM^T, history

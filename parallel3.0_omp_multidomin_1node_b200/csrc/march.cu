@@ -20,12 +20,12 @@
 //                       DBEM1/multidomain.cpp:3086-3225
 #include "march.cuh"
 
+#include <algorithm>
 #include <atomic>
+#include <numeric>
+
+#include "gmres.cuh"
 #include "tdbem_common.cuh"
-
-#include <cooperative_groups.h>
-
-namespace cg = cooperative_groups;
 
 namespace tdbem {
 
@@ -33,12 +33,6 @@ namespace {
 
 constexpr int kRhsThreads = 256;
 constexpr int kMaxDevices = 64;        // launch attributes are kept per device
-constexpr int kGmresThreads = 512;
-constexpr int kGmresWarps = kGmresThreads / 32;
-constexpr int kDotChunk = 8;                // basis vectors per Gram-Schmidt reduction
-constexpr int kDotMax = kDotChunk + 1;      // values per cluster reduction
-
-__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
 
 template <int R, int kCpt = (R >= 4 ? 4 : R)>
 struct Lanes {
@@ -75,27 +69,6 @@ __device__ __forceinline__ void load_cases(const double* p, double* v)
     } else {
         v[0] = *p;
     }
-}
-
-template <int CPT>
-__device__ __forceinline__ void ldcg_cases(const double* p, double* v)
-{
-    if constexpr (CPT == 4) {
-        const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-        const double2 b = __ldcg(reinterpret_cast<const double2*>(p + 2));
-        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-    } else if constexpr (CPT == 2) {
-        const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
-        v[0] = a.x; v[1] = a.y;
-    } else {
-        v[0] = __ldcg(p);
-    }
-}
-
-__device__ __forceinline__ void atomic_max_nonneg(double* addr, double v)
-{
-    // non-negative doubles order like their bit patterns
-    atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
 }  // namespace
@@ -551,931 +524,104 @@ cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr,
 }
 
 // ---------------------------------------------------------------------------
-namespace {
-
-// Per-CTA shared state of the cluster GMRES.
-template <int R>
-struct GShared {
-    double part[2][kDotMax][R];          // this CTA's partial sums (read by peers)
-    double wred[kGmresWarps][kDotMax][R];
-    double vals[kDotMax][R];             // cluster-reduced values of a vector reduction
-    double val[R];                       // cluster-reduced value of a scalar reduction
-    double h1[R], phibar[R], f[R], n2b[R], normr[R], nn[R], hn[R];
-    int run[R], flag[R], inner[R], cycles[R], stag[R], check[R], exact[R];
-    int any, any_exact;
-    int abort_src;  // the status word as cluster rank 0 read it
-    int abort;      // rank 0's reading, copied by every CTA of the cluster
-};
-
-// Cluster-wide sums of m values per load case (m <= M <= kDotMax): thread t
-// contributes v[q] to value q of case t % R.  Every CTA adds the C partials
-// in rank order, so all hold the same results, in vals[q][case].  One
-// cluster barrier; the two partial slots alternate so a peer still reading
-// the previous reduction's slot is never overwritten.
-template <int R, int M>
-__device__ void cluster_sum_vec(double (&v)[M], int m, int& slot, GShared<R>& s, cg::cluster_group& cl)
+template <int R, bool kMixed, bool kLocal>
+__global__ void __launch_bounds__(kGmresThreads, 1) gmres_cluster_kernel(const __grid_constant__ MarchData d, int step)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < M; ++q) {
-        if (q < m) {
-#pragma unroll
-            for (int o = 16; o >= R && o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-            if (lane < R) s.wred[w][q][lane] = v[q];
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < m * R; i += blockDim.x) {
-        const int q = i / R, r = i % R;
-        double t = 0.0;
-#pragma unroll
-        for (int ww = 0; ww < kGmresWarps; ++ww) t += s.wred[ww][q][r];
-        s.part[slot][q][r] = t;
-    }
-    cl.sync();
-    const int C = (int)cl.num_blocks();
-    for (int i = threadIdx.x; i < m * R; i += blockDim.x) {
-        const int q = i / R, r = i % R;
-        double t = 0.0;
-        for (int c = 0; c < C; ++c) t += *cl.map_shared_rank(&s.part[slot][q][r], c);
-        s.vals[q][r] = t;
-    }
-    __syncthreads();
-    slot ^= 1;
-}
-
-// Cluster-wide sum per load case of one value, in val[case].
-template <int R>
-__device__ void cluster_sum(double v, int& slot, GShared<R>& s, cg::cluster_group& cl)
-{
-    double a[1] = {v};
-    cluster_sum_vec<R, 1>(a, 1, slot, s, cl);
-    if (threadIdx.x < R) s.val[threadIdx.x] = s.vals[0][threadIdx.x];
-    __syncthreads();
-}
-
-// y[(3p+c)R + r] = (A' v)[p] for the owned perm rows p in [lo, hi), all cases.
-// A warp works on RPW rows at once, LPR lanes per row (BPR blocks of a row
-// in flight, TPB lanes per block for the load cases).
-template <int R, bool kF32>
-__device__ void spmm_owned(const MarchData& d, const double* v, int lo, int hi, double* y)
-{
-    using L = Lanes<R>;
-    constexpr int CPT = L::CPT, TPB = L::TPB;
-    constexpr int BPR = TPB >= 8 ? 1 : 8 / TPB;
-    constexpr int LPR = TPB * BPR;
-    constexpr int RPW = 32 / LPR;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int rsub = lane / LPR, l2 = lane % LPR;
-    const int bsub = l2 / TPB, cgp = l2 % TPB;
-    for (int p0 = lo + w * RPW; p0 < hi; p0 += kGmresWarps * RPW) {
-        const int p = p0 + rsub;
-        double acc[3][CPT];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int q = 0; q < CPT; ++q) acc[c][q] = 0.0;
-        if (p < hi) {
-            const int jb = d.a_rp[p], je = d.a_rp[p + 1];
-#pragma unroll 2
-            for (int j = jb + bsub; j < je; j += BPR) {
-                const int col = d.a_col[j];
-                double x0[CPT], x1[CPT], x2[CPT];
-                ldcg_cases<CPT>(v + (int64_t)(3 * col) * R + cgp * CPT, x0);
-                ldcg_cases<CPT>(v + (int64_t)(3 * col + 1) * R + cgp * CPT, x1);
-                ldcg_cases<CPT>(v + (int64_t)(3 * col + 2) * R + cgp * CPT, x2);
-                if constexpr (kF32) {
-                    const float* a = d.a_val32 + 9 * (int64_t)j;
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        const float f0 = (float)x0[q], f1 = (float)x1[q], f2 = (float)x2[q];
-                        acc[0][q] += (double)(a[0] * f0 + a[1] * f1 + a[2] * f2);
-                        acc[1][q] += (double)(a[3] * f0 + a[4] * f1 + a[5] * f2);
-                        acc[2][q] += (double)(a[6] * f0 + a[7] * f1 + a[8] * f2);
-                    }
-                } else {
-                    const double* a = d.a_val + 9 * (int64_t)j;
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        acc[0][q] += a[0] * x0[q] + a[1] * x1[q] + a[2] * x2[q];
-                        acc[1][q] += a[3] * x0[q] + a[4] * x1[q] + a[5] * x2[q];
-                        acc[2][q] += a[6] * x0[q] + a[7] * x1[q] + a[8] * x2[q];
-                    }
-                }
-            }
-        }
-        // sum the BPR lane groups of a row (lanes differing in the bsub bits)
-#pragma unroll
-        for (int o = TPB; o < LPR; o <<= 1)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) acc[c][q] += __shfl_xor_sync(0xffffffffu, acc[c][q], o);
-        if (p < hi && bsub == 0)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) y[(int64_t)(3 * p + c) * R + cgp * CPT + q] = acc[c][q];
-    }
-    __syncthreads();
-}
-
-// out = M^-1 in on the owned leaves (block-diagonal leaf inverses,
-// GMRES_M_X, DBEM1/pre_gmres.cpp:837-895; sum over k then n as the
-// reference).  One thread per owned output value and load case.
-template <int R, bool kF32>
-__device__ void precond_owned(const MarchData& d, int lo, int hi, const double* in, double* out)
-{
-    const int64_t nout = 3LL * (hi - lo) * R;
-    for (int64_t t = threadIdx.x; t < nout; t += blockDim.x) {
-        const int r = (int)(t % R);
-        const int e = (int)(t / R);           // owned value index
-        const int p = lo + e / 3, c = e % 3;  // perm row and component
-        const int L = d.leaf_of_perm[p];
-        const int b = d.leaf_begin[L], n3 = 3 * d.leaf_count[L];
-        const int rr = 3 * (p - b) + c;
-        const double* src = in + (int64_t)(3 * b) * R + r;
-        double s = 0.0;
-        if constexpr (kF32) {
-            const float* m = d.pinv32 + d.leaf_off[L] + (int64_t)rr * n3;
-            for (int q = 0; q < n3; ++q) s += (double)(m[q] * (float)src[(int64_t)q * R]);
-        } else {
-            const double* m = d.pinv + d.leaf_off[L] + (int64_t)rr * n3;
-            for (int q = 0; q < n3; ++q) s += m[q] * src[(int64_t)q * R];
-        }
-        out[(int64_t)(3 * lo) * R + t] = s;
-    }
-    __syncthreads();
-}
-
-// spmm_owned with v read from the cluster's shared-memory copies: vs is this
-// CTA's copy of its owned values ([3][R] per row, from its first row); the
-// owner and the row within the owner's range come packed in a_colx.  The
-// result goes to y (global) and, when ys is not null, to this CTA's
-// shared-memory copy.
-template <int R, bool kF32>
-__device__ void spmm_owned_dsm(const MarchData& d, const double* vs, int lo, int hi, double* y, double* ys,
-                               cg::cluster_group& cl)
-{
-    using L = Lanes<R>;
-    constexpr int CPT = L::CPT, TPB = L::TPB;
-    constexpr int BPR = TPB >= 8 ? 1 : 8 / TPB;
-    constexpr int LPR = TPB * BPR;
-    constexpr int RPW = 32 / LPR;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int rsub = lane / LPR, l2 = lane % LPR;
-    const int bsub = l2 / TPB, cgp = l2 % TPB;
-    for (int p0 = lo + w * RPW; p0 < hi; p0 += kGmresWarps * RPW) {
-        const int p = p0 + rsub;
-        double acc[3][CPT];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int q = 0; q < CPT; ++q) acc[c][q] = 0.0;
-        if (p < hi) {
-            const int jb = d.a_rp[p], je = d.a_rp[p + 1];
-#pragma unroll 2
-            for (int j = jb + bsub; j < je; j += BPR) {
-                const int cx = d.a_colx[j];
-                const double* src = cl.map_shared_rank(vs, cx >> 24) + (int64_t)(3 * (cx & 0xFFFFFF)) * R + cgp * CPT;
-                double x0[CPT], x1[CPT], x2[CPT];
-                load_cases<CPT>(src, x0);
-                load_cases<CPT>(src + R, x1);
-                load_cases<CPT>(src + 2 * R, x2);
-                if constexpr (kF32) {
-                    const float* a = d.a_val32 + 9 * (int64_t)j;
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        const float f0 = (float)x0[q], f1 = (float)x1[q], f2 = (float)x2[q];
-                        acc[0][q] += (double)(a[0] * f0 + a[1] * f1 + a[2] * f2);
-                        acc[1][q] += (double)(a[3] * f0 + a[4] * f1 + a[5] * f2);
-                        acc[2][q] += (double)(a[6] * f0 + a[7] * f1 + a[8] * f2);
-                    }
-                } else {
-                    const double* a = d.a_val + 9 * (int64_t)j;
-#pragma unroll
-                    for (int q = 0; q < CPT; ++q) {
-                        acc[0][q] += a[0] * x0[q] + a[1] * x1[q] + a[2] * x2[q];
-                        acc[1][q] += a[3] * x0[q] + a[4] * x1[q] + a[5] * x2[q];
-                        acc[2][q] += a[6] * x0[q] + a[7] * x1[q] + a[8] * x2[q];
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int o = TPB; o < LPR; o <<= 1)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) acc[c][q] += __shfl_xor_sync(0xffffffffu, acc[c][q], o);
-        if (p < hi && bsub == 0)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) {
-                    y[(int64_t)(3 * p + c) * R + cgp * CPT + q] = acc[c][q];
-                    if (ys) ys[(int64_t)(3 * (p - lo) + c) * R + cgp * CPT + q] = acc[c][q];
-                }
-    }
-    __syncthreads();
-}
-
-// precond_owned reading its input from this CTA's shared-memory copy
-// (owned values relative to the first owned row): every leaf lies inside
-// one CTA's range.
-template <int R, bool kF32>
-__device__ void precond_owned_smem(const MarchData& d, int lo, int hi, const double* in_s, double* out)
-{
-    const int64_t nout = 3LL * (hi - lo) * R;
-    for (int64_t t = threadIdx.x; t < nout; t += blockDim.x) {
-        const int r = (int)(t % R);
-        const int e = (int)(t / R);
-        const int p = lo + e / 3, c = e % 3;
-        const int L = d.leaf_of_perm[p];
-        const int b = d.leaf_begin[L], n3 = 3 * d.leaf_count[L];
-        const int rr = 3 * (p - b) + c;
-        const double* src = in_s + (int64_t)(3 * (b - lo)) * R + r;
-        double s0 = 0.0, s1 = 0.0;
-        if constexpr (kF32) {
-            const float* m = d.pinv32 + d.leaf_off[L] + (int64_t)rr * n3;
-            int q = 0;
-            for (; q + 1 < n3; q += 2) {
-                s0 += (double)(m[q] * (float)src[(int64_t)q * R]);
-                s1 += (double)(m[q + 1] * (float)src[(int64_t)(q + 1) * R]);
-            }
-            if (q < n3) s0 += (double)(m[q] * (float)src[(int64_t)q * R]);
-        } else {
-            const double* m = d.pinv + d.leaf_off[L] + (int64_t)rr * n3;
-            // the reference's order: one running sum over the leaf's columns
-            for (int q = 0; q < n3; ++q) s0 += m[q] * src[(int64_t)q * R];
-        }
-        out[(int64_t)(3 * lo) * R + t] = s0 + s1;
-    }
-    __syncthreads();
-}
-
-// Mixed-precision forms of the two products above for the Arnoldi step: the
-// Krylov vector V_j and the product A' V_j are mirrored in shared memory as
-// FP32, the FP32 blocks and leaf inverses multiply them with FP32
-// accumulation, and each output is converted to FP64 once.  (Converting
-// every FP64 operand to FP32 and every FP32 product back, as the FP64
-// mirrors needed, cost about as much as the products.)  The Arnoldi
-// iteration only preconditions the FP64 refinement, which checks every
-// solution on the FP64 residual.
-template <int R>
-__device__ void spmm_owned_dsm32(const MarchData& d, const float* vs, int lo, int hi, double* y, float* ys,
-                                 cg::cluster_group& cl)
-{
-    using L = Lanes<R>;
-    constexpr int CPT = L::CPT, TPB = L::TPB;
-    constexpr int BPR = TPB >= 8 ? 1 : 8 / TPB;
-    constexpr int LPR = TPB * BPR;
-    constexpr int RPW = 32 / LPR;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int rsub = lane / LPR, l2 = lane % LPR;
-    const int bsub = l2 / TPB, cgp = l2 % TPB;
-    for (int p0 = lo + w * RPW; p0 < hi; p0 += kGmresWarps * RPW) {
-        const int p = p0 + rsub;
-        float acc[3][CPT];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-            for (int q = 0; q < CPT; ++q) acc[c][q] = 0.0f;
-        if (p < hi) {
-            const int jb = d.a_rp[p], je = d.a_rp[p + 1];
-#pragma unroll 2
-            for (int j = jb + bsub; j < je; j += BPR) {
-                const int cx = d.a_colx[j];
-                const float* src = cl.map_shared_rank(vs, cx >> 24) + (int64_t)(3 * (cx & 0xFFFFFF)) * R + cgp * CPT;
-                float x0[CPT], x1[CPT], x2[CPT];
-                load_cases<CPT>(src, x0);
-                load_cases<CPT>(src + R, x1);
-                load_cases<CPT>(src + 2 * R, x2);
-                const float* a = d.a_val32 + 9 * (int64_t)j;
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) {
-                    acc[0][q] += a[0] * x0[q] + a[1] * x1[q] + a[2] * x2[q];
-                    acc[1][q] += a[3] * x0[q] + a[4] * x1[q] + a[5] * x2[q];
-                    acc[2][q] += a[6] * x0[q] + a[7] * x1[q] + a[8] * x2[q];
-                }
-            }
-        }
-#pragma unroll
-        for (int o = TPB; o < LPR; o <<= 1)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) acc[c][q] += __shfl_xor_sync(0xffffffffu, acc[c][q], o);
-        if (p < hi && bsub == 0)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int q = 0; q < CPT; ++q) {
-                    y[(int64_t)(3 * p + c) * R + cgp * CPT + q] = (double)acc[c][q];
-                    ys[(int64_t)(3 * (p - lo) + c) * R + cgp * CPT + q] = acc[c][q];
-                }
-    }
-    __syncthreads();
-}
-
-template <int R>
-__device__ void precond_owned_smem32(const MarchData& d, int lo, int hi, const float* in_s, double* out)
-{
-    const int64_t nout = 3LL * (hi - lo) * R;
-    for (int64_t t = threadIdx.x; t < nout; t += blockDim.x) {
-        const int r = (int)(t % R);
-        const int e = (int)(t / R);
-        const int p = lo + e / 3, c = e % 3;
-        const int L = d.leaf_of_perm[p];
-        const int b = d.leaf_begin[L], n3 = 3 * d.leaf_count[L];
-        const int rr = 3 * (p - b) + c;
-        const float* src = in_s + (int64_t)(3 * (b - lo)) * R + r;
-        const float* m = d.pinv32 + d.leaf_off[L] + (int64_t)rr * n3;
-        float s0 = 0.0f, s1 = 0.0f;
-        int q = 0;
-        for (; q + 1 < n3; q += 2) {
-            s0 += m[q] * src[(int64_t)q * R];
-            s1 += m[q + 1] * src[(int64_t)(q + 1) * R];
-        }
-        if (q < n3) s0 += m[q] * src[(int64_t)q * R];
-        out[(int64_t)(3 * lo) * R + t] = (double)(s0 + s1);
-    }
-    __syncthreads();
-}
-
-}  // namespace
-
-// GMRES for the R load cases of one step on one thread-block cluster, then
-// the write-back.  Case r stops updating once converged; the cluster stops
-// when every case has.  FP64 mode checks the true residual b - A x after
-// every inner step (maxit = 1, as the reference).  Mixed mode runs the
-// Arnoldi SpMM and the preconditioner in FP32, keeps orthogonalisation,
-// Givens and the residual recurrence r -= f_j A W_j in FP64, and restarts
-// from the explicit FP64 residual until it meets the tolerance.
-template <int R, bool kMixed>
-__device__ __forceinline__ void gmres_body(const MarchData& d, const int step, const int grp)
-{
-    cg::cluster_group cl = cg::this_cluster();
-    __shared__ GShared<R> s;
-    // Another cluster of the same launch (another load-case group) may set
-    // the status word at any time, so CTAs reading it separately could
-    // disagree and leave peers waiting at a cluster barrier.  Rank 0 reads it
-    // once; every CTA copies that reading through distributed shared memory;
-    // the second barrier keeps rank 0 resident until all copies are taken.
-    if (threadIdx.x == 0 && cl.block_rank() == 0) s.abort_src = *(volatile int*)d.status;
-    cl.sync();
-    if (threadIdx.x == 0) s.abort = *cl.map_shared_rank(&s.abort_src, 0);
-    cl.sync();
-    if (s.abort) return;  // uniform over the cluster
-    const int cq = (int)cl.block_rank();
-    const int C = (int)cl.num_blocks();
-    // grp: cluster = group of load cases
-    const int RT = d.R, roff = grp * R;          // total cases, first case of this group
-    const int E = d.E, rs = d.restart;
-    const int64_t n = 3LL * E * R;           // elements of one private vector
-    const int L0 = d.cta_leaf[cq], L1 = d.cta_leaf[cq + 1];
-    const int lo = L0 < L1 ? d.leaf_begin[L0] : 0;
-    const int hi = L0 < L1 ? d.leaf_begin[L1 - 1] + d.leaf_count[L1 - 1] : 0;
-    const int64_t ob = 3LL * lo * R, oe = 3LL * hi * R;  // owned element range
-    double* G = d.givens + ((int64_t)grp * C + cq) * R * d.givens_stride;
-    auto gcs = [&](int r) { return G + (int64_t)r * d.givens_stride; };
-    // givens layout per case: cs[rs+2], sn[rs+2], h[rs+2], rcol[rs+2]
-    const int gl = rs + 2;
-    int slot = 0;
-    double* b = d.bp + (int64_t)grp * n;
-    double* x = d.x + (int64_t)grp * n;
-    double* rv = d.rv + (int64_t)grp * n;
-    double* u = d.u + (int64_t)grp * n;
-    double* const Vb = d.V + (int64_t)grp * (rs + 1) * n;
-    double* const Wb = d.W + (int64_t)grp * (rs + 1) * n;
-    double* const AWb = d.AW + (int64_t)grp * (rs + 1) * n;
-    // Krylov vector copies in shared memory (when d.dsm_rows > 0): V_j and
-    // V_{j+1} alternate in vs[0], vs[1]; xsm mirrors x; aws holds A V_j for
-    // the preconditioner.  Peers read vs and xsm through distributed shared
-    // memory in the sparse products.
-    extern __shared__ __align__(16) double dsm[];
-    const bool use_dsm = d.dsm_rows > 0;
-    const int64_t S = 3LL * d.dsm_rows * R;
-    // FP64 mode: vs[0], vs[1], xsm, aws, all FP64; mixed mode: xsm in FP64,
-    // then FP32 mirrors vs32[0], vs32[1] of V_j and aws32 of A' V_j (mirror i
-    // at base + i S: offsets, not pointer arrays, which would live in local
-    // memory)
-    double* const vs64 = dsm;
-    double* const xsm = kMixed ? dsm : dsm + 2 * S;
-    double* const aws = dsm + 3 * S;
-    float* const vs32 = reinterpret_cast<float*>(dsm + S);
-    float* const aws32 = vs32 + 2 * S;
-    // private copy of this group's right-hand side columns
-    for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x)
-        b[t] = d.b[(t / R) * RT + roff + (t % R)];
-    __syncthreads();
-
-    double part = 0.0;
-    // mixed mode starts from the solutions of the previous steps extrapolated
-    // linearly (x_{s-1} at step 2); the FP64 path starts from zero as the
-    // reference does (DBEM1/multidomain.cpp:3869-3870)
-    const bool warm = kMixed && d.xold != nullptr && step >= 2;
-    double* xold = warm ? d.xold + (int64_t)grp * n : nullptr;
-    if (!warm) {
-        for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-            x[t] = 0.0;
-            if (use_dsm) xsm[t - ob] = 0.0;
-            if (kMixed && d.xold) d.xold[(int64_t)grp * n + t] = 0.0;
-            const double bb = b[t];
-            rv[t] = bb;
-            part += bb * bb;
-        }
-        cluster_sum<R>(part, slot, s, cl);
-        if (threadIdx.x < R) {
-            const int r = threadIdx.x;
-            s.n2b[r] = sqrt(s.val[r]);
-            const double tolb = d.tol * s.n2b[r];
-            s.flag[r] = (s.n2b[r] == 0.0 || s.n2b[r] <= tolb) ? 0 : 1;
-            s.inner[r] = 0;
-            s.cycles[r] = 0;
-        }
-        __syncthreads();
-    } else {
-        for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-            const double x1 = x[t], x2 = xold[t];
-            const double x0 = step == 2 ? x1 : 2.0 * x1 - x2;
-            xold[t] = x1;
-            x[t] = x0;
-            if (use_dsm) xsm[t - ob] = x0;
-        }
-        cl.sync();  // the start vector is complete in every CTA
-        if (use_dsm)
-            spmm_owned_dsm<R, false>(d, xsm, lo, hi, u, nullptr, cl);
-        else
-            spmm_owned<R, false>(d, x, lo, hi, u);
-        double acc[2] = {0.0, 0.0};
-        for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-            const double bb = b[t], rr = bb - u[t];
-            rv[t] = rr;
-            acc[0] += bb * bb;
-            acc[1] += rr * rr;
-        }
-        cluster_sum_vec<R, 2>(acc, 2, slot, s, cl);
-        if (threadIdx.x < R) {
-            const int r = threadIdx.x;
-            s.n2b[r] = sqrt(s.vals[0][r]);
-            const double tolb = d.tol * s.n2b[r];
-            s.flag[r] = (s.n2b[r] == 0.0 || sqrt(s.vals[1][r]) <= tolb) ? 0 : 1;
-            s.inner[r] = 0;
-            s.cycles[r] = 0;
-        }
-        __syncthreads();
-    }
-    const int max_cycles = kMixed ? 8 : 1;
-    for (int cycle = 0; cycle < max_cycles; ++cycle) {
-        if (threadIdx.x == 0) {
-            int a = 0;
-            for (int r = 0; r < R; ++r) a |= s.flag[r] == 1;
-            s.any = a;
-        }
-        __syncthreads();
-        if (!s.any) break;
-        // vh = M^-1 r, V_1 = vh / |vh|, x0 kept in W's last column
-        precond_owned<R, kMixed>(d, lo, hi, rv, u);
-        part = 0.0;
-        for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) part += u[t] * u[t];
-        cluster_sum<R>(part, slot, s, cl);
-        if (threadIdx.x < R) {
-            const int r = threadIdx.x;
-            s.h1[r] = sqrt(s.val[r]);
-            s.phibar[r] = s.h1[r];
-            s.run[r] = s.flag[r] == 1;
-            s.stag[r] = 0;
-            if (s.run[r]) s.cycles[r]++;
-        }
-        __syncthreads();
-        double* X0 = Wb + (int64_t)rs * n;
-        static_assert(kGmresThreads % R == 0, "a thread's values all belong to one case");
-        const int tr0 = (int)((ob + threadIdx.x) % R);  // the case of every value this thread owns
-        const bool run0 = s.run[tr0] != 0;
-        const double inv_h1 = run0 ? 1.0 / s.h1[tr0] : 0.0;
-        for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-            const double v1 = run0 ? u[t] * inv_h1 : 0.0;
-            Vb[t] = v1;
-            if (use_dsm) {
-                if constexpr (kMixed) vs32[t - ob] = (float)v1;
-                else vs64[t - ob] = v1;
-            }
-            X0[t] = x[t];
-        }
-        cl.sync();  // V_1 complete
-        for (int j = 1; j <= rs; ++j) {
-            if (threadIdx.x == 0) {
-                int a = 0;
-                for (int r = 0; r < R; ++r) a |= s.run[r];
-                s.any = a;
-            }
-            __syncthreads();
-            if (!s.any) break;
-            const double* Vj = Vb + (int64_t)(j - 1) * n;
-            double* AWj = AWb + (int64_t)(j - 1) * n;
-            if (use_dsm) {
-                if constexpr (kMixed) {
-                    spmm_owned_dsm32<R>(d, vs32 + ((j - 1) & 1) * S, lo, hi, AWj, aws32, cl);  // A V_j
-                    precond_owned_smem32<R>(d, lo, hi, aws32, u);                             // u = M^-1 A V_j
-                } else {
-                    spmm_owned_dsm<R, false>(d, vs64 + ((j - 1) & 1) * S, lo, hi, AWj, aws, cl);
-                    precond_owned_smem<R, false>(d, lo, hi, aws, u);
-                }
-            } else {
-                spmm_owned<R, kMixed>(d, Vj, lo, hi, AWj);
-                precond_owned<R, kMixed>(d, lo, hi, AWj, u);
-            }
-            // Classical Gram-Schmidt applied twice (CGS2): each sweep over the
-            // owned values handles up to kDotChunk basis vectors and ends in
-            // one cluster reduction, instead of one reduction per basis
-            // vector as in MGS (DBEM1/pre_gmres.cpp:1462-1485).  The basis
-            // and the Hessenberg column are MGS's up to rounding.
-            const int tr = (int)((ob + threadIdx.x) % R);  // the case of every value this thread owns
-            const double* hcol = gcs(tr) + 2 * gl;
-            const double* ccol = gcs(tr) + 4 * gl;
-            // sweep 1: h_k = V_k . u
-            for (int k0 = 1; k0 <= j; k0 += kDotChunk) {
-                const int nk = min(kDotChunk, j - k0 + 1);
-                double acc[kDotChunk];
-#pragma unroll
-                for (int q = 0; q < kDotChunk; ++q) acc[q] = 0.0;
-                for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                    const double ut = u[t];
-#pragma unroll
-                    for (int q = 0; q < kDotChunk; ++q)
-                        if (q < nk) acc[q] += Vb[(int64_t)(k0 - 1 + q) * n + t] * ut;
-                }
-                cluster_sum_vec<R, kDotChunk>(acc, nk, slot, s, cl);
-                for (int i = threadIdx.x; i < nk * R; i += blockDim.x)
-                    gcs(i % R)[2 * gl + k0 + i / R] = s.vals[i / R][i % R];
-                __syncthreads();
-            }
-            // sweep 2: u' = u - sum_k h_k V_k (kept in u), c_k = V_k . u',
-            // and |u'|^2 with the first chunk
-            for (int k0 = 1; k0 <= j; k0 += kDotChunk) {
-                const int nk = min(kDotChunk, j - k0 + 1);
-                double acc[kDotMax];
-#pragma unroll
-                for (int q = 0; q < kDotMax; ++q) acc[q] = 0.0;
-                for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                    double ut = u[t];
-                    if (k0 == 1) {
-#pragma unroll 4
-                        for (int k = 1; k <= j; ++k) ut -= hcol[k] * Vb[(int64_t)(k - 1) * n + t];
-                        u[t] = ut;
-                        acc[kDotChunk] += ut * ut;
-                    }
-#pragma unroll
-                    for (int q = 0; q < kDotChunk; ++q)
-                        if (q < nk) acc[q] += Vb[(int64_t)(k0 - 1 + q) * n + t] * ut;
-                }
-                cluster_sum_vec<R, kDotMax>(acc, k0 == 1 ? kDotMax : nk, slot, s, cl);
-                for (int i = threadIdx.x; i < nk * R; i += blockDim.x)
-                    gcs(i % R)[4 * gl + k0 + i / R] = s.vals[i / R][i % R];
-                if (k0 == 1 && threadIdx.x < R) s.nn[threadIdx.x] = s.vals[kDotChunk][threadIdx.x];
-                __syncthreads();
-            }
-            // h(k, j) = h_k + c_k; |u''|^2 = |u'|^2 - sum c_k^2 unless that
-            // cancels (near breakdown): then u'' and its norm explicitly
-            if (threadIdx.x < R) {
-                const int r = threadIdx.x;
-                double* h = gcs(r) + 2 * gl;
-                const double* c = gcs(r) + 4 * gl;
-                double cc = 0.0;
-                for (int k = 1; k <= j; ++k) {
-                    cc += c[k] * c[k];
-                    h[k] += c[k];
-                }
-                const double est = s.nn[r] - cc;
-                s.exact[r] = !(est > 1.0e-4 * s.nn[r]);
-                s.hn[r] = s.exact[r] ? 0.0 : sqrt(est);
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int a = 0;
-                for (int r = 0; r < R; ++r) a |= s.exact[r];
-                s.any_exact = a;
-            }
-            __syncthreads();
-            if (s.any_exact) {
-                part = 0.0;
-                for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                    double ut = u[t];
-                    for (int k = 1; k <= j; ++k) ut -= ccol[k] * Vb[(int64_t)(k - 1) * n + t];
-                    u[t] = ut;
-                    part += ut * ut;
-                }
-                cluster_sum<R>(part, slot, s, cl);
-                if (threadIdx.x < R) s.hn[threadIdx.x] = sqrt(s.val[threadIdx.x]);
-                __syncthreads();
-            }
-            // Givens: R(1:j, j) = G_{j-1}..G_1 h(1:j), new rotation from (R(j,j), h(j+1))
-            if (threadIdx.x < R) {
-                const int r = threadIdx.x;
-                double* cs = gcs(r);
-                double* sn = cs + gl;
-                double* h = sn + gl;
-                double* rc = h + gl;
-                const double hn = s.hn[r];
-                h[j + 1] = hn;
-                for (int k = 1; k <= j; ++k) rc[k] = h[k];
-                for (int i = 1; i < j; ++i) {
-                    const double a = rc[i], bb = rc[i + 1];
-                    rc[i] = cs[i] * a - sn[i] * bb;
-                    rc[i + 1] = sn[i] * a + cs[i] * bb;
-                }
-                const double rt = rc[j];
-                double c, sv, temp;
-                if (hn == 0.0) {
-                    c = 1.0;
-                    sv = 0.0;
-                } else if (hn * hn > rt * rt) {
-                    temp = rt / hn;
-                    sv = 1.0 / sqrt(1.0 + fabs(temp) * fabs(temp));
-                    c = -temp * sv;
-                } else {
-                    temp = hn / rt;
-                    c = 1.0 / sqrt(1.0 + fabs(temp) * fabs(temp));
-                    sv = -temp * c;
-                }
-                rc[j] = c * rt - sv * hn;
-                cs[j] = c;
-                sn[j] = sv;
-                s.f[r] = c * s.phibar[r];
-                s.phibar[r] = sv * s.phibar[r];
-                if (s.run[r] && s.f[r] == 0.0) s.stag[r] = 1;
-            }
-            __syncthreads();
-            // sweep 3: V_{j+1} = (u' - sum_k c_k V_k) / h(j+1, j) (zero when
-            // h(j+1, j) <= 1e-12, DBEM1/pre_gmres.cpp:1481-1485);
-            // W_j = (V_j - sum_l W_l R(l,j)) / R(j,j); x += f_j W_j; the same
-            // recurrence on A V_j gives A W_j and the residual r -= f_j A W_j
-            double* Vn = Vb + (int64_t)j * n;
-            double* const vsn = vs64 + (j & 1) * S;
-            float* const vsn32 = vs32 + (j & 1) * S;
-            double* Wj = Wb + (int64_t)(j - 1) * n;
-            const bool sub = !s.any_exact;
-            const double hn_t = s.hn[tr];
-            const bool run_t = s.run[tr] != 0;
-            const double f_t = s.f[tr];
-            const double* rc_t = gcs(tr) + 3 * gl;
-            // one reciprocal per case and step: every value this thread owns
-            // belongs to case tr, so the loops below multiply instead of
-            // dividing (FP64 division is a long instruction sequence)
-            const double inv_rjj = 1.0 / rc_t[j];
-            const bool vzero = hn_t <= 1.0e-12;
-            const double inv_hn = vzero ? 0.0 : 1.0 / hn_t;
-            part = 0.0;
-            for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                double ut = u[t];
-                if (sub) {
-#pragma unroll 4
-                    for (int k = 1; k <= j; ++k) ut -= ccol[k] * Vb[(int64_t)(k - 1) * n + t];
-                }
-                const double vn = vzero ? 0.0 : ut * inv_hn;
-                Vn[t] = vn;
-                if (use_dsm) {
-                    if constexpr (kMixed) vsn32[t - ob] = (float)vn;
-                    else vsn[t - ob] = vn;
-                }
-                if (!run_t) {
-                    Wj[t] = 0.0;
-                    AWj[t] = 0.0;
-                } else {
-                    double wv = Vj[t];
-                    double aw = AWj[t];
-#pragma unroll 4
-                    for (int l = 1; l <= j - 1; ++l) {
-                        wv -= Wb[(int64_t)(l - 1) * n + t] * rc_t[l];
-                        aw -= AWb[(int64_t)(l - 1) * n + t] * rc_t[l];
-                    }
-                    wv *= inv_rjj;
-                    aw *= inv_rjj;
-                    Wj[t] = wv;
-                    AWj[t] = aw;
-                    const double xn = x[t] + f_t * wv;
-                    x[t] = xn;
-                    if (use_dsm) xsm[t - ob] = xn;
-                    rv[t] -= f_t * aw;
-                }
-                part += rv[t] * rv[t];
-            }
-            cluster_sum<R>(part, slot, s, cl);  // also orders V_{j+1} and x for the next step
-            if (threadIdx.x < R) {
-                const int r = threadIdx.x;
-                s.check[r] = 0;
-                if (s.run[r]) {
-                    s.inner[r]++;
-                    const double normr = sqrt(s.val[r]);
-                    const double tolb = d.tol * s.n2b[r];
-                    if (normr <= tolb) {
-                        s.check[r] = 1;            // verify with the true residual
-                    } else if (s.stag[r]) {
-                        s.run[r] = 0;
-                        s.flag[r] = 3;
-                    } else if (kMixed && fabs(s.phibar[r]) <= 1.0e-5 * s.h1[r]) {
-                        s.run[r] = 0;              // FP32 Krylov space exhausted: refine
-                    }
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int a = 0;
-                for (int r = 0; r < R; ++r) a |= s.check[r];
-                s.any = a;
-            }
-            __syncthreads();
-            if (s.any) {
-                // the reference's stopping test is on b - A x (DBEM1/pre_gmres.cpp:1566-1578)
-                cl.sync();
-                if (use_dsm)
-                    spmm_owned_dsm<R, false>(d, xsm, lo, hi, u, nullptr, cl);
-                else
-                    spmm_owned<R, false>(d, x, lo, hi, u);
-                part = 0.0;
-                for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                    const double tr = b[t] - u[t];
-                    if (s.check[t % R]) rv[t] = tr;
-                    part += tr * tr;
-                }
-                cluster_sum<R>(part, slot, s, cl);
-                if (threadIdx.x < R) {
-                    const int r = threadIdx.x;
-                    if (s.check[r] && sqrt(s.val[r]) <= d.tol * s.n2b[r]) {
-                        s.run[r] = 0;
-                        s.flag[r] = 0;
-                    } else if (s.check[r] && kMixed) {
-                        s.run[r] = 0;              // refine from the FP64 residual
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        if constexpr (kMixed) {
-            // explicit FP64 residual of the refined x
-            cl.sync();
-            if (use_dsm)
-                spmm_owned_dsm<R, false>(d, xsm, lo, hi, rv, nullptr, cl);
-            else
-                spmm_owned<R, false>(d, x, lo, hi, rv);
-            part = 0.0;
-            for (int64_t t = ob + threadIdx.x; t < oe; t += blockDim.x) {
-                rv[t] = b[t] - rv[t];
-                part += rv[t] * rv[t];
-            }
-            cluster_sum<R>(part, slot, s, cl);
-            if (threadIdx.x < R) {
-                const int r = threadIdx.x;
-                if (s.flag[r] == 1 && sqrt(s.val[r]) <= d.tol * s.n2b[r]) s.flag[r] = 0;
-            }
-            __syncthreads();
-        }
-    }
-    if (threadIdx.x < R && cq == 0) {
-        const int r = threadIdx.x;
-        int* fl = d.step_flags + ((int64_t)(step - 1) * RT + roff + r) * 3;
-        fl[0] = s.flag[r];
-        fl[1] = s.cycles[r];
-        fl[2] = s.inner[r];
-        if (s.flag[r] != 0) atomicExch(d.status, 1);
-    }
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int r = 0; r < R; ++r) a |= s.flag[r] != 0;
-        s.any = a;
-    }
-    cl.sync();  // x complete; the failure decision is uniform
-    if (s.any || d.solve_only) {
-        cl.sync();
-        return;
-    }
-
-    // ---- write-back (ScatterUnknownToBoundary + AllLocToAbs +
-    //      BuildPhysicalStateFromBoundary) ----
-    const int nh = d.nh;
-    const int xs = step % 3;
-    const int64_t gtid = (int64_t)cq * blockDim.x + threadIdx.x, gstride = (int64_t)C * blockDim.x;
-    for (int64_t t = gtid; t < (int64_t)E * R; t += gstride) {
-        const int64_t i = t / R;
-        const int r = (int)(t % R), rg = roff + r;
-        const double* T = d.itf_trans + 9 * i;
-        const double* in = d.known_lu + (((int64_t)rg * (d.nstep + 1) + step) * E + i) * 3;
-        double lu[3], lt[3];
-        if (d.uref_known[i]) {
-            for (int c = 0; c < 3; ++c) lu[c] = d.uref_sign[i] * in[c];
-        } else {
-            const int64_t pb = d.perm_of_unk[d.uref_block[i]];
-            const double v0 = ldcg(x + (3 * pb) * R + r), v1 = ldcg(x + (3 * pb + 1) * R + r),
-                         v2 = ldcg(x + (3 * pb + 2) * R + r);
-            for (int c = 0; c < 3; ++c) lu[c] = d.uref_sign[i] * (T[3 * c] * v0 + T[3 * c + 1] * v1 + T[3 * c + 2] * v2);
-        }
-        if (d.tref_known[i]) {
-            for (int c = 0; c < 3; ++c) lt[c] = d.tref_sign[i] * in[c];
-        } else {
-            const int64_t pb = d.perm_of_unk[d.tref_block[i]];
-            const double v0 = ldcg(x + (3 * pb) * R + r), v1 = ldcg(x + (3 * pb + 1) * R + r),
-                         v2 = ldcg(x + (3 * pb + 2) * R + r);
-            for (int c = 0; c < 3; ++c) lt[c] = d.tref_sign[i] * (T[3 * c] * v0 + T[3 * c + 1] * v1 + T[3 * c + 2] * v2);
-        }
-        const double* F = d.trans + 9 * i;
-        double gu[3], gt[3];
-        for (int c = 0; c < 3; ++c) {
-            gu[c] = F[c] * lu[0] + F[3 + c] * lu[1] + F[6 + c] * lu[2];
-            gt[c] = F[c] * lt[0] + F[3 + c] * lt[1] + F[6 + c] * lt[2];
-        }
-        double* ou = d.out_lu + (((int64_t)rg * (d.nstep + 1) + step) * E + i) * 3;
-        double* ot = d.out_lt + (((int64_t)rg * (d.nstep + 1) + step) * E + i) * 3;
-        for (int c = 0; c < 3; ++c) {
-            ou[c] = gu[c];
-            ot[c] = gt[c];
-        }
-        if (d.hist_owner[i]) {
-            const int64_t hb = d.hist_block[i];
-            double* XU = d.xring + (((int64_t)xs * 2 + 0) * nh + hb) * 3 * RT + rg;
-            double* XT = d.xring + (((int64_t)xs * 2 + 1) * nh + hb) * 3 * RT + rg;
-            for (int c = 0; c < 3; ++c) {
-                XU[c * RT] = d.hu_sign[i] * gu[c];
-                XT[c * RT] = d.ht_sign[i] * gt[c];
-            }
-        }
-    }
-    if (d.rec_x && grp == 0)
-        for (int64_t uu = gtid; uu < E; uu += gstride) {
-            const int64_t pb = d.perm_of_unk[uu];
-            for (int c = 0; c < 3; ++c) d.rec_x[(int64_t)(step - 1) * 3 * E + 3 * uu + c] = ldcg(x + (3 * pb + c) * R);
-        }
-    cl.sync();  // X_s complete
-    // W_{s-1} = (X_s + 2 X_{s-1}) + X_{s-2};  W_s = 2 X_s + X_{s-1}
-    // (BuildConvolutionVector's coefficients 1, 2, 1 and summation order;
-    //  X_0 and unsolved states are zero, DBEM1/multidomain.cpp:3201-3225)
-    const int SW = d.SW;
-    const int x1 = (step + 2) % 3, x2 = (step + 1) % 3;
-    const int wa = (step - 1) % SW, wb = step % SW;
-    const int64_t per_type = (int64_t)nh * 3 * RT;
-    for (int64_t tt = gtid; tt < 2LL * nh * 3 * R; tt += gstride) {
-        // this group's cases only: (type, history column, component, case)
-        const int64_t type = tt / ((int64_t)nh * 3 * R);
-        const int64_t nc = (tt / R) % ((int64_t)nh * 3);
-        const int64_t rest = nc * RT + roff + (tt % R);
-        const double Xs = ldcg(d.xring + ((int64_t)xs * 2 + type) * per_type + rest);
-        const double Xm1 = ldcg(d.xring + ((int64_t)x1 * 2 + type) * per_type + rest);
-        const double Xm2 = ldcg(d.xring + ((int64_t)x2 * 2 + type) * per_type + rest);
-        const double wcomplete = (Xs + 2.0 * Xm1) + Xm2;
-        const double wpartial = 2.0 * Xs + Xm1;
-        d.wring[((int64_t)wa * 2 + type) * per_type + rest] = wcomplete;
-        d.wring[((int64_t)wb * 2 + type) * per_type + rest] = wpartial;
-    }
-    // interface audit (PrintInterfaceError, DBEM1/multidomain.cpp:3227-3257)
-    for (int64_t t = gtid; t < (int64_t)d.n_itf * R; t += gstride) {
-        const int64_t pi = t / R;
-        const int r = roff + (int)(t % R);
-        const int a = d.itf_pairs[2 * pi], bb = d.itf_pairs[2 * pi + 1];
-        const int64_t base = ((int64_t)r * (d.nstep + 1) + step) * E;
-        const double* ua = d.out_lu + (base + a) * 3;
-        const double* ub = d.out_lu + (base + bb) * 3;
-        const double* ta = d.out_lt + (base + a) * 3;
-        const double* tb = d.out_lt + (base + bb) * 3;
-        double jump = 0.0, bal = 0.0;
-        for (int c = 0; c < 3; ++c) {
-            jump = fmax(jump, fabs(ua[c] - ub[c]));
-            bal = fmax(bal, fabs(tb[c] - d.itf_sign[pi] * ta[c]));
-        }
-        atomic_max_nonneg(d.audit + 2 * (step - 1), jump);
-        atomic_max_nonneg(d.audit + 2 * (step - 1) + 1, bal);
-    }
-    cl.sync();  // no CTA leaves while a peer may still read its shared memory
-}
-
-template <int R, bool kMixed>
-__global__ void __launch_bounds__(kGmresThreads, 1) gmres_cluster_kernel(MarchData d, int step)
-{
-    gmres_body<R, kMixed>(d, step, (int)(blockIdx.x / cg::this_cluster().num_blocks()));
+    gmres_body<R, kMixed, kLocal>(d, step, (int)(blockIdx.x / cg::this_cluster().num_blocks()));
 }
 
 // Several models' GMRES of one step in one launch: cluster m solves model m
 // (one group of R load cases each; every model laid out for the launch's
 // cluster size); models whose march is shorter skip.
-template <int R, bool kMixed>
+template <int R, bool kMixed, bool kLocal>
 __global__ void __launch_bounds__(kGmresThreads, 1) gmres_models_kernel(const MarchData* ds, int step)
 {
     __shared__ MarchData sd;
     load_model(ds, (int)(blockIdx.x / cg::this_cluster().num_blocks()), sd);
     if (step > sd.nstep) return;
-    gmres_body<R, kMixed>(sd, step, 0);
+    gmres_body<R, kMixed, kLocal>(sd, step, 0);
 }
 
 // ---------------------------------------------------------------------------
 namespace {
 
-template <int R, bool kMixed>
-cudaError_t launch_gmres(const MarchData& d, int step, cudaStream_t s)
+// Dynamic shared memory of the GMRES kernel at most (of the 227 KB a CTA may
+// have; the several-models form keeps its model there too).
+constexpr size_t kGmresDsmMax = 224 * 1024;
+// Basis vectors kept in shared memory at most: solves take 6 to 18 steps, and
+// what shared memory leaves is L1.
+constexpr int kVcapMax = 20, kVcapMin = 10;
+
+// Threads of a GMRES CTA owning `rows` rows: a small range does not run its
+// barriers over idle warps, but a warp per dot product pays.
+int gmres_threads(int rows, int Rg)
 {
+    const int n = 3 * rows * Rg;
+    return n <= 192 ? 256 : kGmresThreads;
+}
+
+// Caches leaf inverses and basis vectors in `room` bytes of shared memory and
+// returns the bytes taken.  A step reads the inverses behind its product, whose
+// stream of A' evicts them from L1 (one load case on the 3,072-element bar:
+// 5,600 cycles per application against 2,200 cached); for one or two cases,
+// whose vectors are short, only when kVcapMin vectors fit beside them.
+size_t gmres_caches(MarchData& d, size_t room, int Rg, bool mixed)
+{
+    const size_t vec = sizeof(double) * 3 * (size_t)d.dsm_rows * Rg;
+    const size_t leaf = 16 * (size_t)d.dsm_rows +
+                        ((size_t)d.leaf_max * (mixed ? sizeof(float) : sizeof(double)) + 15) / 16 * 16;
+    const size_t want = (size_t)std::min(d.restart + 1, kVcapMax);
+    const size_t least = std::min<size_t>(want, Rg <= 2 ? kVcapMin : 0);
+    size_t used = 0;
+    d.leaf_cap = 0;
+    if (leaf + least * vec <= room) {
+        d.leaf_cap = d.leaf_max;
+        used = leaf;
+    }
+    d.vcap = (int)std::min<size_t>((room - used) / vec, want);
+    return used + vec * (size_t)d.vcap;
+}
+
+// Raises a kernel's dynamic shared memory to the most the device allows and
+// lets it run in clusters of 16, once per device: changing attributes between
+// launches (models of different sizes marched side by side) would be a
+// host-side attribute change per launch.  Returns that size in cap.
+template <class K>
+cudaError_t gmres_attributes(K kernel, std::atomic<int> (&dyn_max)[kMaxDevices], int& cap)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    cap = dyn_max[dev].load();
+    if (cap != 0) return cudaSuccess;
+    cudaFuncAttributes fa{};
+    int optin = 0;
+    if ((e = cudaFuncGetAttributes(&fa, kernel)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+    cap = optin - (int)fa.sharedSizeBytes;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+    dyn_max[dev].store(cap);
+    return cudaSuccess;
+}
+
+template <int R, bool kMixed, bool kLocal>
+cudaError_t launch_gmres_form(const MarchData& d0, int step, cudaStream_t s)
+{
+    MarchData d = d0;
+    static std::atomic<int> dyn_max[kMaxDevices];
+    int cap = 0;
+    cudaError_t e = gmres_attributes(gmres_cluster_kernel<R, kMixed, kLocal>, dyn_max, cap);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(d.cluster * d.groups);
-    cfg.blockDim = dim3(kGmresThreads);
-    cfg.dynamicSmemBytes = gmres_dsm_bytes(d.dsm_rows, R, kMixed);
+    cfg.blockDim = dim3(gmres_threads(d.own_rows, R));
+    cfg.dynamicSmemBytes = gmres_dsm_bytes(d.dsm_rows, d.halo_rows, R, kMixed);
     cfg.stream = s;
+    if (cfg.dynamicSmemBytes > (size_t)cap) return cudaErrorInvalidValue;
+    // the rest of the shared memory goes to leaf inverses and basis vectors
+    if (kLocal) cfg.dynamicSmemBytes += gmres_caches(d, (size_t)cap - cfg.dynamicSmemBytes, R, kMixed);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = d.cluster;
@@ -1483,31 +629,14 @@ cudaError_t launch_gmres(const MarchData& d, int step, cudaStream_t s)
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // the function attributes are set once per device, to the most the device
-    // allows: changing them between launches (models of different sizes
-    // marched side by side) would be a host-side attribute change per launch
-    static std::atomic<int> dyn_max[kMaxDevices];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-    int cap = dyn_max[dev].load();
-    if (cap == 0) {
-        cudaFuncAttributes fa{};
-        int optin = 0;
-        if ((e = cudaFuncGetAttributes(&fa, gmres_cluster_kernel<R, kMixed>)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
-        cap = optin - (int)fa.sharedSizeBytes;
-        if ((e = cudaFuncSetAttribute(gmres_cluster_kernel<R, kMixed>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      cap)) != cudaSuccess)
-            return e;
-        if ((e = cudaFuncSetAttribute(gmres_cluster_kernel<R, kMixed>,
-                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-            return e;
-        dyn_max[dev].store(cap);
-    }
-    if (cfg.dynamicSmemBytes > (size_t)cap) return cudaErrorInvalidValue;
-    return cudaLaunchKernelEx(&cfg, gmres_cluster_kernel<R, kMixed>, d, step);
+    return cudaLaunchKernelEx(&cfg, gmres_cluster_kernel<R, kMixed, kLocal>, d, step);
+}
+
+template <int R, bool kMixed>
+cudaError_t launch_gmres(const MarchData& d, int step, cudaStream_t s)
+{
+    return d.dsm_rows > 0 ? launch_gmres_form<R, kMixed, true>(d, step, s)
+                          : launch_gmres_form<R, kMixed, false>(d, step, s);
 }
 
 template <int R, bool kMixed>
@@ -1525,13 +654,13 @@ int cluster_size_for(int device)
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (c > 8 && cudaFuncSetAttribute(gmres_cluster_kernel<R, kMixed>,
+        if (c > 8 && cudaFuncSetAttribute(gmres_cluster_kernel<R, kMixed, true>,
                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gmres_cluster_kernel<R, kMixed>, &cfg) == cudaSuccess && n >= 1)
+        if (cudaOccupancyMaxActiveClusters(&n, gmres_cluster_kernel<R, kMixed, true>, &cfg) == cudaSuccess && n >= 1)
             return c;
         cudaGetLastError();
     }
@@ -1688,11 +817,118 @@ cudaError_t march_step(const MarchData& d, int step, cudaStream_t s, cudaStream_
 
 cudaError_t gmres_solve_single(const MarchData& d, cudaStream_t s) { return launch_gmres<1, false>(d, 1, s); }
 
-size_t gmres_dsm_bytes(int rows, int Rg, bool mixed)
+namespace {
+
+size_t gmres_shared_bytes(int Rg)
 {
-    // FP64: four FP64 vectors; mixed: one FP64 vector and three FP32 ones
-    const size_t per = mixed ? sizeof(double) + 3 * sizeof(float) : 4 * sizeof(double);
-    return rows > 0 ? per * 3 * (size_t)rows * Rg : 0;
+    switch (Rg) {
+    case 1: return (sizeof(GShared<1>) + 15) / 16 * 16;
+    case 2: return (sizeof(GShared<2>) + 15) / 16 * 16;
+    case 4: return (sizeof(GShared<4>) + 15) / 16 * 16;
+    case 8: return (sizeof(GShared<8>) + 15) / 16 * 16;
+    case 16: return (sizeof(GShared<16>) + 15) / 16 * 16;
+    default: return (sizeof(GShared<32>) + 15) / 16 * 16;
+    }
+}
+
+}  // namespace
+
+size_t gmres_dsm_bytes(int rows, int halo, int Rg, bool mixed)
+{
+    const size_t row = 3 * (size_t)Rg, stride = Rg == 1 ? 4 : row, m = mixed ? sizeof(float) : sizeof(double);
+    // shared state; product vector with its halo, work vector, product
+    return gmres_shared_bytes(Rg) + (size_t)(rows + halo) * stride * sizeof(double) +
+           (size_t)rows * (row * sizeof(double) + row * m);
+}
+
+bool gmres_dsm_fits(int rows, int halo, int Rg, bool mixed)
+{
+    return rows > 0 && gmres_dsm_bytes(rows, halo, Rg, mixed) <= kGmresDsmMax;
+}
+
+int gmres_row_capacity(int own_rows) { return (own_rows + 3) / 4 * 4; }  // 16-byte aligned vectors
+
+void gmres_tile_index(const std::vector<int32_t>& cta_row, int own_cap, const std::vector<int32_t>& rp,
+                      const std::vector<int32_t>& col, GmresTileIndex& out)
+{
+    const int C = (int)cta_row.size() - 1, E = cta_row[C];
+    std::vector<int32_t> owner((size_t)E), slot((size_t)E, -1), mark((size_t)E, -1), remote, order;
+    for (int c = 0; c < C; ++c)
+        for (int p = cta_row[c]; p < cta_row[c + 1]; ++p) owner[p] = c;
+    out = GmresTileIndex{};
+    out.cs.assign((size_t)C + 1, 0);
+    out.halo.assign((size_t)C, 0);
+    std::vector<std::vector<int2>> send((size_t)C);
+    for (int c = 0; c < C; ++c) {
+        // rows of other CTAs that this CTA's rows use, in perm order
+        remote.clear();
+        for (int j = rp[cta_row[c]]; j < rp[cta_row[c + 1]]; ++j)
+            if (owner[col[j]] != c && mark[col[j]] != c) {
+                mark[col[j]] = c;
+                remote.push_back(col[j]);
+            }
+        std::sort(remote.begin(), remote.end());
+        for (size_t i = 0; i < remote.size(); ++i) {
+            const int q = remote[i], o = owner[q];
+            slot[q] = own_cap + (int)i;
+            send[o].push_back(int2{(int)(((uint32_t)c << 24) | (uint32_t)(q - cta_row[o])), slot[q]});
+        }
+        out.halo[c] = (int32_t)remote.size();
+        out.halo_max = std::max(out.halo_max, (int)remote.size());
+        out.cs[c] = (int32_t)out.sp.size();
+        // longest rows first: a slice's rows are of about one length (little
+        // padding), and the warps' last slices are the short ones
+        order.resize((size_t)(cta_row[c + 1] - cta_row[c]));
+        std::iota(order.begin(), order.end(), cta_row[c]);
+        std::stable_sort(order.begin(), order.end(),
+                         [&](int a, int b) { return rp[a + 1] - rp[a] > rp[b + 1] - rp[b]; });
+        for (size_t i0 = 0; i0 < order.size(); i0 += 4) {
+            const size_t i1 = std::min(i0 + 4, order.size());
+            const int most = rp[order[i0] + 1] - rp[order[i0]];
+            out.sp.push_back(int2{(int)(out.col.size() / 32), most});
+            for (size_t i = i0; i < i0 + 4; ++i) out.rows.push_back(i < i1 ? order[i] - cta_row[c] : -1);
+            const size_t base = out.col.size(), tiles = (size_t)(most + 7) / 8;
+            // padding: a zero block at the CTA's first row
+            out.col.resize(base + 32 * tiles, 0);
+            out.colg.resize(base + 32 * tiles, cta_row[c]);
+            out.src.resize(base + 32 * tiles, -1);
+            for (size_t i = i0; i < i1; ++i)
+                for (int p = order[i], j = rp[p]; j < rp[p + 1]; ++j) {
+                    const int b = j - rp[p], q = col[j];
+                    const size_t at = base + 32 * (size_t)(b / 8) + 8 * (i - i0) + b % 8;
+                    out.col[at] = owner[q] == c ? q - cta_row[c] : slot[q];
+                    out.colg[at] = q;
+                    out.src[at] = j;
+                }
+        }
+    }
+    out.cs[C] = (int32_t)out.sp.size();
+    out.send_ptr.assign((size_t)C + 1, 0);
+    for (int c = 0; c < C; ++c) {
+        out.send.insert(out.send.end(), send[c].begin(), send[c].end());
+        out.send_ptr[c + 1] = (int32_t)out.send.size();
+    }
+}
+
+// Tile values from row-major 3x3 blocks; a block of the padding is zero.
+__global__ void gather_tiles_kernel(int64_t n, const int32_t* src, const double* val9, double* out, float* out32)
+{
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t tile = t / 288, c = (t - tile * 288) / 32, l = t & 31;
+        const int32_t j = src[tile * 32 + l];
+        const double v = j < 0 ? 0.0 : val9[9 * (int64_t)j + c];
+        out[t] = v;
+        if (out32) out32[t] = (float)v;
+    }
+}
+
+cudaError_t gather_tiles(int64_t tiles, const int32_t* src, const double* val9, double* out, float* out32,
+                         cudaStream_t s)
+{
+    if (tiles <= 0) return cudaSuccess;
+    const int64_t n = tiles * 288;
+    gather_tiles_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1184), 256, 0, s>>>(n, src, val9, out, out32);
+    return cudaGetLastError();
 }
 
 namespace {
@@ -1701,7 +937,7 @@ namespace {
 // every model, then one GMRES cluster of C CTAs per model.
 template <int R, bool kMixed>
 cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models, int total_rows, int cluster,
-                          size_t gmres_dsm, int max_K, int step, int phase, cudaStream_t s)
+                          size_t gmres_dsm, bool local, int max_K, int step, int phase, cudaStream_t s)
 {
     constexpr int kC = R >= 4 ? 4 : R;
     const size_t smem = sizeof(int) * (size_t)(max_K + 1);
@@ -1712,25 +948,11 @@ cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models,
     rhs_models_kernel<R, kMixed, false, kC><<<total_rows, kRhsThreads, smem, s>>>(ds, row_off, n_models, step, phase);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    static std::atomic<int> dyn_max[kMaxDevices];
-    int dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
-    int cap = dyn_max[dev].load();
-    if (cap == 0) {
-        cudaFuncAttributes fa{};
-        int optin = 0;
-        if ((e = cudaFuncGetAttributes(&fa, gmres_models_kernel<R, kMixed>)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
-        cap = optin - (int)fa.sharedSizeBytes;
-        if ((e = cudaFuncSetAttribute(gmres_models_kernel<R, kMixed>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      cap)) != cudaSuccess)
-            return e;
-        if ((e = cudaFuncSetAttribute(gmres_models_kernel<R, kMixed>,
-                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-            return e;
-        dyn_max[dev].store(cap);
-    }
+    static std::atomic<int> dyn_max[2][kMaxDevices];
+    int cap = 0;
+    e = local ? gmres_attributes(gmres_models_kernel<R, kMixed, true>, dyn_max[1], cap)
+              : gmres_attributes(gmres_models_kernel<R, kMixed, false>, dyn_max[0], cap);
+    if (e != cudaSuccess) return e;
     if (gmres_dsm > (size_t)cap) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster * n_models);
@@ -1744,20 +966,22 @@ cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed>, ds, step);
+    return local ? cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed, true>, ds, step)
+                 : cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed, false>, ds, step);
 }
 
 }  // namespace
 
 cudaError_t march_models_step(const MarchData* ds, const int* row_off, int n_models, int total_rows, int R,
-                              bool mixed, int cluster, size_t gmres_dsm, int max_K, int step, int phase, cudaStream_t s)
+                              bool mixed, int cluster, size_t gmres_dsm, bool local, int max_K, int step, int phase,
+                              cudaStream_t s)
 {
 #define TDBEM_MODELS_CASE(RR)                                                                                      \
     case RR:                                                                                                       \
-        return mixed ? models_step_r<RR, true>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, max_K, step, \
-                                               phase, s)                                                           \
-                     : models_step_r<RR, false>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, max_K, step, \
-                                                phase, s);
+        return mixed ? models_step_r<RR, true>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, local, max_K,    \
+                                               step, phase, s)                                                     \
+                     : models_step_r<RR, false>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, local, max_K,   \
+                                                step, phase, s);
     switch (R) {
         TDBEM_MODELS_CASE(1)
         TDBEM_MODELS_CASE(2)

@@ -16,6 +16,12 @@ namespace tdbem {
 // unk_of[p] = preferred unknown of row_of[p]), so the preconditioner is
 // block diagonal and every GMRES CTA owns one contiguous perm range.
 // Vectors over the 3E unknowns are stored [3E][R], load case fastest.
+struct RowLeaf {
+    int64_t off;    // of the leaf's dense block
+    int32_t begin;  // its first perm row
+    int32_t n3;     // 3 x its rows
+};
+
 struct MarchData {
     int E;            // elements = equation rows = unknown blocks
     int n_known;      // known blocks
@@ -51,24 +57,39 @@ struct MarchData {
     const double* known_sign;
     const int32_t* k_elem;  // per KnownM block: known_elem of its column
     const double* k_sgn;    // per KnownM block: known_sign of its column
-    // permuted system matrix A' and preconditioner
-    const int32_t* a_rp;
-    const int32_t* a_col;
-    const double* a_val;    // [nnz][9]
-    const float* a_val32;
+    // permuted system matrix A' and preconditioner, laid out for the GMRES
+    // cluster (GmresTiles): CTA c owns the perm rows cta_row[c] .. cta_row[c+1]
+    // and the slices (4 rows each) g_cs[c] .. g_cs[c+1]; slice s starts at tile
+    // g_sp[s].x of 4 rows x 8 blocks, g_sp[s].y blocks in its longest row, its
+    // rows (within the range, -1 past the end) at g_rows[4 s]; a tile holds 32 columns and 9 planes of 32 values, padded with zero blocks.
+    // Columns are rows of the CTA's product vector (g_col): its own rows, then
+    // from dsm_rows on the g_halo[c] rows of other CTAs that its rows use, which
+    // their owners send (g_send_ptr[c] .. of g_send: x = peer << 24 | own row,
+    // y = row there); or perm rows (g_colg)
+    const int32_t* cta_row;
+    const int32_t* g_cs;
+    const int2* g_sp;
+    const int32_t* g_rows;
+    const int32_t* g_halo;
+    const int32_t* g_send_ptr;
+    const int2* g_send;
+    const int32_t* g_col;
+    const int32_t* g_colg;
+    const double* g_val;
+    const float* g_val32;
     const int32_t* row_of;  // perm -> equation row
     const int32_t* perm_of_unk; // unknown block -> perm
-    const int32_t* leaf_begin;
-    const int32_t* leaf_count;
-    const int32_t* leaf_of_perm;  // perm index -> leaf
-    const int64_t* leaf_off;  // offset of each leaf's dense inverse
-    const double* pinv;       // dense (3L x 3L) leaf inverses, row-major
+    const RowLeaf* row_leaf;  // leaf of each perm row
+    const double* pinv;       // dense (3L x 3L) leaf inverses, column-major
     const float* pinv32;
-    const int32_t* cta_leaf;  // [C+1] leaf range per GMRES CTA of the cluster
-    // A' columns as (owner CTA rank << 24) | row within the owner's range,
-    // for Krylov vectors read from the cluster's shared memory
-    const int32_t* a_colx;
-    int dsm_rows;             // rows of the largest owned range; 0 = vectors read from global memory
+    const double* pmat;       // the leaves' dense blocks, column-major
+    const double* minv;       // largest Frobenius norm of a leaf inverse
+    int own_rows;             // rows of the largest owned range
+    int dsm_rows;             // row capacity of the shared-memory vectors; 0 = vectors in global memory
+    int halo_rows;            // largest g_halo
+    int leaf_max;             // values of the largest CTA's leaf inverses
+    int leaf_cap;             // room for cached leaf inverses, in values (0: not cached), and
+    int vcap;                 // basis vectors kept in shared memory; both set at launch
     // per-element write-back data
     const int64_t* uref_block; const double* uref_sign; const int32_t* uref_known;
     const int64_t* tref_block; const double* tref_sign; const int32_t* tref_known;
@@ -77,9 +98,8 @@ struct MarchData {
     const double* itf_trans;    // [E][9] local transform of interface B sides (identity elsewhere)
     const double* trans;        // [E][9] element frames
     const int32_t* bcid;
-    const int32_t* itf_pairs;   // [I][2] eleA, eleB
-    const double* itf_sign;     // [I]
-    int n_itf;
+    const int32_t* itf_a;       // [E] A-side element of an interface's B-side element, else -1
+    const double* itf_asign;    // [E] its normal sign
     // state
     double* xring;    // [3][2][nh][3][R] physical history states X_s (type 0 = U, 1 = T)
     double* wring;    // [SW][2][nh][3][R] combined history vectors
@@ -89,15 +109,14 @@ struct MarchData {
     // GMRES: `groups` clusters, cluster g solves load cases [g*Rg, (g+1)*Rg)
     // with private Krylov storage ([3E][Rg] per vector) at offset g
     int groups;
-    double* bp;       // [groups][3E][Rg] right-hand side copy
     double* x;        // [groups][3E][Rg] perm solution
     double* xold;     // [groups][3E][Rg] solution of the step before (mixed-mode start vector), or null
-    double* rv;       // [groups][3E][Rg] residual
-    double* u;        // [groups][3E][Rg] Arnoldi work vector
-    double* V;        // [groups][restart+1][3E][Rg]
-    double* W;        // [groups][restart+1][3E][Rg] (last column keeps the refinement start x)
-    double* AW;       // [groups][restart+1][3E][Rg] A W_j (mixed: residual recurrence)
-    double* givens;   // [groups][C][Rg] cs, sn, h, rcol, c ([restart+2] each, kGivensArrays)
+    double* V;        // [groups][restart+1][3E][Rg] basis vectors beyond vcap
+    // vectors of the global-memory form (dsm_rows = 0): solution, product, work
+    double* rv;       // [groups][3E][Rg]
+    double* aw;       // [groups][3E][Rg]
+    double* u;        // [groups][3E][Rg]
+    double* givens;   // [groups][C][Rg] small arrays of gmres_givens_doubles(restart) each
     int* status;      // [0] abort
     int* step_flags;  // [nstep][R][3] flag, refinements, inner iterations
     double* audit;    // [nstep][2] max interface jump, balance
@@ -114,10 +133,31 @@ struct MarchData {
     int solve_only;          // 1: GMRES alone, no write-back, history update or audit (bare solve)
 };
 
-// Arrays of restart+2 doubles per (GMRES CTA, load case) in MarchData::givens:
-// rotation cosines and sines, the Hessenberg column, its rotated copy and the
-// second Gram-Schmidt pass's coefficients.
+// Small arrays per (GMRES CTA, load case) in MarchData::givens: restart+2
+// doubles each of rotation cosines and sines, the Hessenberg column, the second
+// Gram-Schmidt pass's coefficients and the rotated right-hand side (the columns
+// that do not fit in shared memory), then the rotated Hessenberg columns.
 constexpr int kGivensArrays = 5;
+constexpr int64_t gmres_givens_doubles(int restart)
+{
+    return (int64_t)kGivensArrays * (restart + 2) + (int64_t)(restart + 1) * (restart + 2) / 2;
+}
+constexpr int kGmresClusterMax = 16;
+
+// A' in the tile form of MarchData::g_*, built on the host as block indices and
+// gathered on the device (gather_tiles): src[tile][32] is the block of the
+// row-major array, or -1.  own_cap: row capacity of the owned part of a CTA's
+// product vector.
+struct GmresTileIndex {
+    std::vector<int32_t> cs, rows, halo, send_ptr, col, colg, src;
+    std::vector<int2> sp, send;
+    int halo_max = 0;
+};
+int gmres_row_capacity(int own_rows);
+void gmres_tile_index(const std::vector<int32_t>& cta_row, int own_cap, const std::vector<int32_t>& rp,
+                      const std::vector<int32_t>& col, GmresTileIndex& out);
+cudaError_t gather_tiles(int64_t tiles, const int32_t* src, const double* val9, double* out, float* out32,
+                         cudaStream_t s);
 
 // Run layout of the stacked history blocks of steps k >= kr (MarchData r_*),
 // built on the device from the stacked arrays (kptr on the host and the
@@ -168,16 +208,16 @@ int gmres_cluster_size(int device, int R, bool mixed);
 // phase 2: only the bulk (history steps k >= 3) of `step` into the models'
 // bulk buffers.  ds: device array of the models' MarchData (each laid out for
 // `cluster`); row_off: [n_models + 1] prefix sums of their element counts;
-// gmres_dsm: the largest dynamic shared memory any model's GMRES needs;
+// gmres_dsm: the largest dynamic shared memory any model's GMRES needs; local:
+// every model's vectors are in shared memory (dsm_rows > 0), else none's are;
 // max_K: the largest history length.
 cudaError_t march_models_step(const MarchData* ds, const int* row_off, int n_models, int total_rows, int R,
-                              bool mixed, int cluster, size_t gmres_dsm, int max_K, int step, int phase,
+                              bool mixed, int cluster, size_t gmres_dsm, bool local, int max_K, int step, int phase,
                               cudaStream_t s);
 // The FP64 single-load GMRES step kernel on caller-supplied storage: d.R = 1,
-// d.groups = 1, d.nstep = 1, step 1.  Every pointer it writes (b, bp, x, rv,
-// u, V, W, AW, givens, status, step_flags, and unless d.solve_only the
-// write-back targets out_lu, out_lt, xring, wring, audit) must be sized for
-// that shape.
+// d.groups = 1, d.nstep = 1, step 1.  Every pointer it writes (b, x, rv,
+// aw, u, V, givens, status, step_flags, and unless d.solve_only the write-back
+// targets out_lu, out_lt, xring, wring, audit) must be sized for that shape.
 cudaError_t gmres_solve_single(const MarchData& d, cudaStream_t s);
 // Adjoint march, step n: adj[type][col][3] (type 0 = U, 1 = T) = the
 // transposed history convolution of the adjoint right-hand sides
@@ -251,11 +291,11 @@ cudaError_t adjoint_known(int n_known, const int32_t* kt_ptr, const int32_t* kt_
                           double* gk, cudaStream_t s);
 cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr, const int32_t* trow,
                         const double* tval, const double* lam, double* adj, cudaStream_t s);
-// Dynamic shared memory of the GMRES kernel for Rg load cases per cluster
-// and owned ranges of at most `rows` rows (0 when rows == 0).
-size_t gmres_dsm_bytes(int rows, int Rg, bool mixed);
-// Largest dynamic shared memory the GMRES kernel takes for the shared-memory
-// Krylov path; owned ranges needing more fall back to global memory.
-constexpr size_t kGmresDsmMax = 200 * 1024;
+// Shared memory of the GMRES kernel for Rg load cases per cluster, a row
+// capacity of `rows` (0: the global-memory form) and `halo` rows from other
+// CTAs, without cached leaf inverses and basis vectors; and whether that fits
+// (else the global-memory form runs).
+size_t gmres_dsm_bytes(int rows, int halo, int Rg, bool mixed);
+bool gmres_dsm_fits(int rows, int halo, int Rg, bool mixed);
 
 }  // namespace tdbem
