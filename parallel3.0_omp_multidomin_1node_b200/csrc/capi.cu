@@ -472,6 +472,9 @@ struct tdbem_handle {
     DevBuf d_r_ptr, d_r_meta, d_r_off, d_r_val;  // run layout of steps k >= run_k (T-step history pass)
     int64_t r_nb = 0, r_runs = 0;
     int run_k = 0;
+    DevBuf d_hg_ptr, d_hg_meta, d_hg_off, d_hg_val, d_hg_rows;  // group layout instead, for 8 or more load cases
+    int64_t hg_steps = 0, hg_segs = 0;
+    int hg_n = 0;  // groups (0: no group layout)
     DevBuf d_k_rp, d_k_col, d_k_val, d_k_elem, d_k_sgn;
     DevBuf d_a_rp, d_a_col, d_a_val, d_row_of, d_unk_of, d_perm_of_unk;
     DevBuf d_leaf_begin, d_leaf_count, d_leaf_off, d_row_leaf;
@@ -819,6 +822,33 @@ tdbem_status compact(tdbem_handle* h, const PairSpace& ps, const DevBuf& flags, 
     return TDBEM_OK;
 }
 
+// Orders rows so that each G in turn are neighbours: halves at a multiple of G
+// along the longest side of their nodes' box, and each half again.
+void bisect_rows(const std::vector<double>& node, int32_t* b, int32_t* e, int G)
+{
+    const int64_t n = e - b;
+    if (n <= G) return;
+    double lo[3], hi[3];
+    for (int c = 0; c < 3; ++c) {
+        lo[c] = hi[c] = node[3 * (size_t)b[0] + c];
+        for (const int32_t* i = b; i < e; ++i) {
+            lo[c] = std::min(lo[c], node[3 * (size_t)*i + c]);
+            hi[c] = std::max(hi[c], node[3 * (size_t)*i + c]);
+        }
+    }
+    int axis = 0;
+    for (int c = 1; c < 3; ++c)
+        if (hi[c] - lo[c] > hi[axis] - lo[axis]) axis = c;
+    std::sort(b, e, [&](int32_t i, int32_t j) {
+        const double x = node[3 * (size_t)i + axis], y = node[3 * (size_t)j + axis];
+        return x < y || (x == y && i < j);
+    });
+    int32_t* m = b + (n / 2 + G - 1) / G * G;
+    if (m >= e) m = e - (n % G ? n % G : G);
+    bisect_rows(node, b, m, G);
+    bisect_rows(node, m, e, G);
+}
+
 // Run layout of the history steps k >= 2T + 1 for the T-step history pass
 // (two or more load cases; T = 2, or 3 with TDBEM_HISTORY_STEPS=3 and at
 // least 7 history steps; off with TDBEM_RUNS=0).  Left out, and the march
@@ -838,8 +868,9 @@ tdbem_status build_runs(tdbem_handle* h, cudaStream_t s)
     h->d_r_meta.release();
     h->d_r_off.release();
     h->d_r_val.release();
-    h->r_nb = h->r_runs = 0;
-    h->run_k = 0;
+    for (DevBuf* b : {&h->d_hg_ptr, &h->d_hg_meta, &h->d_hg_off, &h->d_hg_val, &h->d_hg_rows}) b->release();
+    h->r_nb = h->r_runs = h->hg_steps = h->hg_segs = 0;
+    h->run_k = h->hg_n = 0;
     const int E = (int)h->E, K = h->K;
     if (K < kRunK || h->R < 2 || h->h_nnz == 0) return TDBEM_OK;
     if (const char* v = std::getenv("TDBEM_RUNS"))
@@ -850,6 +881,48 @@ tdbem_status build_runs(tdbem_handle* h, cudaStream_t s)
     const bool mixed = h->precision == TDBEM_PRECISION_MIXED;
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    constexpr int G = kGroupRows;
+    if (h->R >= 8 && (double)history_groups_bytes(nb, mixed) * 1.1 + (double)(1ull << 30) <= (double)free_b) {
+        // groups: neighbouring rows of one domain, by bisection of its nodes
+        std::vector<int32_t> place((size_t)E, 0), rows, perm_of_row((size_t)E), list;
+        for (int64_t p = 0; p < E; ++p) perm_of_row[h->repid[p]] = (int32_t)p;
+        for (int d = 0; d < h->D; ++d) {
+            list.resize((size_t)h->dom_count[d]);
+            std::iota(list.begin(), list.end(), h->dom_begin[d]);
+            bisect_rows(h->node, list.data(), list.data() + list.size(), G);
+            while (rows.size() % G) rows.push_back(-1);
+            for (int32_t r : list) {
+                place[r] = (int32_t)rows.size();
+                rows.push_back(perm_of_row[r]);
+            }
+        }
+        while (rows.size() % G) rows.push_back(-1);
+        const int groups = (int)(rows.size() / G);
+        HistoryGroups hg;
+        const void* vals = mixed ? static_cast<const void*>(h->d_h_val32.p) : static_cast<const void*>(h->d_h_val.p);
+        const cudaError_t e =
+            build_history_groups(E, K, kRunK, place, groups, h->h_kptr, h->d_h_kptr.as<int64_t>(),
+                                 h->d_h_col.as<uint32_t>(), vals, h->h_nnz, mixed, hg, s);
+        h->d_hg_ptr.adopt(hg.ptr, sizeof(int64_t) * (groups + 1));
+        h->d_hg_meta.adopt(hg.meta, sizeof(uint2) * (size_t)hg.segments);
+        h->d_hg_off.adopt(hg.off, sizeof(int64_t) * (size_t)hg.segments);
+        h->d_hg_val.adopt(hg.val, (mixed ? sizeof(float) : sizeof(double)) * 96 * (size_t)hg.steps);
+        if (e == cudaSuccess && hg.kr > 0) {
+            CUDA_TRY(up(h->d_hg_rows, rows, s));
+            CUDA_TRY(cudaStreamSynchronize(s));
+            h->hg_n = groups;
+            h->hg_steps = hg.steps;
+            h->hg_segs = hg.segments;
+            h->run_k = hg.kr;
+            return TDBEM_OK;
+        }
+        // out of device memory part way, or too little in common between
+        // neighbouring rows: the run layout
+        for (DevBuf* b : {&h->d_hg_ptr, &h->d_hg_meta, &h->d_hg_off, &h->d_hg_val}) b->release();
+        if (e != cudaErrorMemoryAllocation) CUDA_TRY(e);
+        cudaGetLastError();
+        CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    }
     if ((double)history_runs_bytes(nb, mixed) * 1.1 + (double)(1ull << 30) > (double)free_b) return TDBEM_OK;
     HistoryRuns hr;
     const void* vals = mixed ? static_cast<const void*>(h->d_h_val32.p) : static_cast<const void*>(h->d_h_val.p);
@@ -1291,6 +1364,15 @@ struct MarchRun {
         d.r_val32 = h->d_r_val.as<float>();
         d.r_nb = h->r_nb;
         d.kr = h->run_k;
+        d.hg_n = h->hg_n;
+        // a CTA's warps get about a dozen segments each
+        d.hg_split = 1;
+        while (d.hg_n > 0 && d.hg_split < 8 && h->hg_segs > (int64_t)d.hg_n * d.hg_split * 2 * 4 * 12) d.hg_split *= 2;
+        d.hg_ptr = h->d_hg_ptr.as<int64_t>();
+        d.hg_meta = h->d_hg_meta.as<uint2>();
+        d.hg_off = h->d_hg_off.as<int64_t>();
+        d.hg_val = h->d_hg_val.p;
+        d.hg_rows = h->d_hg_rows.as<int32_t>();
         d.k_rp = h->d_k_rp.as<int32_t>();
         d.k_col = h->d_k_col.as<int32_t>();
         d.k_val = h->d_k_val.as<double>();
@@ -1450,14 +1532,17 @@ struct MarchRun {
                         // distinct W slots: t0 + h - k over the launch's (h, k)
                         const int slots = (t0 + T - 1 - kr) - std::max(t0 - klast, 0) + 1;
                         const int steps_out = std::min(T, N - t0 + 1);
-                        hb = (double)(cum[klast] - cum[kr - 1]) * 9.0 * vs + (double)h->r_runs * 16.0 +
+                        hb = (double)(cum[klast] - cum[kr - 1]) * 9.0 * vs +
+                             (double)(h->hg_n ? h->hg_segs : h->r_runs) * 16.0 +
                              std::max(slots, 0) * slot_b + (double)E * 24.0 * R * steps_out + steps_out * known_b;
                         for (int hh = 0; hh < T; ++hh)
                             rep.history_block_steps +=
                                 (double)std::max<int64_t>(cum[std::min(t0 + hh, K)] - cum[kr - 1], 0);
+                        // (groups: the full history's count from the first pass on)
                         rep.history_vector_loads +=
-                            (double)(cum[std::min(t0, K)] > cum[kr - 1] ? cum[std::min(t0, K)] - cum[kr - 1] : 0) +
-                            (double)(T - 1) * h->r_runs;
+                            h->hg_n ? (double)h->hg_steps * 4.0 / 3.0 + (double)(T - 1) * h->hg_segs
+                                  : (double)(cum[std::min(t0, K)] > cum[kr - 1] ? cum[std::min(t0, K)] - cum[kr - 1] : 0) +
+                                        (double)(T - 1) * h->r_runs;
                         ++rep.history_launches;
                     }
                 } else if (step + 1 <= N) {

@@ -91,6 +91,10 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t addr, uint32_t rank)
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+__device__ __forceinline__ void peer_load1(uint32_t addr, double& v)
+{
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+}
 // asynchronous stores into a peer's shared memory, counted by its mbarrier
 __device__ __forceinline__ void push8(uint32_t addr, unsigned long long v, uint32_t bar)
 {

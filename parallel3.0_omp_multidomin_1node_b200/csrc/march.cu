@@ -423,6 +423,250 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same part of the right-hand sides over the group layout (8 or more load
+// cases): a cluster of CTAs takes a group of 8 rows.  What bounds it: FP64
+// multiply-adds (1.0 ms a launch at full rate on the 3,072-element bar with 32
+// load cases).  bulk_steps_kernel spends 2.1 ms there: it reads a history
+// vector of 768 bytes from L2 per block and two steps, 17.6 GB, and converts
+// every FP32 block value in each lane that uses it, at a quarter of the
+// multiply-add rate.  Here a segment is a product of matrices on the FP64
+// tensor path (m8n8k4, as fast as scalar FP64 and one operand load per eight
+// products): 24 equation components by 3 x steps, times 3 x steps by load
+// cases, once per time step with the vectors shifted by a step.  A warp walks
+// segments; the fragments and vectors come to its ring of stages by cp.async,
+// kChunk steps each, and a vector read serves 8 rows and T steps, a value 8 T
+// products.  The CTAs of a cluster split the segments (a CTA of some 0.2 ms
+// does not hold up the GMRES clusters that wait for its SM) and sum in rank
+// order.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(__cvta_generic_to_global(src)) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// c += a b, 8 x 4 by 4 x 8: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
+// c[l / 4][2 (l % 4)], c[l / 4][2 (l % 4) + 1]
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b)
+{
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c0), "+d"(c1) : "d"(a), "d"(b));
+}
+
+template <int R, int T, class V>
+struct GroupPass {
+    // 8 cases make little of a step: longer chunks for them
+    static constexpr int NW = 4, kThreads = 32 * NW, kChunk = R == 8 ? 8 : 4, kStages = 3, NT = R / 8;
+    static constexpr int kSteps = kChunk / 4 * 3;                                 // contraction steps of a chunk
+    static constexpr int kRowLen = R + 4;                                         // padded: no bank conflicts between fragment rows
+    static constexpr int kVecs = (kChunk + T - 1) * 3 * kRowLen;                  // doubles of a stage's vectors
+    static constexpr int kStage = kVecs * 8 + kSteps * 3 * 32 * (int)sizeof(V);  // bytes
+    static constexpr int kSums = T * 24 * R;                            // doubles of a CTA's sums
+    static constexpr size_t kRing = (size_t)NW * kStages * kStage, kRed = sizeof(double) * (size_t)(NW + 1) * kSums;
+    static constexpr size_t kBytes = kRing > kRed ? kRing : kRed;
+};
+
+template <int R, int T, class V>
+__global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kernel(const __grid_constant__ MarchData d,
+                                                                                   int t0, int split)
+{
+    using P = GroupPass<R, T, V>;
+    constexpr int NT = P::NT, NW = P::NW;
+    const int group = (int)blockIdx.x / split, rank = (int)blockIdx.x % split;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // runs beside GMRES launches that may set the status word: the cluster
+    // takes rank 0's reading
+    __shared__ int stop, stop_all;
+    if (threadIdx.x == 0) stop = *(volatile int*)d.status;
+    unsigned char* const ring = reinterpret_cast<unsigned char*>(dsm) + w * P::kStages * P::kStage;
+    for (int i = lane; i < P::kStages * P::kStage / 8; i += 32) reinterpret_cast<double*>(ring)[i] = 0.0;
+    __syncthreads();
+    if (split > 1) {
+        cluster_barrier();
+        if (threadIdx.x == 0) stop_all = *cg::this_cluster().map_shared_rank(&stop, 0);
+        cluster_barrier();
+        if (stop_all) return;
+    } else if (stop) {
+        return;
+    }
+    const int SW = d.SW, klast = t0 + T - 1 < d.K ? t0 + T - 1 : d.K;  // last step of the last sum
+    const int64_t slot_len = 2LL * d.nh * 3 * R;
+    const int64_t seg_end = __ldg(d.hg_ptr + group + 1);
+    const int seg_step = NW * split;
+    // a position in the warp's sequence of chunks: its segments of the group
+    // (longest first; the warps take them in turn, every other round in reverse,
+    // so their totals are alike), kChunk steps at a time
+    struct Pos {
+        int64_t seg;
+        int skip;            // to the warp's next segment
+        const V* val;        // first fragment of the segment
+        const double* vec;   // its (type, column) in slot 0 of the ring of vectors
+        int k0, len, j;      // first step, steps within the last sum, next step
+    };
+    const int mine = rank * NW + w;
+    auto next_seg = [&](Pos& p) {
+        p.seg += p.skip;
+        p.skip = 2 * seg_step - p.skip;
+    };
+    auto load_seg = [&](Pos& p) {
+        // segments that start past the last sum's steps are skipped
+        for (; p.seg < seg_end; next_seg(p)) {
+            const uint2 mt = __ldg(d.hg_meta + p.seg);
+            p.k0 = (int)(mt.y >> 16);
+            p.len = min((int)(mt.y & 0xFFFFu), klast - p.k0 + 1);
+            p.val = static_cast<const V*>(d.hg_val) + __ldg(d.hg_off + p.seg) * 96;
+            p.vec = d.wring + ((int64_t)(mt.x >> 20) * d.nh + (mt.x & 0xFFFFFu)) * 3 * R;
+            p.j = 0;
+            if (p.len > 0) return;
+        }
+    };
+    auto advance = [&](Pos& p) {
+        p.j += P::kChunk;
+        if (p.j >= p.len) {
+            next_seg(p);
+            load_seg(p);
+        }
+    };
+    // One chunk into a stage: the vectors W_{t0+T-1-k0-j} and on, backwards in
+    // time, one more than its steps need (its last fragment may reach into the
+    // next step), then the fragments of its ceil(3 n / 4) contraction steps.
+    // Vectors of steps not yet reached (only while t0 < K) are slots that are
+    // still zero.
+    auto issue = [&](const Pos& p, int stage) {
+        const int n = min(P::kChunk, p.len - p.j), vecs = min(n + T, P::kChunk + T - 1), ks = (3 * n + 3) / 4;
+        const uint32_t vdst = shared_addr(ring + stage * P::kStage), fdst = vdst + P::kVecs * 8;
+        constexpr int kPieces = 3 * R / 2, kPer = 16 / sizeof(V);  // 16-byte pieces of a vector, values of a piece
+        const int slot0 = ((t0 + T - 1 - p.k0 - p.j) % SW + SW) % SW;
+        auto vector_piece = [&](int q, int slot, int i) {
+            copy16(vdst + 8 * ((3 * q + i / (R / 2)) * P::kRowLen + 2 * (i % (R / 2))), p.vec + slot * slot_len + 2 * i);
+        };
+        if constexpr (kPieces < 16) {
+            // a warp's copy takes pieces of several vectors
+#pragma unroll 2
+            for (int i = lane; i < vecs * kPieces; i += 32) {
+                const int q = i / kPieces;
+                vector_piece(q, slot0 >= q ? slot0 - q : slot0 - q + SW, i % kPieces);
+            }
+        } else {
+            int slot = slot0;
+#pragma unroll 1
+            for (int q = 0; q < vecs; ++q) {
+#pragma unroll
+                for (int i0 = 0; i0 < kPieces; i0 += 32)
+                    if (i0 + lane < kPieces) vector_piece(q, slot, i0 + lane);
+                slot = slot == 0 ? SW - 1 : slot - 1;
+            }
+        }
+        const V* f = p.val + (p.j / 4) * 288;
+#pragma unroll 2
+        for (int i = lane; i < ks * 96 / kPer; i += 32) copy16(fdst + 16 * i, f + kPer * i);
+    };
+    double acc[3][NT][T][2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int h = 0; h < T; ++h) acc[i][q][h][0] = acc[i][q][h][1] = 0.0;
+    Pos cur{}, ahead{};
+    cur.seg = __ldg(d.hg_ptr + group) + mine;
+    cur.skip = 2 * (seg_step - mine) - 1;
+    load_seg(cur);
+    ahead = cur;
+    for (int i = 0; i < P::kStages - 1; ++i) {
+        if (ahead.seg < seg_end) {
+            issue(ahead, i);
+            advance(ahead);
+        }
+        copy_commit();
+    }
+    int stage = 0, fill = P::kStages - 1;
+#pragma unroll 1
+    while (cur.seg < seg_end) {
+        copy_wait<P::kStages - 2>();
+        __syncwarp();  // the stage's copies of all lanes; and the stage to fill is free
+        if (ahead.seg < seg_end) {
+            issue(ahead, fill);
+            advance(ahead);
+        }
+        copy_commit();
+        fill = fill + 1 == P::kStages ? 0 : fill + 1;
+        const double* vs = reinterpret_cast<const double*>(ring + stage * P::kStage) + (lane & 3) * P::kRowLen + (lane >> 2);
+        const V* fs = reinterpret_cast<const V*>(ring + stage * P::kStage + P::kVecs * 8) + lane;
+        const int n = min(P::kChunk, cur.len - cur.j), ks = (3 * n + 3) / 4;
+#pragma unroll
+        for (int s = 0; s < P::kSteps; ++s) {
+            if (s >= ks) break;
+            double a[3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) a[i] = (double)fs[(3 * s + i) * 32];
+#pragma unroll
+            for (int h = 0; h < T; ++h)
+#pragma unroll
+                for (int q = 0; q < NT; ++q) {
+                    const double b = vs[(4 * s + 3 * (T - 1 - h)) * P::kRowLen + 8 * q];
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) mma_f64(acc[i][q][h][0], acc[i][q][h][1], a[i], b);
+                }
+        }
+        advance(cur);
+        stage = stage + 1 == P::kStages ? 0 : stage + 1;
+    }
+    copy_wait<0>();
+    __syncthreads();
+    // the warps' sums; then, summed over them, with this CTA's share of the
+    // KnownM terms of the T steps: [h][row component][case]
+    double* const red = dsm;
+    double* const sums = dsm + NW * P::kSums;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int h = 0; h < T; ++h)
+                *reinterpret_cast<double2*>(red + w * P::kSums + (h * 24 + 8 * i + (lane >> 2)) * R + 8 * q + 2 * (lane & 3)) =
+                    make_double2(acc[i][q][h][0], acc[i][q][h][1]);
+    __syncthreads();
+    for (int t = threadIdx.x; t < P::kSums; t += P::kThreads) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) s += red[q * P::kSums + t];
+        sums[t] = s;
+    }
+    __syncthreads();
+    const int32_t* rows = d.hg_rows + (int64_t)group * 8;
+#pragma unroll 1
+    for (int i = mine; i < 8 * T; i += seg_step) {
+        const int p = __ldg(rows + i % 8), h = i / 8;
+        if (p < 0 || t0 + h > d.nstep) continue;
+        double ka[3];
+        known_share<R, 1>(d, d.row_of[p], t0 + h, 0, lane, ka);
+        if (lane < R)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) sums[(h * 24 + 3 * (i % 8) + c) * R + lane] += ka[c];
+    }
+    if (split > 1) cluster_barrier();
+    else __syncthreads();
+    const int64_t E3R = 3LL * d.E * R;
+    // each CTA adds up and writes its share of the group's sums
+    for (int t = rank * P::kThreads + threadIdx.x; t < P::kSums; t += split * P::kThreads) {
+        const int h = t / (24 * R), m = t / R % 24, r = t % R, p = __ldg(rows + m / 3);
+        if (p < 0 || t0 + h > d.nstep) continue;
+        double s = 0.0;
+        for (int q = 0; q < split; ++q) {
+            double v;
+            peer_load1(peer_addr(shared_addr(sums + t), (uint32_t)q), v);
+            s += v;
+        }
+        d.bulk[(int64_t)((t0 + h) & 7) * E3R + (int64_t)(3 * p + m % 3) * R + r] = s;
+    }
+    if (split > 1) cluster_barrier();  // peers still read this CTA's sums
+}
+
 // Copy one model's MarchData into shared memory (several models per launch).
 __device__ __forceinline__ void load_model(const MarchData* ds, int m, MarchData& sd)
 {
@@ -582,12 +826,12 @@ size_t gmres_caches(MarchData& d, size_t room, int Rg, bool mixed)
     return used + vec * (size_t)d.vcap;
 }
 
-// Raises a kernel's dynamic shared memory to the most the device allows and
-// lets it run in clusters of 16, once per device: changing attributes between
+// Raises a kernel's dynamic shared memory to the most the device allows and,
+// `clusters`, lets it run in clusters of 16, once per device: changing attributes between
 // launches (models of different sizes marched side by side) would be a
 // host-side attribute change per launch.  Returns that size in cap.
 template <class K>
-cudaError_t gmres_attributes(K kernel, std::atomic<int> (&dyn_max)[kMaxDevices], int& cap)
+cudaError_t kernel_attributes(K kernel, std::atomic<int> (&dyn_max)[kMaxDevices], int& cap, bool clusters = true)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -601,7 +845,9 @@ cudaError_t gmres_attributes(K kernel, std::atomic<int> (&dyn_max)[kMaxDevices],
     if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
     cap = optin - (int)fa.sharedSizeBytes;
     if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+    if (clusters &&
+        (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+        return e;
     dyn_max[dev].store(cap);
     return cudaSuccess;
 }
@@ -612,7 +858,7 @@ cudaError_t launch_gmres_form(const MarchData& d0, int step, cudaStream_t s)
     MarchData d = d0;
     static std::atomic<int> dyn_max[kMaxDevices];
     int cap = 0;
-    cudaError_t e = gmres_attributes(gmres_cluster_kernel<R, kMixed, kLocal>, dyn_max, cap);
+    cudaError_t e = kernel_attributes(gmres_cluster_kernel<R, kMixed, kLocal>, dyn_max, cap);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(d.cluster * d.groups);
@@ -701,9 +947,36 @@ cudaError_t launch_rhs(const MarchData& d, int step, bool bulk, int add_bulk, cu
 // bar and kept out: staging the history vectors and block values through
 // shared memory with cp.async (72% more instructions, 1.5x slower) and L1
 // prefetches of the coming vectors (slower at every distance tried).
+template <int R, int T, class V>
+cudaError_t launch_bulk_groups(const MarchData& d, int t0, cudaStream_t s)
+{
+    using P = GroupPass<R, T, V>;
+    static std::atomic<int> dyn_max[kMaxDevices];
+    int cap = 0;
+    const cudaError_t e = kernel_attributes(bulk_groups_kernel<R, T, V>, dyn_max, cap, false);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(d.hg_n * d.hg_split);
+    cfg.blockDim = dim3(P::kThreads);
+    cfg.dynamicSmemBytes = P::kBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = d.hg_split;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, bulk_groups_kernel<R, T, V>, d, t0, d.hg_split);
+}
+
 template <int R, bool kMixed>
 cudaError_t launch_bulk_steps(const MarchData& d, int t0, cudaStream_t s)
 {
+    if constexpr (R >= 8) {
+        using V = typename std::conditional<kMixed, float, double>::type;
+        if (d.hg_n > 0) return d.kr >= 7 ? launch_bulk_groups<R, 3, V>(d, t0, s) : launch_bulk_groups<R, 2, V>(d, t0, s);
+    }
     constexpr int kC = R >= 2 ? 2 : 1;
     if (d.kr >= 7) bulk_steps_kernel<R, kMixed, kC, 3><<<d.E, kRhsThreads, 0, s>>>(d, t0);
     else bulk_steps_kernel<R, kMixed, kC, 2><<<d.E, kRhsThreads, 0, s>>>(d, t0);
@@ -950,8 +1223,8 @@ cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models,
     if (e != cudaSuccess) return e;
     static std::atomic<int> dyn_max[2][kMaxDevices];
     int cap = 0;
-    e = local ? gmres_attributes(gmres_models_kernel<R, kMixed, true>, dyn_max[1], cap)
-              : gmres_attributes(gmres_models_kernel<R, kMixed, false>, dyn_max[0], cap);
+    e = local ? kernel_attributes(gmres_models_kernel<R, kMixed, true>, dyn_max[1], cap)
+              : kernel_attributes(gmres_models_kernel<R, kMixed, false>, dyn_max[0], cap);
     if (e != cudaSuccess) return e;
     if (gmres_dsm > (size_t)cap) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};

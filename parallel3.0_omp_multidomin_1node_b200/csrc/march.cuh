@@ -49,6 +49,17 @@ struct MarchData {
     const float* r_val32;   // SoA [9][r_nb] (mixed)
     int64_t r_nb;
     int kr;
+    // group layout of the same blocks, instead of the run layout when there are
+    // groups (8 or more load cases): per group of 8 rows, segments of one (type,
+    // column) pair over consecutive steps, longest first; a segment of n steps is
+    // a 24 x 3n matrix (zero where a row has no block) in fragments of 8 x 4:
+    // [ceil(3n / 4)][3][lane]
+    int hg_n, hg_split;     // groups, CTAs per group
+    const int64_t* hg_ptr;  // [hg_n+1] first segment of each group
+    const uint2* hg_meta;   // x = (type << 20) | column, y = (first step << 16) | length
+    const int64_t* hg_off;  // first of each segment's ceil(3n / 4) contraction steps
+    const void* hg_val;     // [contraction step][3][32], FP32 (mixed) or FP64
+    const int32_t* hg_rows; // [hg_n][8] perm rows, -1 past the end
     // KnownM (natural rows), known blocks map to (element, sign)
     const int32_t* k_rp;
     const int32_t* k_col;
@@ -177,6 +188,24 @@ cudaError_t build_history_runs(int E, int K, int kr, const std::vector<int64_t>&
                                cudaStream_t s);
 // Device memory the build takes at most for nb blocks (outputs included).
 size_t history_runs_bytes(int64_t nb, bool mixed);
+
+// Group layout of the same blocks (MarchData hg_*): place[row] = group * 8 + slot
+// of every equation row.  Left empty (kr = 0) when the sizes exceed the sort's
+// indices or the blocks fill less than kGroupFillMin of the matrices.
+struct HistoryGroups {
+    int64_t* ptr = nullptr;   // [groups+1]
+    uint2* meta = nullptr;    // [segments]
+    int64_t* off = nullptr;   // [segments]
+    void* val = nullptr;      // [steps][3][32]
+    int64_t steps = 0, segments = 0;  // contraction steps
+    int kr = 0;
+};
+constexpr double kGroupFillMin = 0.4;
+constexpr int kGroupRows = 8;
+cudaError_t build_history_groups(int E, int K, int kr, const std::vector<int32_t>& place, int groups,
+                                 const std::vector<int64_t>& kptr, const int64_t* d_kptr, const uint32_t* d_col,
+                                 const void* d_val, int64_t nnz, bool mixed, HistoryGroups& out, cudaStream_t s);
+size_t history_groups_bytes(int64_t nb, bool mixed);
 
 // Sizes of the R template instantiations.
 bool march_supported_loads(int R);

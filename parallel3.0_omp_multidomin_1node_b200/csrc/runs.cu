@@ -13,6 +13,12 @@
 // k >= kr by (row, type, column, k), cut runs where the pair changes or k
 // jumps, order each row's runs longest first (so the lane groups of one warp
 // walk runs of similar length), and gather the block values into that order.
+//
+// The group layout (8 or more load cases) does the same for groups of
+// neighbouring rows of one domain, whose waves arrive at about the same steps:
+// a segment is one (type, column) pair over the steps in which any of the rows
+// has a block, a matrix of the rows' blocks in the tensor path's fragments, so
+// one history vector serves all the rows.
 #include "march.cuh"
 
 #include <climits>
@@ -110,6 +116,99 @@ __global__ void run_gather_kernel(int n_runs, int64_t nb, int64_t nnz, const int
         const int64_t src = idx[q + t];
 #pragma unroll
         for (int c = 0; c < 9; ++c) out[c * nb + o + t] = val[c * nnz + src];
+    }
+}
+
+// As run_keys_kernel for groups of rows: key place / 8 << 35 | type << 34 |
+// column << 14 | k << 3 | place % 8, so a group's blocks of one (type, column)
+// come together, steps ascending.
+__global__ void group_keys_kernel(int E, int K, int kr, const int32_t* __restrict__ place,
+                                  const int64_t* __restrict__ kptr, const int64_t* __restrict__ qoff,
+                                  const uint32_t* __restrict__ col, unsigned long long* __restrict__ key,
+                                  uint32_t* __restrict__ idx)
+{
+    const int r = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (r >= E) return;
+    const int64_t beg = kptr[(int64_t)r * (K + 1) + kr - 1], end = kptr[(int64_t)r * (K + 1) + K];
+    const int64_t q0 = qoff[r] - beg;
+    const unsigned long long g = (unsigned)(place[r] / kGroupRows), slot = (unsigned)(place[r] % kGroupRows);
+    for (int64_t i = beg + lane; i < end; i += 32) {
+        const uint32_t cp = col[i];
+        const unsigned long long k = cp >> 21, type = (cp >> 20) & 1u, c = cp & 0xFFFFFu;
+        key[q0 + i] = (g << 35) | (type << 34) | (c << 14) | (k << 3) | slot;
+        idx[q0 + i] = (uint32_t)i;
+    }
+}
+
+// 1 where sorted block q starts a segment: a new (group, type, column) or a
+// step past the next one
+__global__ void group_flags_kernel(int64_t nb, const unsigned long long* __restrict__ key, int* __restrict__ flag)
+{
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < nb; q += (int64_t)gridDim.x * blockDim.x) {
+        const unsigned long long a = key[q];
+        int f = 1;
+        if (q > 0) {
+            const unsigned long long b = key[q - 1];
+            f = (b >> 14) != (a >> 14) || ((a >> 3) & 0x7FFull) > ((b >> 3) & 0x7FFull) + 1;
+        }
+        flag[q] = f;
+    }
+}
+
+// order key of segment j: group << 16 | (0xFFFF - length in steps); counts the
+// group's segments
+__global__ void group_order_keys_kernel(int n_segs, int64_t nb, const int* __restrict__ start,
+                                        const unsigned long long* __restrict__ key,
+                                        unsigned long long* __restrict__ okey, int* __restrict__ oval,
+                                        int* __restrict__ group_count)
+{
+    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n_segs; j += gridDim.x * blockDim.x) {
+        const int q = start[j], e = (j + 1 < n_segs ? start[j + 1] : (int)nb) - 1;
+        const int len = (int)((key[e] >> 3) & 0x7FFull) - (int)((key[q] >> 3) & 0x7FFull) + 1;
+        const unsigned long long g = key[q] >> 35;
+        okey[j] = (g << 16) | (unsigned long long)(0xFFFF - len);
+        oval[j] = j;
+        atomicAdd(group_count + g, 1);
+    }
+}
+
+// contraction steps of n history steps
+__global__ void group_steps_kernel(int n_segs, const unsigned long long* __restrict__ okey, int64_t* __restrict__ steps)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_segs; i += gridDim.x * blockDim.x)
+        steps[i] = (3 * (0xFFFF - (int64_t)(okey[i] & 0xFFFFull)) + 3) / 4;
+}
+
+// one warp per segment (in final order): header, then its blocks to their
+// places in the fragments (which start at zero): entry (3 slot + i, 3 (k - k0) +
+// j) of the segment's matrix
+template <class V>
+__global__ void group_scatter_kernel(int n_segs, int64_t nb, int64_t nnz, const int* __restrict__ order,
+                                     const int* __restrict__ start, const unsigned long long* __restrict__ okey,
+                                     const int64_t* __restrict__ off, const unsigned long long* __restrict__ key,
+                                     const uint32_t* __restrict__ idx, const V* __restrict__ val,
+                                     uint2* __restrict__ meta, int64_t* __restrict__ s_off, V* __restrict__ out)
+{
+    const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (i >= n_segs) return;
+    const int j = order[i], q = start[j], e = j + 1 < n_segs ? start[j + 1] : (int)nb;
+    const int64_t o = off[i];
+    const unsigned long long a = key[q];
+    const int k0 = (int)((a >> 3) & 0x7FFull);
+    if (lane == 0) {
+        meta[i] = make_uint2((unsigned)((a >> 34) & 1u) << 20 | (unsigned)((a >> 14) & 0xFFFFFu),
+                             ((unsigned)k0 << 16) | (unsigned)(0xFFFF - (okey[i] & 0xFFFFull)));
+        s_off[i] = o;
+    }
+    for (int t = q + lane; t < e; t += 32) {
+        const unsigned long long b = key[t];
+        const int step = (int)((b >> 3) & 0x7FFull) - k0, slot = (int)(b & 7u);
+        const int64_t src = idx[t];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) {
+            const int m = 3 * slot + c / 3, kk = 3 * step + c % 3;
+            out[((o + kk / 4) * 3 + m / 8) * 32 + (m % 8) * 4 + kk % 4] = val[c * nnz + src];
+        }
     }
 }
 
@@ -286,6 +385,144 @@ cudaError_t build_history_runs(int E, int K, int kr, const std::vector<int64_t>&
     RUN_TRY(cudaStreamSynchronize(s));
     out.nb = nb;
     out.runs = n_runs;
+    out.kr = kr;
+    return cudaSuccess;
+}
+
+size_t history_groups_bytes(int64_t nb, bool mixed)
+{
+    // per block: sort keys and indices (double-buffered), flags, segment ids and
+    // the radix sort's scratch; per segment (about 70 blocks; counted as 16)
+    // start, order keys and values (double-buffered), length, offset, header;
+    // the matrices at the least fill accepted
+    const size_t per_block = 2 * 8 + 2 * 4 + 4 + 4 + 16, per_seg = 4 + 2 * 8 + 2 * 4 + 8 + 8 + 8 + 8;
+    return (size_t)nb * per_block + (size_t)((double)nb * 9.0 * (mixed ? sizeof(float) : sizeof(double)) / kGroupFillMin) +
+           (size_t)nb / 16 * per_seg;
+}
+
+cudaError_t build_history_groups(int E, int K, int kr, const std::vector<int32_t>& place, int groups,
+                                 const std::vector<int64_t>& kptr, const int64_t* d_kptr, const uint32_t* d_col,
+                                 const void* d_val, int64_t nnz, bool mixed, HistoryGroups& out, cudaStream_t s)
+{
+    out = HistoryGroups{};
+    if (kr < 1 || kr > K) return cudaSuccess;
+    std::vector<int64_t> qoff(E + 1, 0);
+    for (int r = 0; r < E; ++r)
+        qoff[r + 1] = qoff[r] + kptr[(size_t)r * (K + 1) + K] - kptr[(size_t)r * (K + 1) + kr - 1];
+    const int64_t nb = qoff[E];
+    if (nb <= 0 || nb > INT_MAX || nnz >= (int64_t)UINT_MAX) return cudaSuccess;
+    const int n = (int)nb;
+    Tmp d_qoff, d_place, k1, k2, i1, i2, flag, segid;
+    RUN_TRY(d_qoff.alloc(sizeof(int64_t) * (E + 1)));
+    RUN_TRY(cudaMemcpyAsync(d_qoff.p, qoff.data(), sizeof(int64_t) * (E + 1), cudaMemcpyHostToDevice, s));
+    RUN_TRY(d_place.alloc(sizeof(int32_t) * E));
+    RUN_TRY(cudaMemcpyAsync(d_place.p, place.data(), sizeof(int32_t) * E, cudaMemcpyHostToDevice, s));
+    RUN_TRY(k1.alloc(8 * (size_t)nb));
+    RUN_TRY(k2.alloc(8 * (size_t)nb));
+    RUN_TRY(i1.alloc(4 * (size_t)nb));
+    RUN_TRY(i2.alloc(4 * (size_t)nb));
+    group_keys_kernel<<<(E + 7) / 8, 256, 0, s>>>(E, K, kr, d_place.as<int32_t>(), d_kptr, d_qoff.as<int64_t>(),
+                                                 d_col, k1.as<unsigned long long>(), i1.as<uint32_t>());
+    RUN_TRY(cudaGetLastError());
+    const int end_bit = 35 + bits_for((unsigned long long)groups);
+    size_t bytes = 0;
+    RUN_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, k1.as<unsigned long long>(), k2.as<unsigned long long>(),
+                                            i1.as<uint32_t>(), i2.as<uint32_t>(), n, 0, end_bit, s));
+    {
+        Tmp temp;
+        RUN_TRY(temp.alloc(bytes));
+        RUN_TRY(cub::DeviceRadixSort::SortPairs(temp.p, bytes, k1.as<unsigned long long>(),
+                                                k2.as<unsigned long long>(), i1.as<uint32_t>(), i2.as<uint32_t>(), n,
+                                                0, end_bit, s));
+    }
+    RUN_TRY(flag.alloc(4 * (size_t)nb));
+    RUN_TRY(segid.alloc(4 * (size_t)nb));
+    group_flags_kernel<<<1184, 256, 0, s>>>(nb, k2.as<unsigned long long>(), flag.as<int>());
+    RUN_TRY(cudaGetLastError());
+    RUN_TRY(cub::DeviceScan::InclusiveSum(nullptr, bytes, flag.as<int>(), segid.as<int>(), n, s));
+    {
+        Tmp temp;
+        RUN_TRY(temp.alloc(bytes));
+        RUN_TRY(cub::DeviceScan::InclusiveSum(temp.p, bytes, flag.as<int>(), segid.as<int>(), n, s));
+    }
+    int n_segs = 0;
+    RUN_TRY(cudaMemcpyAsync(&n_segs, segid.as<int>() + (nb - 1), sizeof(int), cudaMemcpyDeviceToHost, s));
+    RUN_TRY(cudaStreamSynchronize(s));
+    k1.release();  // not needed past the sort
+    i1.release();
+    Tmp start, okey1, okey2, ov1, ov2, lens, offs, gcnt, gptr;
+    RUN_TRY(start.alloc(4 * (size_t)n_segs));
+    run_starts_kernel<<<1184, 256, 0, s>>>(nb, flag.as<int>(), segid.as<int>(), start.as<int>());
+    RUN_TRY(cudaGetLastError());
+    RUN_TRY(okey1.alloc(8 * (size_t)n_segs));
+    RUN_TRY(okey2.alloc(8 * (size_t)n_segs));
+    RUN_TRY(ov1.alloc(4 * (size_t)n_segs));
+    RUN_TRY(ov2.alloc(4 * (size_t)n_segs));
+    RUN_TRY(gcnt.alloc(sizeof(int) * (groups + 1)));
+    RUN_TRY(gptr.alloc(sizeof(int) * (groups + 1)));
+    RUN_TRY(cudaMemsetAsync(gcnt.p, 0, sizeof(int) * (groups + 1), s));
+    group_order_keys_kernel<<<1184, 256, 0, s>>>(n_segs, nb, start.as<int>(), k2.as<unsigned long long>(),
+                                                 okey1.as<unsigned long long>(), ov1.as<int>(), gcnt.as<int>());
+    RUN_TRY(cudaGetLastError());
+    const int end2 = 16 + bits_for((unsigned long long)groups);
+    RUN_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, okey1.as<unsigned long long>(),
+                                            okey2.as<unsigned long long>(), ov1.as<int>(), ov2.as<int>(), n_segs, 0,
+                                            end2, s));
+    {
+        Tmp temp;
+        RUN_TRY(temp.alloc(bytes));
+        RUN_TRY(cub::DeviceRadixSort::SortPairs(temp.p, bytes, okey1.as<unsigned long long>(),
+                                                okey2.as<unsigned long long>(), ov1.as<int>(), ov2.as<int>(), n_segs,
+                                                0, end2, s));
+    }
+    RUN_TRY(lens.alloc(8 * (size_t)(n_segs + 1)));
+    RUN_TRY(offs.alloc(8 * (size_t)(n_segs + 1)));
+    RUN_TRY(cudaMemsetAsync(lens.p, 0, 8 * (size_t)(n_segs + 1), s));
+    group_steps_kernel<<<1184, 256, 0, s>>>(n_segs, okey2.as<unsigned long long>(), lens.as<int64_t>());
+    RUN_TRY(cudaGetLastError());
+    RUN_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, lens.as<int64_t>(), offs.as<int64_t>(), n_segs + 1, s));
+    {
+        Tmp temp;
+        RUN_TRY(temp.alloc(bytes));
+        RUN_TRY(cub::DeviceScan::ExclusiveSum(temp.p, bytes, lens.as<int64_t>(), offs.as<int64_t>(), n_segs + 1, s));
+    }
+    RUN_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, gcnt.as<int>(), gptr.as<int>(), groups + 1, s));
+    {
+        Tmp temp;
+        RUN_TRY(temp.alloc(bytes));
+        RUN_TRY(cub::DeviceScan::ExclusiveSum(temp.p, bytes, gcnt.as<int>(), gptr.as<int>(), groups + 1, s));
+    }
+    std::vector<int> hp(groups + 1);
+    int64_t steps = 0;
+    RUN_TRY(cudaMemcpyAsync(hp.data(), gptr.p, sizeof(int) * (groups + 1), cudaMemcpyDeviceToHost, s));
+    RUN_TRY(cudaMemcpyAsync(&steps, offs.as<int64_t>() + n_segs, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    RUN_TRY(cudaStreamSynchronize(s));
+    if ((double)nb * 9.0 < kGroupFillMin * 96.0 * (double)steps) return cudaSuccess;
+    std::vector<int64_t> hp64(hp.begin(), hp.end());
+    RUN_TRY(cudaMalloc(reinterpret_cast<void**>(&out.ptr), sizeof(int64_t) * (groups + 1)));
+    RUN_TRY(cudaMemcpyAsync(out.ptr, hp64.data(), sizeof(int64_t) * (groups + 1), cudaMemcpyHostToDevice, s));
+    RUN_TRY(cudaMalloc(reinterpret_cast<void**>(&out.meta), sizeof(uint2) * (size_t)n_segs));
+    RUN_TRY(cudaMalloc(reinterpret_cast<void**>(&out.off), sizeof(int64_t) * (size_t)n_segs));
+    const size_t val_bytes = (mixed ? sizeof(float) : sizeof(double)) * 96 * (size_t)steps;
+    RUN_TRY(cudaMalloc(&out.val, val_bytes));
+    RUN_TRY(cudaMemsetAsync(out.val, 0, val_bytes, s));
+    const int gb = (int)(((int64_t)n_segs * 32 + 255) / 256);
+    if (mixed)
+        group_scatter_kernel<float><<<gb, 256, 0, s>>>(n_segs, nb, nnz, ov2.as<int>(), start.as<int>(),
+                                                       okey2.as<unsigned long long>(), offs.as<int64_t>(),
+                                                       k2.as<unsigned long long>(), i2.as<uint32_t>(),
+                                                       static_cast<const float*>(d_val), out.meta, out.off,
+                                                       static_cast<float*>(out.val));
+    else
+        group_scatter_kernel<double><<<gb, 256, 0, s>>>(n_segs, nb, nnz, ov2.as<int>(), start.as<int>(),
+                                                        okey2.as<unsigned long long>(), offs.as<int64_t>(),
+                                                        k2.as<unsigned long long>(), i2.as<uint32_t>(),
+                                                        static_cast<const double*>(d_val), out.meta, out.off,
+                                                        static_cast<double*>(out.val));
+    RUN_TRY(cudaGetLastError());
+    RUN_TRY(cudaStreamSynchronize(s));
+    out.steps = steps;
+    out.segments = n_segs;
     out.kr = kr;
     return cudaSuccess;
 }
