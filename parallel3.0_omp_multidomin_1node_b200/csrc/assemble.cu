@@ -2,6 +2,7 @@
 // history block quadrature, block-CCSR compaction, history stacking and the
 // mapped-leaf preconditioner inverses.
 #include "assemble.cuh"
+#include "hist_pairs.cuh"
 #include "quad.cuh"
 
 namespace tdbem {
@@ -210,69 +211,6 @@ __device__ uint8_t step0_pair(const QuadRules& q, const MT& M, const QElem& e, c
                     for (int c = 0; c < 3; ++c) out1[r * 3 + c] = 0.0 + sign * blk[c * 3 + r];
                 if (maxabs9(out1) > 1.0e-14) fl |= 4;
             }
-        }
-    }
-    return fl;
-}
-
-// History step k blocks of one pair (AssembleMultiDomainHistoryStep,
-// DBEM1/multidomain.cpp:2329-2378, ComputeT2Block / T1Block / UBlock
-// :1739-1813): acc = MTS (T2 then T1 accumulated), mgs = MGS (U), both
-// transposed and signed; returns flags bit0 MTS, bit1 MGS.  self_t2 is the
-// field element's singular T2 block (used at k <= 1 when s == f).
-template <class MT, class S = typename MT::Scalar>
-__device__ uint8_t history_pair(const QuadRules& q, const MT& M, const QElem& e, const DofRefs& dr, int f, bool self,
-                                const S* self_t2, const double* src, int k, S* acc, S* mgs)
-{
-    const double n = (double)k;
-    const bool self_k = (k <= 1 && self);
-    const int c2 = self_k ? 3 : q_need_cal(M, e.center, e.radius, 2, n, src);
-    const int c1 = q_need_cal(M, e.center, e.radius, 1, n, src);
-    uint8_t fl = 0;
-    S blk[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) acc[i] = 0.0;
-    bool present = false;
-    const double su = dr.hu_sign[f], st = dr.ht_sign[f];
-    if (c2 || c1) {
-        // T2 block
-        if (self_k) {
-            for (int i = 0; i < 9; ++i) blk[i] = self_t2[i];
-        } else if (c2 == 1) {
-            w_int_t_pw(q, M, e, 2, src, n, blk);
-        } else if (c2 == 2) {
-            w_int_t_regular(q, M, e, src, n, blk);
-        }
-        if (c2 && su != 0.0 && admit(blk)) {
-            for (int r = 0; r < 3; ++r)
-                for (int c = 0; c < 3; ++c) acc[r * 3 + c] += su * blk[c * 3 + r];
-            present = true;
-            if (maxabs9(acc) <= 1.0e-14) {
-                present = false;
-                for (int i = 0; i < 9; ++i) acc[i] = 0.0;
-            }
-        }
-        // T1 block
-        if (c1 == 1) w_int_t_pw(q, M, e, 1, src, n, blk);
-        else if (c1 == 2) w_int_t_regular(q, M, e, src, n, blk);
-        if (c1 && su != 0.0 && admit(blk)) {
-            for (int r = 0; r < 3; ++r)
-                for (int c = 0; c < 3; ++c) acc[r * 3 + c] += su * blk[c * 3 + r];
-            present = true;
-            if (maxabs9(acc) <= 1.0e-14) {
-                present = false;
-                for (int i = 0; i < 9; ++i) acc[i] = 0.0;
-            }
-        }
-        if (present) fl |= 1;
-    }
-    if (c1) {
-        if (c1 == 1) w_int_u_pw(q, M, e, src, n, blk);
-        else w_int_u_regular(q, M, e, src, n, blk);
-        if (st != 0.0 && admit(blk)) {
-            for (int r = 0; r < 3; ++r)
-                for (int c = 0; c < 3; ++c) mgs[r * 3 + c] = 0.0 + st * blk[c * 3 + r];
-            if (maxabs9(mgs) > 1.0e-14) fl |= 2;
         }
     }
     return fl;
@@ -516,28 +454,164 @@ __global__ void __launch_bounds__(128) step0_kernel(PairSpace ps, const QuadRule
     if (lane == 0) flags[p] = fl;
 }
 
-// History step k blocks, one warp per pair: slot 0 = MTS, slot 1 = MGS.
-__global__ void __launch_bounds__(128) history_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr,
-                                                      int k, double* blocks, uint8_t* flags)
+// Steps k >= 1 in which a pair's history blocks can be nonzero (its T2 part is
+// active at step k - 1, its T1 and U parts at k; a self pair's singular T2 block
+// counts at k = 1): range[p] = first << 16 | count, up to maxn.  One thread per
+// pair.
+__global__ void history_range_kernel(PairSpace ps, const DynaMat* mats, ElemGeom g, int maxn, uint32_t* range,
+                                     int64_t* slots)
 {
-    __shared__ QuadRules q;
-    load_rules(rules, &q);
-    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (p >= ps.n_pairs) return;
-    const int lane = threadIdx.x & 31;
+    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p > ps.n_pairs) return;
+    if (p == ps.n_pairs) {
+        slots[p] = 0;
+        return;
+    }
     int d, s, f;
     decode_pair(ps, p, d, s, f);
-    const DynaMat& M = c_mats[d];
+    const PairClass cls(mats[d], g.center + 3 * (int64_t)f, g.radius[f], g.node + 3 * (int64_t)s);
+    int first = 0, last = 0;
+    bool before = cls(0) != 0 || s == f;
+    for (int k = 1; k <= maxn; ++k) {
+        const bool now = cls(k) != 0;
+        if (now || before) {
+            if (!first) first = k;
+            last = k;
+        }
+        before = now;
+    }
+    const int n = first ? last - first + 1 : 0;
+    range[p] = ((uint32_t)first << 16) | (uint32_t)n;
+    slots[p] = n;
+}
+
+namespace {
+
+// CTA b's field element and sources: CTAs run over the domains' (chunk of
+// kPairSources sources, field element), fields fastest.
+__device__ __forceinline__ bool pair_cta(const PairSpace& ps, int64_t b, int& d, int& f, int& s0, int& s1)
+{
+    for (d = 0; d < ps.n_domains; ++d) {
+        const int nd = ps.dom_count[d];
+        const int64_t n = (int64_t)nd * ((nd + kPairSources - 1) / kPairSources);
+        if (b < n) {
+            f = ps.dom_begin[d] + (int)(b % nd);
+            s0 = (int)(b / nd) * kPairSources;
+            s1 = min(s0 + kPairSources, nd);
+            s0 += ps.dom_begin[d];
+            s1 += ps.dom_begin[d];
+            return true;
+        }
+        b -= n;
+    }
+    return false;
+}
+
+}  // namespace
+
+int64_t pair_ctas(const PairSpace& ps, const int32_t* dom_count)
+{
+    int64_t n = 0;
+    for (int d = 0; d < ps.n_domains; ++d) n += (int64_t)dom_count[d] * ((dom_count[d] + kPairSources - 1) / kPairSources);
+    return n;
+}
+size_t pair_smem(bool dual)
+{
+    return sizeof(PairTable) + kPairWarps * (dual ? sizeof(PairWarp<QDual>) : sizeof(PairWarp<double>));
+}
+
+// History blocks of every pair and step: step k's at slot[pair] + k - first, two
+// of 9 values (MTS, MGS) and their flags; counts[(row * maxn + k - 1) * 2 + type]
+// (type 1 = MGS) of the blocks kept.  A CTA takes a field element, its warps the
+// sources; only those of rows [r0, r1).  Slots run by rows, from slot0 here; no
+// values are kept without blocks, no counts without counts.  The 2,058-element
+// bar (36 steps): 707 ms -> 27.7 ms.
+__global__ void __launch_bounds__(32 * kPairWarps, 2) history_pairs_kernel(PairSpace ps, const QuadRules* rules,
+                                                                          const DynaMat* mats, ElemGeom g, DofRefs dr,
+                                                                          const uint32_t* range, const int64_t* slot,
+                                                                          int r0, int r1, int64_t slot0, int maxn,
+                                                                          double* blocks, uint8_t* flags, int* counts)
+{
+    extern __shared__ __align__(16) unsigned char pair_sm[];
+    __shared__ DynaMat M;
+    PairTable& tb = *reinterpret_cast<PairTable*>(pair_sm);
+    PairWarp<double>& pw = reinterpret_cast<PairWarp<double>*>(pair_sm + sizeof(PairTable))[threadIdx.x >> 5];
+    int d, f, s0, s1;
+    if (!pair_cta(ps, blockIdx.x, d, f, s0, s1)) return;
+    s0 = max(s0, r0);
+    s1 = min(s1, r1);
+    if (s0 >= s1) return;
     QElem e;
     load_elem(g, f, e);
-    const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
-    double acc[9], mgs[9];
-    const uint8_t fl = history_pair(q, M, e, dr, f, s == f, g.on_t2 + 9 * (int64_t)f, src, k, acc, mgs);
-    if (lane < 9) {
-        blocks[(p * 2 + 0) * 9 + lane] = (fl & 1) ? acc[lane] : 0.0;
-        blocks[(p * 2 + 1) * 9 + lane] = (fl & 2) ? mgs[lane] : 0.0;
+    fill_table(tb, *rules, e.cc);
+    if (threadIdx.x == 0) M = mats[d];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nd = ps.dom_count[d], b = ps.dom_begin[d];
+    const double su = dr.hu_sign[f], st = dr.ht_sign[f];
+    for (int s = s0 + (threadIdx.x >> 5); s < s1; s += kPairWarps) {
+        const int64_t p = ps.pair_off[d] + (int64_t)(s - b) * nd + (f - b);
+        const uint32_t rg = range[p];
+        const int ka = (int)(rg >> 16), n = (int)(rg & 0xFFFFu);
+        if (n == 0) continue;
+        const int64_t o = slot[p] - slot0 - ka;
+        const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+        const double* self_t2 = g.on_t2 + 9 * (int64_t)f;
+        pair_steps(M, tb, pw, e, src, s == f, ka, ka + n - 1,
+                   [&](int k, int c2, int c1, const double* t2, const double* t1, const double* u) {
+                       double mts, mgs;
+                       const int fl = stored_blocks<double>(lane, c2, c1, c2 == 3 ? self_t2 : t2, t1, u, su, st, mts, mgs);
+                       if (blocks && lane < 9 && (fl & 1)) blocks[(o + k) * 18 + lane] = mts;
+                       if (blocks && lane < 9 && (fl & 2)) blocks[(o + k) * 18 + 9 + lane] = mgs;
+                       if (blocks && lane == 0) flags[o + k] = (uint8_t)fl;
+                       if (counts && lane < 2 && (fl & (1 << lane)))
+                           atomicAdd(counts + ((int64_t)s * maxn + k - 1) * 2 + lane, 1);
+                   });
     }
-    if (lane == 0) flags[p] = fl;
+}
+
+// The kept blocks to the stacked layout (MarchData h_*): a warp per (row, step)
+// walks the row's pairs in order of their history columns, MGS_k first, then
+// MTS_k negated; rows [r0, r1).
+__global__ void history_stack_kernel(PairSpace ps, int r0, int r1, int64_t slot0, int K, int64_t nnz,
+                                     const int32_t* domain, const int32_t* order, const int64_t* col_h,
+                                     const uint32_t* range, const int64_t* slot, const double* blocks,
+                                     const uint8_t* flags, const int64_t* kptr, const int* counts, int maxn,
+                                     uint32_t* col, double* val)
+{
+    const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (t >= (int64_t)(r1 - r0) * K) return;
+    const int row = r0 + (int)(t / K), k = (int)(t % K) + 1, d = domain[row], nd = ps.dom_count[d], b = ps.dom_begin[d];
+    const int n1 = counts[((int64_t)row * maxn + k - 1) * 2 + 1], n0 = counts[((int64_t)row * maxn + k - 1) * 2];
+    if (n0 + n1 == 0) return;
+    int64_t at[2] = {kptr[(int64_t)row * (K + 1) + k - 1] + n1, kptr[(int64_t)row * (K + 1) + k - 1]};
+    const int64_t p0 = ps.pair_off[d] + (int64_t)(row - b) * nd;
+    const unsigned below = (1u << lane) - 1u;
+    for (int j0 = 0; j0 < nd; j0 += 32) {
+        const int j = j0 + lane, f = j < nd ? order[b + j] : 0;
+        int fl = 0;
+        int64_t o = 0;
+        if (j < nd) {
+            const uint32_t rg = range[p0 + f - b];
+            const int ka = (int)(rg >> 16), n = (int)(rg & 0xFFFFu);
+            if (k >= ka && k < ka + n) {
+                o = slot[p0 + f - b] - slot0 + k - ka;
+                fl = flags[o];
+            }
+        }
+#pragma unroll
+        for (int type = 0; type < 2; ++type) {
+            const unsigned on = __ballot_sync(0xffffffffu, (fl >> type) & 1);
+            if ((fl >> type) & 1) {
+                const int64_t q = at[type] + __popc(on & below);
+                col[q] = ((uint32_t)k << 21) | ((uint32_t)type << 20) | (uint32_t)col_h[f];
+                const double* src = blocks + o * 18 + 9 * type;
+#pragma unroll
+                for (int c = 0; c < 9; ++c) val[c * nnz + q] = type ? src[c] : -src[c];
+            }
+            at[type] += __popc(on);
+        }
+    }
 }
 
 // Count the blocks each row receives from a pair buffer: mask selects the
@@ -951,58 +1025,75 @@ __global__ void __launch_bounds__(128) grad_step0_kernel(PairSpace ps, const Qua
     }
 }
 
-// History part, one warp per pair over k = 1..K: the stacked -MTS_k
+// History part, one warp per pair over the pair's steps k: the stacked -MTS_k
 // (traction kernel) and MGS_k (displacement kernel) blocks add
 // lam_n^T (-dMTS_k W0 + dMGS_k W1) with the convolution vector the march
 // used at step n >= 2, W_m = [m+1 < n] X_{m+1} + 2 X_m + X_{m-1},
-// m = n - k (X_0 = X_-1 = 0).
-__global__ void __launch_bounds__(128) grad_history_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g,
-                                                           DofRefs dr, const QDual* self_d, GradState gs,
-                                                           double* part)
+// m = n - k (X_0 = X_-1 = 0).  480 elements, 200 steps: about 92 ms with the
+// blocks computed step by step, 10.3 ms.
+__global__ void __launch_bounds__(32 * kPairWarps) grad_history_kernel(PairSpace ps, const QuadRules* rules,
+                                                                       const DynaMatD* mats, ElemGeom g, DofRefs dr,
+                                                                       const uint32_t* range, const QDual* self_d,
+                                                                       GradState gs, double* part)
 {
-    __shared__ QuadRules q;
-    load_rules(rules, &q);
-    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (p >= ps.n_pairs) return;
-    const int lane = threadIdx.x & 31;
-    int d, s, f;
-    decode_pair(ps, p, d, s, f);
-    const DynaMatD& M = c_dmats[d];
+    extern __shared__ __align__(16) unsigned char pair_sm[];
+    __shared__ DynaMatD M;
+    PairTable& tb = *reinterpret_cast<PairTable*>(pair_sm);
+    PairWarp<QDual>& pw = reinterpret_cast<PairWarp<QDual>*>(pair_sm + sizeof(PairTable))[threadIdx.x >> 5];
+    int d, f, s0, s1;
+    if (!pair_cta(ps, blockIdx.x, d, f, s0, s1)) return;
     QElem e;
     load_elem(g, f, e);
-    const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+    fill_table(tb, *rules, e.cc);
+    if (threadIdx.x == 0) M = mats[d];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nd = ps.dom_count[d], b = ps.dom_begin[d];
+    const double su = dr.hu_sign[f], st = dr.ht_sign[f];
     const QDual* self_t2 = self_d + 27 * (int64_t)f + 18;
-    const int64_t hb = gs.col_h[f];
-    const int64_t E3 = 3 * (int64_t)gs.E, X3 = 3 * (int64_t)gs.nh;
-    double ge = 0.0, gu = 0.0;
-    for (int k = 1; k <= gs.K; ++k) {
-        QDual acc[9], mgs[9];
-        const uint8_t fl = history_pair(q, M, e, dr, f, s == f, self_t2, src, k, acc, mgs);
-        if (!fl) continue;
-        for (int n = (k > 2 ? k : 2) + lane; n <= gs.N; n += 32) {
-            const int m = n - k;
-            const double* l = gs.lam + n * E3 + 3 * (int64_t)s;
-            for (int type = 0; type < 2; ++type) {
-                if (!(fl & (1 << type))) continue;
-                const double* xm = gs.xh + ((int64_t)m * 2 + type) * X3 + 3 * hb;
-                double w[3] = {2.0 * xm[0], 2.0 * xm[1], 2.0 * xm[2]};
-                if (m + 1 < n) {
-                    const double* xp = gs.xh + ((int64_t)(m + 1) * 2 + type) * X3 + 3 * hb;
-                    for (int c = 0; c < 3; ++c) w[c] += xp[c];
-                }
-                if (m >= 1) {
-                    const double* xq = gs.xh + ((int64_t)(m - 1) * 2 + type) * X3 + 3 * hb;
-                    for (int c = 0; c < 3; ++c) w[c] += xq[c];
-                }
-                contract_add(type ? mgs : acc, l, w, type ? 1.0 : -1.0, type == 1, ge, gu);
-            }
+    const int64_t hb = gs.col_h[f], E3 = 3 * (int64_t)gs.E, X3 = 3 * (int64_t)gs.nh;
+    for (int s = s0 + (threadIdx.x >> 5); s < s1; s += kPairWarps) {
+        const int64_t p = ps.pair_off[d] + (int64_t)(s - b) * nd + (f - b);
+        const int ka = (int)(range[p] >> 16), cnt = (int)(range[p] & 0xFFFFu);
+        double ge = 0.0, gu = 0.0;
+        if (cnt) {
+            const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+            pair_steps(M, tb, pw, e, src, s == f, ka, ka + cnt - 1,
+                       [&](int k, int c2, int c1, const QDual* t2, const QDual* t1, const QDual* u) {
+                           QDual mts, mgs;
+                           const int fl =
+                               stored_blocks<QDual>(lane, c2, c1, c2 == 3 ? self_t2 : t2, t1, u, su, st, mts, mgs);
+                           if (!fl) return;
+                           if (lane < 9) {
+                               pw.out[lane] = mts;
+                               pw.out[9 + lane] = mgs;
+                           }
+                           __syncwarp();
+                           for (int n = (k > 2 ? k : 2) + lane; n <= gs.N; n += 32) {
+                               const int m = n - k;
+                               const double* l = gs.lam + n * E3 + 3 * (int64_t)s;
+                               for (int type = 0; type < 2; ++type) {
+                                   if (!(fl & (1 << type))) continue;
+                                   const double* xm = gs.xh + ((int64_t)m * 2 + type) * X3 + 3 * hb;
+                                   double w[3] = {2.0 * xm[0], 2.0 * xm[1], 2.0 * xm[2]};
+                                   if (m + 1 < n) {
+                                       const double* xp = gs.xh + ((int64_t)(m + 1) * 2 + type) * X3 + 3 * hb;
+                                       for (int c = 0; c < 3; ++c) w[c] += xp[c];
+                                   }
+                                   if (m >= 1) {
+                                       const double* xq = gs.xh + ((int64_t)(m - 1) * 2 + type) * X3 + 3 * hb;
+                                       for (int c = 0; c < 3; ++c) w[c] += xq[c];
+                                   }
+                                   contract_add(pw.out + 9 * type, l, w, type ? 1.0 : -1.0, type == 1, ge, gu);
+                               }
+                           }
+                       });
         }
-    }
-    ge = qwarp_sum(ge);
-    gu = qwarp_sum(gu);
-    if (lane == 0) {
-        part[2 * p] = ge;
-        part[2 * p + 1] = gu;
+        ge = qwarp_sum(ge);
+        gu = qwarp_sum(gu);
+        if (lane == 0) {
+            part[2 * p] = ge;
+            part[2 * p + 1] = gu;
+        }
     }
 }
 

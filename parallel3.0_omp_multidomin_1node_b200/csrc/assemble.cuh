@@ -75,8 +75,20 @@ __global__ void singular_kernel(int E, const QuadRules* rules, const double* sec
                                 ElemGeom g);
 __global__ void step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr, double* blocks,
                              uint8_t* flags);
-__global__ void history_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr, int k, double* blocks,
-                               uint8_t* flags);
+__global__ void history_range_kernel(PairSpace ps, const DynaMat* mats, ElemGeom g, int maxn, uint32_t* range,
+                                     int64_t* slots);
+__global__ void history_pairs_kernel(PairSpace ps, const QuadRules* rules, const DynaMat* mats, ElemGeom g, DofRefs dr,
+                                     const uint32_t* range, const int64_t* slot, int r0, int r1, int64_t slot0,
+                                     int maxn, double* blocks, uint8_t* flags, int* counts);
+__global__ void history_stack_kernel(PairSpace ps, int r0, int r1, int64_t slot0, int K, int64_t nnz,
+                                     const int32_t* domain, const int32_t* order, const int64_t* col_h,
+                                     const uint32_t* range, const int64_t* slot, const double* blocks,
+                                     const uint8_t* flags, const int64_t* kptr, const int* counts, int maxn,
+                                     uint32_t* col, double* val);
+int64_t pair_ctas(const PairSpace& ps, const int32_t* dom_count);  // CTAs of the pair kernels, and their
+size_t pair_smem(bool dual);                                       // dynamic shared memory
+// out[0..n] = exclusive sum of in[0..n)
+cudaError_t exclusive_sum(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s);
 __global__ void count_rows_kernel(PairSpace ps, const uint8_t* flags, int mask, int E, int* counts);
 __global__ void scatter_rows_kernel(PairSpace ps, const uint8_t* flags, const double* blocks, int mask, int E,
                                     const int64_t* row_start, ScatterCols sc, int32_t* out_col, double* out_val);
@@ -89,8 +101,8 @@ __global__ void history_states_kernel(int N, int E, int nh, const int32_t* hist_
                                       const double* out_lt, double* xh);
 __global__ void grad_step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr, const QDual* self_d,
                                   GradState gs, double* part);
-__global__ void grad_history_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr,
-                                    const QDual* self_d, GradState gs, double* part);
+__global__ void grad_history_kernel(PairSpace ps, const QuadRules* rules, const DynaMatD* mats, ElemGeom g, DofRefs dr,
+                                    const uint32_t* range, const QDual* self_d, GradState gs, double* part);
 __global__ void to_float_kernel(const double* in, float* out, int64_t n);
 __global__ void leaf_inverse_kernel(int n_leaves, const int32_t* leaf_begin, const int32_t* leaf_count,
                                     const int64_t* leaf_off, const int32_t* a_rp, const int32_t* a_col,

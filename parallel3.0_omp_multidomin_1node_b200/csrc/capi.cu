@@ -11,6 +11,7 @@
 #include "tdbem_common.cuh"
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -464,7 +465,7 @@ struct tdbem_handle {
     int rhs_cpt = 0;              // history pass: load cases per thread (0 = the default for R)
     std::vector<int32_t> ap_rp, ap_col;  // A' structure (perm space), for re-laying the GMRES clusters
     // device buffers
-    DevBuf d_rules, d_secpw_pos, d_secpw_val, d_points, d_elements;
+    DevBuf d_mats, d_rules, d_secpw_pos, d_secpw_val, d_points, d_elements;
     DevBuf g_cc, g_center, g_radius, g_rpw, g_rcen, g_node, g_trans, g_u1, g_t1, g_t2, g_bcid, g_domain, g_surface;
     DevBuf d_uref_sign, d_tref_sign, d_hu_sign, d_ht_sign, d_itf_trans, d_uref_block, d_tref_block, d_hist_block;
     DevBuf d_uref_known, d_tref_known, d_hist_owner, d_known_elem, d_known_sign, d_itf_a, d_itf_asign;
@@ -700,6 +701,7 @@ tdbem_status tdbem_md_create(const tdbem_problem* pr, int32_t device, tdbem_hand
     CUDA_TRY(up(h->d_points, h->points, s));
     CUDA_TRY(up(h->d_elements, h->elements, s));
     CUDA_TRY(upload_materials(h->mats.data(), h->D, s));
+    CUDA_TRY(up(h->d_mats, h->mats, s));
     CUDA_TRY(h->g_cc.alloc(E * 24 * 8));
     CUDA_TRY(h->g_center.alloc(E * 3 * 8));
     CUDA_TRY(h->g_radius.alloc(E * 8));
@@ -992,6 +994,170 @@ tdbem_status stack_history(tdbem_handle* h, std::vector<std::vector<int64_t>>& m
     return TDBEM_OK;
 }
 
+// Pair space over the domains, the GlobalDofMap references and the
+// per-field-element column maps of the Step0 and history blocks (device
+// copies), shared by the assembly and the material gradient.
+struct PairSetup {
+    std::vector<int64_t> poff;
+    DevBuf dom_begin, dom_count, pair_off, col_a0, col_a1, col_k, col_h;
+    PairSpace ps{};
+    DofRefs dr{};
+};
+
+tdbem_status pair_setup(tdbem_handle* h, PairSetup& P, cudaStream_t s)
+{
+    const int64_t E = h->E;
+    P.poff.assign(h->D + 1, 0);
+    for (int d = 0; d < h->D; ++d) P.poff[d + 1] = P.poff[d] + (int64_t)h->dom_count[d] * h->dom_count[d];
+    CUDA_TRY(up(P.dom_begin, h->dom_begin, s));
+    CUDA_TRY(up(P.dom_count, h->dom_count, s));
+    CUDA_TRY(up(P.pair_off, P.poff, s));
+    P.ps = PairSpace{h->D, P.poff[h->D], P.dom_begin.as<int32_t>(), P.dom_count.as<int32_t>(),
+                     P.pair_off.as<int64_t>()};
+    P.dr = DofRefs{h->d_uref_sign.as<double>(), h->d_tref_sign.as<double>(), h->d_hu_sign.as<double>(),
+                   h->d_ht_sign.as<double>(), h->d_itf_trans.as<double>()};
+    // A slot 0: the interface element's U unknown or the outer element's
+    // unknown; A slot 1: the interface T unknown; KnownM: the known block
+    std::vector<int64_t> a0(E), a1(E), kc(E), hc(E);
+    for (int64_t i = 0; i < E; ++i) {
+        a0[i] = h->surface[i] ? h->uref_block[i] : (h->bcid[i] == 123 ? h->tref_block[i] : h->uref_block[i]);
+        a1[i] = h->tref_block[i];
+        kc[i] = h->bcid[i] == 123 ? h->uref_block[i] : h->tref_block[i];
+        hc[i] = h->hist_block[i];
+    }
+    CUDA_TRY(up(P.col_a0, a0, s));
+    CUDA_TRY(up(P.col_a1, a1, s));
+    CUDA_TRY(up(P.col_k, kc, s));
+    CUDA_TRY(up(P.col_h, hc, s));
+    return TDBEM_OK;
+}
+
+// Most history steps the pair kernels count (their step numbers are 16-bit); a
+// history this long exceeds the packed column format anyway.
+constexpr int kHistoryStepsMax = 30000;
+
+// History blocks of all steps up to maxn, stacked: each pair's steps, the pairs'
+// blocks, then the rows' blocks in place.  The pairs' blocks (144 bytes a step of
+// a pair, both types side by side) go to a workspace of at most a third of the
+// free memory (TDBEM_HISTORY_SCRATCH bytes), so that the stacked matrix, of about
+// their size, fits beside it.  What needs more is counted first, then computed
+// again over ranges of rows.
+tdbem_status assemble_history(tdbem_handle* h, const PairSetup& P, int maxn, cudaStream_t s)
+{
+    const int E = (int)h->E;
+    const PairSpace ps = P.ps;
+    const ElemGeom g = h->geom();
+    maxn = std::max(maxn, 0);
+    h->K = 0;
+    h->hist_mts_blocks = h->hist_mgs_blocks = 0;
+    DevBuf range, slots, offs, blocks, flags, counts, order;
+    std::vector<int> c(2 * (size_t)E * maxn, 0);
+    std::vector<int64_t> row_slot;      // slots before each row (offs at its first pair)
+    std::vector<std::array<int, 2>> chunks;
+    auto pairs_pass = [&](int r0, int r1, int64_t slot0, bool keep, bool count) -> cudaError_t {
+        history_pairs_kernel<<<(unsigned)pair_ctas(ps, h->dom_count.data()), 256, pair_smem(false), s>>>(
+            ps, h->d_rules.as<QuadRules>(), h->d_mats.as<DynaMat>(), g, P.dr, range.as<uint32_t>(), offs.as<int64_t>(),
+            r0, r1, slot0, maxn, keep ? blocks.as<double>() : nullptr, flags.as<uint8_t>(),
+            count ? counts.as<int>() : nullptr);
+        return cudaGetLastError();
+    };
+    if (maxn > 0) {
+        CUDA_TRY(range.alloc(sizeof(uint32_t) * (size_t)ps.n_pairs));
+        CUDA_TRY(slots.alloc(sizeof(int64_t) * (size_t)(ps.n_pairs + 1)));
+        CUDA_TRY(offs.alloc(sizeof(int64_t) * (size_t)(ps.n_pairs + 1)));
+        history_range_kernel<<<ceil_div(ps.n_pairs + 1, 256), 256, 0, s>>>(ps, h->d_mats.as<DynaMat>(), g, maxn,
+                                                                           range.as<uint32_t>(), slots.as<int64_t>());
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(exclusive_sum(slots.as<int64_t>(), offs.as<int64_t>(), ps.n_pairs + 1, s));
+        slots.release();
+        row_slot.assign((size_t)E + 1, 0);
+        int64_t row_pair = 0;
+        for (int d = 0; d < h->D; ++d) {
+            // a domain's rows start nd pairs apart
+            const int64_t nd = h->dom_count[d];
+            if (nd == 0) continue;
+            CUDA_TRY(cudaMemcpy2DAsync(row_slot.data() + h->dom_begin[d], sizeof(int64_t), offs.as<int64_t>() + row_pair,
+                                       sizeof(int64_t) * nd, sizeof(int64_t), (size_t)nd, cudaMemcpyDeviceToHost, s));
+            row_pair += nd * nd;
+        }
+        CUDA_TRY(cudaMemcpyAsync(&row_slot[E], offs.as<int64_t>() + ps.n_pairs, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+        size_t free_bytes = 0, total_bytes = 0;
+        CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+        int64_t limit = (int64_t)(free_bytes / 3);
+        if (const char* v = std::getenv("TDBEM_HISTORY_SCRATCH")) limit = std::min<int64_t>(limit, std::atoll(v));
+        const int64_t slot_bytes = 18 * sizeof(double) + 1;
+        int64_t most = 1;
+        for (int r = 0; r < E;) {
+            int r1 = r + 1;
+            while (r1 < E && (row_slot[r1 + 1] - row_slot[r]) * slot_bytes <= limit) ++r1;
+            chunks.push_back({r, r1});
+            most = std::max(most, row_slot[r1] - row_slot[r]);
+            r = r1;
+        }
+        CUDA_TRY(blocks.alloc(sizeof(double) * 18 * (size_t)most));
+        CUDA_TRY(flags.alloc((size_t)most));
+        CUDA_TRY(counts.alloc(sizeof(int) * c.size()));
+        CUDA_TRY(cudaMemsetAsync(counts.p, 0, counts.bytes, s));
+        CUDA_TRY(cudaFuncSetAttribute(history_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)pair_smem(false)));
+        CUDA_TRY(pairs_pass(0, E, 0, chunks.size() == 1, true));
+        CUDA_TRY(cudaMemcpyAsync(c.data(), counts.p, counts.bytes, cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    for (int r = 0; r < E; ++r)
+        for (int k = maxn; k > h->K; --k)
+            if (c[2 * ((size_t)r * maxn + k - 1)] + c[2 * ((size_t)r * maxn + k - 1) + 1] > 0) {
+                h->K = k;
+                break;
+            }
+    const int K = h->K;
+    h->h_kptr.assign((size_t)E * (K + 1), 0);
+    int64_t pos = 0;
+    for (int r = 0; r < E; ++r) {
+        h->h_kptr[(size_t)r * (K + 1)] = pos;
+        for (int k = 1; k <= K; ++k) {
+            const int n0 = c[2 * ((size_t)r * maxn + k - 1)], n1 = c[2 * ((size_t)r * maxn + k - 1) + 1];
+            h->hist_mts_blocks += n0;
+            h->hist_mgs_blocks += n1;
+            pos += n0 + n1;
+            h->h_kptr[(size_t)r * (K + 1) + k] = pos;
+        }
+    }
+    h->h_nnz = pos;
+    if (h->n_hist >= (1 << 20) || K >= (1 << 11))
+        return fail(TDBEM_INVALID_INPUT, "history columns or steps exceed the packed column format");
+    CUDA_TRY(up(h->d_h_kptr, h->h_kptr, s));
+    CUDA_TRY(h->d_h_col.alloc(sizeof(uint32_t) * std::max<int64_t>(pos, 1)));
+    CUDA_TRY(h->d_h_val.alloc(sizeof(double) * 9 * std::max<int64_t>(pos, 1)));
+    if (pos > 0) {
+        // each domain's field elements in order of their history columns
+        std::vector<int32_t> by_col((size_t)E);
+        std::iota(by_col.begin(), by_col.end(), 0);
+        for (int d = 0; d < h->D; ++d)
+            std::sort(by_col.begin() + h->dom_begin[d], by_col.begin() + h->dom_begin[d] + h->dom_count[d],
+                      [&](int32_t a, int32_t b) { return h->hist_block[a] < h->hist_block[b]; });
+        CUDA_TRY(up(order, by_col, s));
+        for (const std::array<int, 2>& rows : chunks) {
+            const int64_t slot0 = row_slot[rows[0]];
+            if (chunks.size() > 1) CUDA_TRY(pairs_pass(rows[0], rows[1], slot0, true, false));
+            history_stack_kernel<<<ceil_div((int64_t)(rows[1] - rows[0]) * K, 8), 256, 0, s>>>(
+                ps, rows[0], rows[1], slot0, K, pos, h->g_domain.as<int32_t>(), order.as<int32_t>(),
+                P.col_h.as<int64_t>(), range.as<uint32_t>(), offs.as<int64_t>(), blocks.as<double>(),
+                flags.as<uint8_t>(), h->d_h_kptr.as<int64_t>(), counts.as<int>(), maxn, h->d_h_col.as<uint32_t>(),
+                h->d_h_val.as<double>());
+            CUDA_TRY(cudaGetLastError());
+        }
+        CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    if (h->precision == TDBEM_PRECISION_MIXED) {
+        CUDA_TRY(h->d_h_val32.alloc(sizeof(float) * 9 * std::max<int64_t>(pos, 1)));
+        to_float_kernel<<<1184, 256, 0, s>>>(h->d_h_val.as<double>(), h->d_h_val32.as<float>(), 9 * pos);
+        CUDA_TRY(cudaGetLastError());
+    }
+    return TDBEM_OK;
+}
+
 // Last history step that can hold a nonzero block, from the reference's own
 // skip rule.  A history block of step k integrates the kernels U(k), T1(k)
 // and T2(k) of field element e at source node s of the same domain; each is
@@ -1259,44 +1425,6 @@ FILE* open_diagnostic_csv(const std::string& path, const char* header)
     FILE* f = std::fopen(path.c_str(), "a");
     if (f && fresh) std::fprintf(f, "%s\n", header);
     return f;
-}
-
-// Pair space over the domains, the GlobalDofMap references and the
-// per-field-element column maps of the Step0 and history blocks (device
-// copies), shared by the assembly and the material gradient.
-struct PairSetup {
-    std::vector<int64_t> poff;
-    DevBuf dom_begin, dom_count, pair_off, col_a0, col_a1, col_k, col_h;
-    PairSpace ps{};
-    DofRefs dr{};
-};
-
-tdbem_status pair_setup(tdbem_handle* h, PairSetup& P, cudaStream_t s)
-{
-    const int64_t E = h->E;
-    P.poff.assign(h->D + 1, 0);
-    for (int d = 0; d < h->D; ++d) P.poff[d + 1] = P.poff[d] + (int64_t)h->dom_count[d] * h->dom_count[d];
-    CUDA_TRY(up(P.dom_begin, h->dom_begin, s));
-    CUDA_TRY(up(P.dom_count, h->dom_count, s));
-    CUDA_TRY(up(P.pair_off, P.poff, s));
-    P.ps = PairSpace{h->D, P.poff[h->D], P.dom_begin.as<int32_t>(), P.dom_count.as<int32_t>(),
-                     P.pair_off.as<int64_t>()};
-    P.dr = DofRefs{h->d_uref_sign.as<double>(), h->d_tref_sign.as<double>(), h->d_hu_sign.as<double>(),
-                   h->d_ht_sign.as<double>(), h->d_itf_trans.as<double>()};
-    // A slot 0: the interface element's U unknown or the outer element's
-    // unknown; A slot 1: the interface T unknown; KnownM: the known block
-    std::vector<int64_t> a0(E), a1(E), kc(E), hc(E);
-    for (int64_t i = 0; i < E; ++i) {
-        a0[i] = h->surface[i] ? h->uref_block[i] : (h->bcid[i] == 123 ? h->tref_block[i] : h->uref_block[i]);
-        a1[i] = h->tref_block[i];
-        kc[i] = h->bcid[i] == 123 ? h->uref_block[i] : h->tref_block[i];
-        hc[i] = h->hist_block[i];
-    }
-    CUDA_TRY(up(P.col_a0, a0, s));
-    CUDA_TRY(up(P.col_a1, a1, s));
-    CUDA_TRY(up(P.col_k, kc, s));
-    CUDA_TRY(up(P.col_h, hc, s));
-    return TDBEM_OK;
 }
 
 // One march of one handle, split so that several handles' marches can be
@@ -1668,44 +1796,10 @@ tdbem_status tdbem_md_assemble(tdbem_handle* h, void* stream)
         if (tdbem_status st = history_step_bound(h, s, kb); st != TDBEM_OK) return st;
         maxn = std::min(maxn, kb);
     }
-    std::vector<std::unique_ptr<DevBuf>> keep;
-    std::vector<std::vector<int64_t>> mts_rp, mgs_rp;
-    std::vector<HistK> hk;
-    int last = 0;
-    for (int k = 1; k <= maxn; ++k) {
-        history_kernel<<<ceil_div(ps.n_pairs, warps_per_cta), 32 * warps_per_cta, 0, s>>>(
-            ps, h->d_rules.as<QuadRules>(), g, dr, k, blocks.as<double>(), flags.as<uint8_t>());
-        CUDA_TRY(cudaGetLastError());
-        ScatterCols sh{{0, 1, 1}, {P.col_h.as<int64_t>(), P.col_h.as<int64_t>(), P.col_h.as<int64_t>()}};
-        std::vector<int64_t> rt, rg;
-        auto trp = std::make_unique<DevBuf>(), tcol = std::make_unique<DevBuf>(), tval = std::make_unique<DevBuf>();
-        auto grp = std::make_unique<DevBuf>(), gcol = std::make_unique<DevBuf>(), gval = std::make_unique<DevBuf>();
-        tdbem_status st = compact(h, ps, flags, blocks, 1, sh, rt, *trp, *tcol, *tval, s);
-        if (st != TDBEM_OK) return st;
-        st = compact(h, ps, flags, blocks, 2, sh, rg, *grp, *gcol, *gval, s);
-        if (st != TDBEM_OK) return st;
-        const bool empty = rt[E] == 0 && rg[E] == 0;
-        if (!empty) last = k;
-        mts_rp.push_back(rt);
-        mgs_rp.push_back(rg);
-        hk.push_back(HistK{trp->as<int64_t>(), tcol->as<int32_t>(), tval->as<double>(), grp->as<int64_t>(),
-                           gcol->as<int32_t>(), gval->as<double>()});
-        keep.push_back(std::move(trp));
-        keep.push_back(std::move(tcol));
-        keep.push_back(std::move(tval));
-        keep.push_back(std::move(grp));
-        keep.push_back(std::move(gcol));
-        keep.push_back(std::move(gval));
-    }
-    h->K = last;
-    mts_rp.resize(last);
-    mgs_rp.resize(last);
-    hk.resize(last);
     blocks.release();
     flags.release();
-    tdbem_status st = stack_history(h, mts_rp, mgs_rp, hk, s);
+    tdbem_status st = assemble_history(h, P, std::min(maxn, kHistoryStepsMax), s);
     if (st != TDBEM_OK) return st;
-    keep.clear();  // the per-step matrices, before the run layout takes its memory
     if ((st = build_runs(h, s)) != TDBEM_OK) return st;
     const tdbem_status done = finish_setup(h, s);
     h->assembly_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
@@ -3095,6 +3189,8 @@ tdbem_status material_gradient(tdbem_handle* h, cudaStream_t s, double* grad)
     std::vector<DynaMatD> dm;
     for (const DynaMat& m : h->mats) dm.push_back(build_mat_dual(m));
     CUDA_TRY(upload_materials_dual(dm.data(), (int)dm.size(), s));
+    DevBuf d_dm, range, slots;
+    CUDA_TRY(up(d_dm, dm, s));
     PairSetup P;
     if (tdbem_status st = pair_setup(h, P, s); st != TDBEM_OK) return st;
     const int64_t np = P.ps.n_pairs;
@@ -3130,6 +3226,13 @@ tdbem_status material_gradient(tdbem_handle* h, cudaStream_t s, double* grad)
                        P.col_k.as<int64_t>(),
                        P.col_h.as<int64_t>()};
     std::fill(grad, grad + 2 * (size_t)h->D, 0.0);
+    // history steps 1..K of each pair
+    CUDA_TRY(range.alloc(sizeof(uint32_t) * (size_t)std::max<int64_t>(np, 1)));
+    CUDA_TRY(slots.alloc(sizeof(int64_t) * (size_t)(np + 1)));
+    history_range_kernel<<<ceil_div(np + 1, 256), 256, 0, s>>>(P.ps, h->d_mats.as<DynaMat>(), g, h->K,
+                                                               range.as<uint32_t>(), slots.as<int64_t>());
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaFuncSetAttribute(grad_history_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(true)));
     std::vector<double> pv;
     const int warps = 4;
     for (int pass = 0; pass < 2 && np > 0; ++pass) {
@@ -3137,8 +3240,9 @@ tdbem_status material_gradient(tdbem_handle* h, cudaStream_t s, double* grad)
             grad_step0_kernel<<<ceil_div(np, warps), 32 * warps, 0, s>>>(P.ps, h->d_rules.as<QuadRules>(), g, P.dr,
                                                                          self_d.as<QDual>(), gs, part.as<double>());
         else
-            grad_history_kernel<<<ceil_div(np, warps), 32 * warps, 0, s>>>(P.ps, h->d_rules.as<QuadRules>(), g, P.dr,
-                                                                           self_d.as<QDual>(), gs, part.as<double>());
+            grad_history_kernel<<<(unsigned)pair_ctas(P.ps, h->dom_count.data()), 256, pair_smem(true), s>>>(
+                P.ps, h->d_rules.as<QuadRules>(), d_dm.as<DynaMatD>(), g, P.dr, range.as<uint32_t>(), self_d.as<QDual>(),
+                gs, part.as<double>());
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(download(pv, part, 2 * (size_t)np, s));
         CUDA_TRY(cudaStreamSynchronize(s));

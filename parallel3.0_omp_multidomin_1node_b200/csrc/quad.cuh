@@ -449,26 +449,4 @@ __device__ __forceinline__ void w_int_t_pw(const QuadRules& q, const MT& M, cons
     for (int i = 0; i < 9; ++i) out[i] = qwarp_sum(c[i]);
 }
 
-// IntDynaUijJudge / IntDynaTijJudge(typeT, ..., T_ID)
-// (DBEM1/dsquareelementdyna.cpp:1603-1616, 1677-1690)
-template <class MT, class S = typename MT::Scalar>
-__device__ __forceinline__ int w_judge_u(const QuadRules& q, const MT& M, const QElem& e, const double* src,
-                                         double n, S* out)
-{
-    const int f = q_need_cal(M, e.center, e.radius, 1, n, src);
-    if (f == 1) w_int_u_pw(q, M, e, src, n, out);
-    else if (f == 2) w_int_u_regular(q, M, e, src, n, out);
-    return f;
-}
-
-template <class MT, class S = typename MT::Scalar>
-__device__ __forceinline__ int w_judge_t(const QuadRules& q, const MT& M, const QElem& e, int type,
-                                         const double* src, double n, S* out)
-{
-    const int f = q_need_cal(M, e.center, e.radius, type, n, src);
-    if (f == 1) w_int_t_pw(q, M, e, type, src, n, out);
-    else if (f == 2) w_int_t_regular(q, M, e, src, n, out);
-    return f;
-}
-
 }  // namespace tdbem

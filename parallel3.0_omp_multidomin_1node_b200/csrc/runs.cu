@@ -19,6 +19,7 @@
 // a segment is one (type, column) pair over the steps in which any of the rows
 // has a block, a matrix of the rows' blocks in the tensor path's fragments, so
 // one history vector serves all the rows.
+#include "assemble.cuh"
 #include "march.cuh"
 
 #include <climits>
@@ -387,6 +388,15 @@ cudaError_t build_history_runs(int E, int K, int kr, const std::vector<int64_t>&
     out.runs = n_runs;
     out.kr = kr;
     return cudaSuccess;
+}
+
+cudaError_t exclusive_sum(const int64_t* in, int64_t* out, int64_t n, cudaStream_t s)
+{
+    size_t bytes = 0;
+    RUN_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, s));
+    Tmp temp;
+    RUN_TRY(temp.alloc(bytes));
+    return cub::DeviceScan::ExclusiveSum(temp.p, bytes, in, out, n, s);
 }
 
 size_t history_groups_bytes(int64_t nb, bool mixed)
