@@ -851,14 +851,27 @@ void bisect_rows(const std::vector<double>& node, int32_t* b, int32_t* e, int G)
     bisect_rows(node, m, e, G);
 }
 
+// One load case takes the T-step pass over the step-major matrices from this
+// size on, the L2's: what fits there the one-step pass reads fast enough to hide
+// beside GMRES, and the longer head costs more than it saves.  Steps of bars
+// with one load case, one-step -> T = 2: 0.02 GB 86.9 -> 88.2 us, 0.19 GB 129.6 ->
+// 126.8, 0.44 GB 145.4 -> 143.2, 0.82 GB 197.8 -> 188.7, 1.68 GB 339 -> 218.
+constexpr double kRowsPassBytes = 126e6;
+double history_bytes(const tdbem_handle* h)
+{
+    return (double)h->h_nnz * (h->precision == TDBEM_PRECISION_MIXED ? 40.0 : 76.0);
+}
+
 // Run layout of the history steps k >= 2T + 1 for the T-step history pass
-// (two or more load cases; T = 2, or 3 with TDBEM_HISTORY_STEPS=3 and at
+// (two or more load cases; one reads the step-major matrices, always with
+// TDBEM_RUNS=2; T = 2, or 3 with TDBEM_HISTORY_STEPS=3 and at
 // least 7 history steps; off with TDBEM_RUNS=0).  Left out, and the march
 // keeps the one-step pass, when the build would not fit in free device
 // memory.  On the 3,072-element bar with 32 load cases T = 3 makes the
 // history pass 15% faster but doubles the head pass on the GMRES chain
 // (k <= 6): the march is 1% faster in mixed precision and 7% slower in FP64,
 // so T = 2 is the default.
+
 tdbem_status build_runs(tdbem_handle* h, cudaStream_t s)
 {
     int steps = 2;
@@ -874,9 +887,16 @@ tdbem_status build_runs(tdbem_handle* h, cudaStream_t s)
     h->r_nb = h->r_runs = h->hg_steps = h->hg_segs = 0;
     h->run_k = h->hg_n = 0;
     const int E = (int)h->E, K = h->K;
-    if (K < kRunK || h->R < 2 || h->h_nnz == 0) return TDBEM_OK;
-    if (const char* v = std::getenv("TDBEM_RUNS"))
+    if (K < kRunK || h->h_nnz == 0) return TDBEM_OK;
+    bool forced = false;
+    if (const char* v = std::getenv("TDBEM_RUNS")) {
         if (std::atoi(v) == 0) return TDBEM_OK;
+        forced = std::atoi(v) == 2;
+    }
+    if (h->R == 1) {
+        if (forced || history_bytes(h) >= kRowsPassBytes) h->run_k = kRunK;
+        return TDBEM_OK;
+    }
     int64_t nb = 0;
     for (int r = 0; r < E; ++r)
         nb += h->h_kptr[(size_t)r * (K + 1) + K] - h->h_kptr[(size_t)r * (K + 1) + kRunK - 1];
@@ -1660,7 +1680,7 @@ struct MarchRun {
                         // distinct W slots: t0 + h - k over the launch's (h, k)
                         const int slots = (t0 + T - 1 - kr) - std::max(t0 - klast, 0) + 1;
                         const int steps_out = std::min(T, N - t0 + 1);
-                        hb = (double)(cum[klast] - cum[kr - 1]) * 9.0 * vs +
+                        hb = (double)(cum[klast] - cum[kr - 1]) * (9.0 * vs + (R == 1 ? 4.0 : 0.0)) +
                              (double)(h->hg_n ? h->hg_segs : h->r_runs) * 16.0 +
                              std::max(slots, 0) * slot_b + (double)E * 24.0 * R * steps_out + steps_out * known_b;
                         for (int hh = 0; hh < T; ++hh)
@@ -1668,7 +1688,8 @@ struct MarchRun {
                                 (double)std::max<int64_t>(cum[std::min(t0 + hh, K)] - cum[kr - 1], 0);
                         // (groups: the full history's count from the first pass on)
                         rep.history_vector_loads +=
-                            h->hg_n ? (double)h->hg_steps * 4.0 / 3.0 + (double)(T - 1) * h->hg_segs
+                            R == 1    ? (double)T * std::max<int64_t>(cum[std::min(t0, K)] - cum[kr - 1], 0)
+                            : h->hg_n ? (double)h->hg_steps * 4.0 / 3.0 + (double)(T - 1) * h->hg_segs
                                   : (double)(cum[std::min(t0, K)] > cum[kr - 1] ? cum[std::min(t0, K)] - cum[kr - 1] : 0) +
                                         (double)(T - 1) * h->r_runs;
                         ++rep.history_launches;

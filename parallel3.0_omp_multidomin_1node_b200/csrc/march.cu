@@ -423,6 +423,93 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
     }
 }
 
+// The same part of the right-hand sides for one load case, over the step-major
+// matrices of the one-step pass: each block is read once for the T steps (a run's
+// blocks lie 8 bytes apart per lane in the run layout, too thin a read where a
+// vector is one load case), with T vectors of 24 bytes from L2, in column order.
+// What bounds it: HBM, 76 bytes a block (FP64).  On the 3,072-element bar, 1.68 GB
+// of blocks, the one-step pass took 270 us a step, more than the GMRES it runs
+// beside (223 us), and a step 339 us; with T = 2 a step takes 218 us (mixed
+// precision: 201 -> 168).  T = 3 is slower (230), as the head then reads 14% of
+// the blocks on the chain instead of 6%.  Of 256 to 1,024 threads with 1 to 3
+// blocks in flight each, 256 with 3 at two CTAs per SM was fastest in both.
+template <bool kMixed, int T>
+__global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0)
+{
+    constexpr int NW = kRhsThreads / 32, kUnroll = 3;
+    extern __shared__ int slot_of_k[];  // slot of W_{t0-k}
+    __shared__ double red[NW][T][3];
+    const int row = d.row_of[blockIdx.x], K = d.K, SW = d.SW;
+    for (int k = threadIdx.x; k <= K; k += blockDim.x) slot_of_k[k] = (((t0 - k) % SW) + SW) % SW;
+    // runs beside GMRES launches that may set the status word: thread 0's
+    // reading is OR-ed across the CTA by the barrier
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)d.status)) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t nnz = d.h_nnz, *kp = d.h_kptr + (int64_t)row * (K + 1);
+    const int64_t slot_len = 6LL * d.nh;
+    double a[T][3] = {};
+    // part(h0): blocks [beg, end) for the steps t0 + h, h >= h0
+    auto part = [&](auto first, int64_t beg, int64_t end) {
+        constexpr int h0 = decltype(first)::value;
+#pragma unroll kUnroll
+        for (int64_t i = beg + threadIdx.x; i < end; i += kRhsThreads) {
+            const uint32_t cp = __ldcs(d.h_col + i);
+            int slot = slot_of_k[cp >> 21];
+            const double* wc = d.wring + ((int64_t)((cp >> 20) & 1u) * d.nh + (cp & 0xFFFFFu)) * 3;
+            double m[9];
+#pragma unroll
+            for (int c = 0; c < 9; ++c) {
+                if constexpr (kMixed) m[c] = (double)__ldcs(d.h_val32 + c * nnz + i);
+                else m[c] = __ldcs(d.h_val + c * nnz + i);
+            }
+#pragma unroll
+            for (int h = 0; h < T; ++h) {
+                if (h >= h0) {
+                    const double* x = wc + slot * slot_len;
+                    const double x0 = x[0], x1 = x[1], x2 = x[2];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) a[h][c] += m[3 * c] * x0 + m[3 * c + 1] * x1 + m[3 * c + 2] * x2;
+                }
+                slot = slot + 1 == SW ? 0 : slot + 1;
+            }
+        }
+    };
+    const int kb = t0 < K ? t0 : K;  // up to here every step has a stored vector
+    if (kb >= d.kr) part(std::integral_constant<int, 0>{}, kp[d.kr - 1], kp[kb]);
+    // W_{t0+h-k} of t0 < k exists for the later steps only (while t0 < K)
+    if (t0 < K && t0 + 1 >= d.kr) part(std::integral_constant<int, 1>{}, kp[t0], kp[t0 + 1]);
+    if constexpr (T > 2)
+        if (t0 + 1 < K && t0 + 2 >= d.kr) part(std::integral_constant<int, 2>{}, kp[t0 + 1], kp[t0 + 2]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int h = 0; h < T; ++h)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) a[h][c] += __shfl_xor_sync(0xffffffffu, a[h][c], o);
+#pragma unroll 1
+    for (int h = 0; h < T; ++h) {
+        double ka[3] = {0.0, 0.0, 0.0};
+        if (t0 + h <= d.nstep) known_share<1, NW>(d, row, t0 + h, w, lane, ka);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) red[w][h][c] = ka[c];
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int h = 0; h < T; ++h)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) red[w][h][c] += a[h][c];
+    __syncthreads();
+    if (threadIdx.x < 3 * T) {
+        const int h = threadIdx.x / 3, c = threadIdx.x % 3;
+        if (t0 + h > d.nstep) return;
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < NW; ++q) s += red[q][h][c];
+        d.bulk[(int64_t)((t0 + h) & 7) * 3 * d.E + 3 * blockIdx.x + c] = s;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // The same part of the right-hand sides over the group layout (8 or more load
 // cases): a cluster of CTAs takes a group of 8 rows.  What bounds it: FP64
@@ -943,7 +1030,7 @@ cudaError_t launch_rhs(const MarchData& d, int step, bool bulk, int add_bulk, cu
 
 // T-step history pass (T = (kr - 1) / 2, 2 or 3): two load cases per thread
 // (the registers hold the T steps' sums and the window of T history
-// vectors), one for R = 1.  Measured against the two-step form on the 32-load
+// vectors); one load case reads the step-major matrices.  Measured against the two-step form on the 32-load
 // bar and kept out: staging the history vectors and block values through
 // shared memory with cp.async (72% more instructions, 1.5x slower) and L1
 // prefetches of the coming vectors (slower at every distance tried).
@@ -977,9 +1064,14 @@ cudaError_t launch_bulk_steps(const MarchData& d, int t0, cudaStream_t s)
         using V = typename std::conditional<kMixed, float, double>::type;
         if (d.hg_n > 0) return d.kr >= 7 ? launch_bulk_groups<R, 3, V>(d, t0, s) : launch_bulk_groups<R, 2, V>(d, t0, s);
     }
-    constexpr int kC = R >= 2 ? 2 : 1;
-    if (d.kr >= 7) bulk_steps_kernel<R, kMixed, kC, 3><<<d.E, kRhsThreads, 0, s>>>(d, t0);
-    else bulk_steps_kernel<R, kMixed, kC, 2><<<d.E, kRhsThreads, 0, s>>>(d, t0);
+    if constexpr (R == 1) {
+        const size_t slots = sizeof(int) * (d.K + 1);
+        if (d.kr >= 7) bulk_rows_kernel<kMixed, 3><<<d.E, kRhsThreads, slots, s>>>(d, t0);
+        else bulk_rows_kernel<kMixed, 2><<<d.E, kRhsThreads, slots, s>>>(d, t0);
+    } else {
+        if (d.kr >= 7) bulk_steps_kernel<R, kMixed, 2, 3><<<d.E, kRhsThreads, 0, s>>>(d, t0);
+        else bulk_steps_kernel<R, kMixed, 2, 2><<<d.E, kRhsThreads, 0, s>>>(d, t0);
+    }
     return cudaGetLastError();
 }
 
