@@ -470,6 +470,7 @@ struct tdbem_handle {
     DevBuf d_uref_sign, d_tref_sign, d_hu_sign, d_ht_sign, d_itf_trans, d_uref_block, d_tref_block, d_hist_block;
     DevBuf d_uref_known, d_tref_known, d_hist_owner, d_known_elem, d_known_sign, d_itf_a, d_itf_asign;
     DevBuf d_h_kptr, d_h_col, d_h_val, d_h_val32;
+    DevBuf d_hd_ptr, d_hd_tile;  // packed head blocks of one load case
     DevBuf d_r_ptr, d_r_meta, d_r_off, d_r_val;  // run layout of steps k >= run_k (T-step history pass)
     int64_t r_nb = 0, r_runs = 0;
     int run_k = 0;
@@ -855,7 +856,7 @@ void bisect_rows(const std::vector<double>& node, int32_t* b, int32_t* e, int G)
 // size on, the L2's: what fits there the one-step pass reads fast enough to hide
 // beside GMRES, and the longer head costs more than it saves.  Steps of bars
 // with one load case, one-step -> T = 2: 0.02 GB 86.9 -> 88.2 us, 0.19 GB 129.6 ->
-// 126.8, 0.44 GB 145.4 -> 143.2, 0.82 GB 197.8 -> 188.7, 1.68 GB 339 -> 218.
+// 126.8, 0.44 GB 145.4 -> 139.0, 0.82 GB 197.8 -> 185, 1.68 GB 339 -> 200.
 constexpr double kRowsPassBytes = 126e6;
 double history_bytes(const tdbem_handle* h)
 {
@@ -1285,6 +1286,39 @@ tdbem_status gmres_layout(tdbem_handle* h, int G, int C, cudaStream_t s)
     return TDBEM_OK;
 }
 
+// Packed blocks of the head pass of one load case (MarchData hd_*); where they do
+// not fit, the head reads the step-major matrices.
+tdbem_status build_head(tdbem_handle* h, cudaStream_t s)
+{
+    h->d_hd_ptr.release();
+    h->d_hd_tile.release();
+    if (h->R != 1 || h->K < 1 || h->h_nnz == 0) return TDBEM_OK;
+    const int64_t E = h->E;
+    const int head_k = h->K < 3 ? h->K : h->run_k ? h->run_k - 1 : 2;
+    const bool mixed = h->precision == TDBEM_PRECISION_MIXED;
+    std::vector<int32_t> ptr(E + 1, 0);
+    int64_t tiles = 0;
+    for (int64_t p = 0; p < E; ++p) {
+        const int64_t* kp = &h->h_kptr[(size_t)h->repid[p] * (h->K + 1)];
+        tiles += (kp[head_k] - kp[0] + 31) / 32;
+        if (tiles > INT32_MAX) return TDBEM_OK;
+        ptr[p + 1] = (int32_t)tiles;
+    }
+    cudaError_t e = h->d_hd_tile.alloc(head_tile_bytes(mixed) * std::max<int64_t>(tiles, 1));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        h->d_hd_tile.release();
+        return TDBEM_OK;
+    }
+    CUDA_TRY(e);
+    CUDA_TRY(up(h->d_hd_ptr, ptr, s));
+    CUDA_TRY(pack_head((int)E, h->K, head_k, h->d_row_of.as<int32_t>(), h->d_h_kptr.as<int64_t>(),
+                       h->d_h_col.as<uint32_t>(), mixed ? h->d_h_val32.p : h->d_h_val.p, mixed, h->h_nnz,
+                       h->d_hd_ptr.as<int32_t>(), h->d_hd_tile.as<unsigned char>(), s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    return TDBEM_OK;
+}
+
 tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
 {
     const int64_t E = h->E;
@@ -1412,6 +1446,7 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     CUDA_TRY(h->d_u.alloc(vec));
     CUDA_TRY(h->d_bulk.alloc(8 * vec));
     CUDA_TRY(h->d_status.alloc(sizeof(int) * 4));
+    if (tdbem_status st = build_head(h, s); st != TDBEM_OK) return st;
     const int SW = h->K + 1;
     const int64_t nhm = std::max<int64_t>(h->n_hist, 1);
     CUDA_TRY(h->d_xring.alloc(sizeof(double) * 3 * 2 * nhm * 3 * R));
@@ -1512,6 +1547,8 @@ struct MarchRun {
         d.r_val32 = h->d_r_val.as<float>();
         d.r_nb = h->r_nb;
         d.kr = h->run_k;
+        d.hd_ptr = h->d_hd_ptr.as<int32_t>();
+        d.hd_tile = h->d_hd_tile.as<unsigned char>();
         d.hg_n = h->hg_n;
         // a CTA's warps get about a dozen segments each
         d.hg_split = 1;
@@ -1599,7 +1636,7 @@ struct MarchRun {
         CUDA_TRY(cudaSetDevice(h->device));
         const int T = h->run_k >= 5 ? (h->run_k - 1) / 2 : 2;  // steps per history pass
         StepEvents se{E7(k, 0), E7(k, 1), E7(k, 2), E7(k, 3), E7(k, 4), E7(k, 5), E7(k, 6),
-                      k == 1 ? ev[1] : E7(k - 1, 3), k > T ? E7(k - T, 6) : nullptr};
+                      k == 1 ? ev[1] : E7(k - 1, 3), k > T ? E7(R == 1 ? k - 1 : k - T, 6) : nullptr};
         CUDA_TRY(march_step(d, k, s, serial_history ? s : h->side, se, overlap));
         return TDBEM_OK;
     }

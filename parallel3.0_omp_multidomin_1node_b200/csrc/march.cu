@@ -32,6 +32,7 @@ namespace tdbem {
 namespace {
 
 constexpr int kRhsThreads = 256;
+constexpr int kHeadWarps = 4;          // warps per row of head_rows_kernel
 constexpr int kMaxDevices = 64;        // launch attributes are kept per device
 
 template <int R, int kCpt = (R >= 4 ? 4 : R)>
@@ -111,8 +112,9 @@ __global__ void prepare_kernel(MarchData d)
 // (DBEM1/multidomain.cpp:3843-3846): known blocks j = first + w, first + w +
 // NW, ... of the row; lane r < R takes load case r.  The warps' shares are
 // summed with the history sums.
-template <int R, int NW>
-__device__ __forceinline__ void known_share(const MarchData& d, int row, int step, int w, int lane, double (&ka)[3])
+template <int R>
+__device__ __forceinline__ void known_share(const MarchData& d, int row, int step, int w, int NW, int lane,
+                                            double (&ka)[3])
 {
     ka[0] = ka[1] = ka[2] = 0.0;
     if (lane >= R) return;
@@ -232,7 +234,7 @@ __device__ __forceinline__ void rhs_row(const MarchData& d, const int p, const i
     // else the head
     if (kBulk || !add_bulk) {
         double ka[3];
-        known_share<R, NW>(d, row, step, w, lane, ka);
+        known_share<R>(d, row, step, w, NW, lane, ka);
         __syncwarp();
         if (lane < R)
 #pragma unroll
@@ -261,6 +263,94 @@ template <int R, bool kMixed, bool kBulk, int kCpt>
 __global__ void __launch_bounds__(kRhsThreads, R >= 8 ? 2 : 3) rhs_kernel(MarchData d, int step, int add_bulk)
 {
     rhs_row<R, kMixed, kBulk, kCpt>(d, blockIdx.x, step, add_bulk, d.k_lo, d.k_hi);
+}
+
+// The head pass of one load case over its packed blocks (MarchData hd_*): a row
+// takes four warps.  What bounds it is latency: it runs on the
+// chain, after a history pass that has swept the caches.  In the step-major
+// matrices a row's few head blocks lie on ten pages (nine value planes and the
+// columns) that no other row's head shares much of; packed, the part is 6% of the
+// matrices in one piece.  Beside the half pass of bulk_rows_kernel, head of the
+// 3,072-element bar: 47 us with rhs_kernel, 34 with warps over the step-major
+// matrices, 27 packed (102 MB); of 1,728 elements: 24 -> 22 -> 18.  Four
+// warps a row: with one, a step of the 120-element rod takes 69.7 us instead of
+// 67.5 and of the 1,728-element bar 146 instead of 140; with eight, of 480 elements
+// 69.6 instead of 67.1 and of the 3,072-element bar 205 instead of 200.  Loads that leave the blocks in L2
+// make the head as fast and GMRES slower (168 -> 190), so they stream.
+template <bool kMixed>
+__global__ void __launch_bounds__(kRhsThreads, 3) head_rows_kernel(MarchData d, int step, int add_bulk)
+{
+    using V = typename std::conditional<kMixed, float, double>::type;
+    constexpr int NW = kRhsThreads / 32, wpr = kHeadWarps, kUnroll = 4;
+    constexpr size_t kTile = head_tile_bytes(kMixed);
+    __shared__ double red[NW][3];
+    if (*(volatile int*)d.status) return;  // set by GMRES before this launch only
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, part = w % wpr;
+    const int p = blockIdx.x * (NW / wpr) + w / wpr;
+    const bool on = p < d.E;
+    double acc[3] = {0.0, 0.0, 0.0};
+    if (on) {
+        const int t0 = d.hd_ptr[p], t1 = d.hd_ptr[p + 1];
+        const int64_t slot_len = 6LL * d.nh;
+        const int SW = d.SW, s0 = step % SW, k_hi = d.k_hi;
+#pragma unroll kUnroll
+        for (int t = t0 + part; t < t1; t += wpr) {
+            const unsigned char* tile = d.hd_tile + t * kTile;
+            const uint32_t cp = __ldcs(reinterpret_cast<const unsigned*>(tile) + lane);
+            const V* v = reinterpret_cast<const V*>(tile + 128) + lane;
+            double m[9];
+#pragma unroll
+            for (int c = 0; c < 9; ++c) m[c] = (double)__ldcs(v + 32 * c);
+            const int k = (int)(cp >> 21);
+            int slot = s0 - k;
+            if (slot < 0) slot += SW;
+            const double* x = d.wring + slot * slot_len + ((int64_t)((cp >> 20) & 1u) * d.nh + (cp & 0xFFFFFu)) * 3;
+            const bool in = k <= k_hi && cp;  // padding is 0
+            const double x0 = in ? x[0] : 0.0, x1 = in ? x[1] : 0.0, x2 = in ? x[2] : 0.0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) acc[c] += m[3 * c] * x0 + m[3 * c + 1] * x1 + m[3 * c + 2] * x2;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    const int row = on ? d.row_of[p] : 0;
+    if (lane == 0) {
+        if (on && !add_bulk) {
+            double ka[3];
+            known_share<1>(d, row, step, part, wpr, lane, ka);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) acc[c] += ka[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) red[w][c] = acc[c];
+    }
+    __syncthreads();
+    if (on && part == 0 && lane < 3) {
+        double s = 0.0;
+        for (int q = 0; q < wpr; ++q) s += red[w + q][lane];
+        if (add_bulk) s += d.bulk[(int64_t)(step & 7) * 3 * d.E + 3 * p + lane];
+        d.b[3 * p + lane] = s;
+        if (d.rec_rhs) d.rec_rhs[(int64_t)(step - 1) * 3 * d.E + 3 * row + lane] = s;
+    }
+}
+
+// Packs the blocks k <= head_k of each perm row into tiles of 32, zero-padded.
+template <class V>
+__global__ void pack_head_kernel(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
+                                 const V* val, int64_t nnz, const int32_t* ptr, unsigned char* tiles)
+{
+    const int p = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (p >= E) return;
+    const int64_t b = kptr[(int64_t)row_of[p] * (K + 1)], e = kptr[(int64_t)row_of[p] * (K + 1) + head_k];
+    for (int t = ptr[p]; t < ptr[p + 1]; ++t) {
+        const int64_t i = b + (int64_t)(t - ptr[p]) * 32 + lane;
+        unsigned char* tile = tiles + t * head_tile_bytes(sizeof(V) == 4);
+        reinterpret_cast<uint32_t*>(tile)[lane] = i < e ? col[i] : 0u;
+        V* v = reinterpret_cast<V*>(tile + 128) + lane;
+        for (int c = 0; c < 9; ++c) v[32 * c] = i < e ? val[c * nnz + i] : V(0);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -406,7 +496,7 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
     for (int h = 0; h < T; ++h) {
         if (t0 + h > d.nstep) break;
         double ka[3];
-        known_share<R, NW>(d, row, t0 + h, w, lane, ka);
+        known_share<R>(d, row, t0 + h, w, NW, lane, ka);
         if (lane < R)
 #pragma unroll
             for (int c = 0; c < 3; ++c) red[w][h][c][lane] += ka[c];
@@ -432,14 +522,16 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
 // beside (223 us), and a step 339 us; with T = 2 a step takes 218 us (mixed
 // precision: 201 -> 168).  T = 3 is slower (230), as the head then reads 14% of
 // the blocks on the chain instead of 6%.  Of 256 to 1,024 threads with 1 to 3
-// blocks in flight each, 256 with 3 at two CTAs per SM was fastest in both.
+// blocks in flight each, 256 with 3 at two CTAs per SM was fastest in both.  Each
+// GMRES launch of the T has a T-th of the rows beside it (launched as one, a pass
+// held up the next head and GMRES for an SM: 218 -> 206 us with the head above).
 template <bool kMixed, int T>
-__global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0)
+__global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0, int p0)
 {
     constexpr int NW = kRhsThreads / 32, kUnroll = 3;
     extern __shared__ int slot_of_k[];  // slot of W_{t0-k}
     __shared__ double red[NW][T][3];
-    const int row = d.row_of[blockIdx.x], K = d.K, SW = d.SW;
+    const int p = p0 + blockIdx.x, row = d.row_of[p], K = d.K, SW = d.SW;
     for (int k = threadIdx.x; k <= K; k += blockDim.x) slot_of_k[k] = (((t0 - k) % SW) + SW) % SW;
     // runs beside GMRES launches that may set the status word: thread 0's
     // reading is OR-ed across the CTA by the barrier
@@ -489,7 +581,7 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, 
 #pragma unroll 1
     for (int h = 0; h < T; ++h) {
         double ka[3] = {0.0, 0.0, 0.0};
-        if (t0 + h <= d.nstep) known_share<1, NW>(d, row, t0 + h, w, lane, ka);
+        if (t0 + h <= d.nstep) known_share<1>(d, row, t0 + h, w, NW, lane, ka);
         if (lane == 0)
 #pragma unroll
             for (int c = 0; c < 3; ++c) red[w][h][c] = ka[c];
@@ -506,7 +598,7 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, 
         double s = 0.0;
 #pragma unroll
         for (int q = 0; q < NW; ++q) s += red[q][h][c];
-        d.bulk[(int64_t)((t0 + h) & 7) * 3 * d.E + 3 * blockIdx.x + c] = s;
+        d.bulk[(int64_t)((t0 + h) & 7) * 3 * d.E + 3 * p + c] = s;
     }
 }
 
@@ -731,7 +823,7 @@ __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kern
         const int p = __ldg(rows + i % 8), h = i / 8;
         if (p < 0 || t0 + h > d.nstep) continue;
         double ka[3];
-        known_share<R, 1>(d, d.row_of[p], t0 + h, 0, lane, ka);
+        known_share<R>(d, d.row_of[p], t0 + h, 0, 1, lane, ka);
         if (lane < R)
 #pragma unroll
             for (int c = 0; c < 3; ++c) sums[(h * 24 + 3 * (i % 8) + c) * R + lane] += ka[c];
@@ -1024,7 +1116,10 @@ cudaError_t launch_rhs(const MarchData& d, int step, bool bulk, int add_bulk, cu
         if (d.rhs_cpt == 1) return launch_rhs_cpt<R, kMixed, 1>(d, step, bulk, add_bulk, s);
         return launch_rhs_cpt<R, kMixed, 2>(d, step, bulk, add_bulk, s);
     } else {
-        return launch_rhs_cpt<R, kMixed, 1>(d, step, bulk, add_bulk, s);
+        if (bulk || !d.hd_ptr) return launch_rhs_cpt<R, kMixed, 1>(d, step, bulk, add_bulk, s);
+        constexpr int rows = kRhsThreads / 32 / kHeadWarps;
+        head_rows_kernel<kMixed><<<(d.E + rows - 1) / rows, kRhsThreads, 0, s>>>(d, step, add_bulk);
+        return cudaGetLastError();
     }
 }
 
@@ -1058,7 +1153,7 @@ cudaError_t launch_bulk_groups(const MarchData& d, int t0, cudaStream_t s)
 }
 
 template <int R, bool kMixed>
-cudaError_t launch_bulk_steps(const MarchData& d, int t0, cudaStream_t s)
+cudaError_t launch_bulk_steps(const MarchData& d, int t0, int part, cudaStream_t s)
 {
     if constexpr (R >= 8) {
         using V = typename std::conditional<kMixed, float, double>::type;
@@ -1066,8 +1161,10 @@ cudaError_t launch_bulk_steps(const MarchData& d, int t0, cudaStream_t s)
     }
     if constexpr (R == 1) {
         const size_t slots = sizeof(int) * (d.K + 1);
-        if (d.kr >= 7) bulk_rows_kernel<kMixed, 3><<<d.E, kRhsThreads, slots, s>>>(d, t0);
-        else bulk_rows_kernel<kMixed, 2><<<d.E, kRhsThreads, slots, s>>>(d, t0);
+        const int T = d.kr >= 7 ? 3 : 2, p0 = (int)((int64_t)d.E * part / T), p1 = (int)((int64_t)d.E * (part + 1) / T);
+        if (p1 == p0) return cudaSuccess;
+        if (T == 3) bulk_rows_kernel<kMixed, 3><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0);
+        else bulk_rows_kernel<kMixed, 2><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0);
     } else {
         if (d.kr >= 7) bulk_steps_kernel<R, kMixed, 2, 3><<<d.E, kRhsThreads, 0, s>>>(d, t0);
         else bulk_steps_kernel<R, kMixed, 2, 2><<<d.E, kRhsThreads, 0, s>>>(d, t0);
@@ -1084,7 +1181,10 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
     // launched at step e covers steps e + T .. e + 2T - 1
     const int T = d.kr >= 5 ? (d.kr - 1) / 2 : 0;
     const bool pair = overlap && T >= 2;
-    const bool launches = pair && step >= 2 && (step - 2) % T == 0;
+    // one load case: part of the rows beside each of the T GMRES launches, so that
+    // a part ends with its GMRES and the head finds the SMs free
+    const int part = pair && step >= 2 ? (step - 2) % T : 0;
+    const bool launches = pair && step >= 2 && (part == 0 || R == 1);
     cudaError_t e;
     // the first step a pass covers waits for it
     if (pair && step >= 2 + T && (step - 2) % T == 0 && ev.prev_pass) cudaStreamWaitEvent(s, ev.prev_pass, 0);
@@ -1128,9 +1228,9 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
         // after it
         if (ev.prev_gm) cudaStreamWaitEvent(side, ev.prev_gm, 0);
         cudaEventRecord(ev.bulk0, side);
-        const int t0 = step + T;
+        const int t0 = step - part + T;
         if (launches && t0 <= d.nstep) {
-            e = d.mixed ? launch_bulk_steps<R, true>(d0, t0, side) : launch_bulk_steps<R, false>(d0, t0, side);
+            e = d.mixed ? launch_bulk_steps<R, true>(d0, t0, part, side) : launch_bulk_steps<R, false>(d0, t0, part, side);
             if (e != cudaSuccess) return e;
         }
         cudaEventRecord(ev.bulk1, side);
@@ -1285,6 +1385,18 @@ __global__ void gather_tiles_kernel(int64_t n, const int32_t* src, const double*
         out[t] = v;
         if (out32) out32[t] = (float)v;
     }
+}
+
+cudaError_t pack_head(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
+                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, cudaStream_t s)
+{
+    if (mixed)
+        pack_head_kernel<<<(E + 7) / 8, 256, 0, s>>>(E, K, head_k, row_of, kptr, col, static_cast<const float*>(val), nnz,
+                                                     ptr, tiles);
+    else
+        pack_head_kernel<<<(E + 7) / 8, 256, 0, s>>>(E, K, head_k, row_of, kptr, col, static_cast<const double*>(val), nnz,
+                                                     ptr, tiles);
+    return cudaGetLastError();
 }
 
 cudaError_t gather_tiles(int64_t tiles, const int32_t* src, const double* val9, double* out, float* out32,

@@ -39,6 +39,11 @@ struct MarchData {
     const double* h_val;    // SoA [9][nnz]
     const float* h_val32;   // SoA [9][nnz] (mixed)
     int64_t h_nnz;
+    // head pass of one load case: the blocks of the first steps (below kr, or 1 and
+    // 2) of each perm row again, in tiles of 32 columns and 9 planes of 32 values
+    // (head_tile_bytes), zero-padded; null: none
+    const int32_t* hd_ptr;  // [E+1] first tile of each perm row
+    const unsigned char* hd_tile;
     // run layout of the blocks of steps k >= kr = 2T + 1, for the T-step
     // history pass: per equation row, runs of one (type, column) pair over
     // consecutive steps, longest first; kr = 0 when there is none
@@ -207,6 +212,11 @@ cudaError_t build_history_groups(int E, int K, int kr, const std::vector<int32_t
                                  const void* d_val, int64_t nnz, bool mixed, HistoryGroups& out, cudaStream_t s);
 size_t history_groups_bytes(int64_t nb, bool mixed);
 
+// Blocks of steps 1 .. head_k of each perm row to tiles (MarchData hd_*).
+constexpr size_t head_tile_bytes(bool mixed) { return 128 + 9 * 32 * (mixed ? 4 : 8); }
+cudaError_t pack_head(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
+                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, cudaStream_t s);
+
 // Sizes of the R template instantiations.
 bool march_supported_loads(int R);
 cudaError_t march_prepare(const MarchData& d, cudaStream_t s);
@@ -222,8 +232,8 @@ cudaError_t march_prepare(const MarchData& d, cudaStream_t s);
 // chain stream, gm0/gm1 the GMRES kernel, bulk0/bulk1 the overlapped bulk
 // kernel on the side stream; sync orders a later head after the bulk;
 // prev_gm is gm1 of the previous step (the side stream waits on it);
-// prev_pass is sync of step-T (the first step a T-step pass covers waits on
-// it).
+// prev_pass is sync of the launch that ends the pass before: of step-T, of
+// step-1 with one load case (the first step a T-step pass covers waits on it).
 struct StepEvents {
     cudaEvent_t head0, head1, gm0, gm1, bulk0, bulk1, sync, prev_gm, prev_pass;
 };
