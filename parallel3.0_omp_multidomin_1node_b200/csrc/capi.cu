@@ -418,7 +418,8 @@ struct EventPool {
 
 struct tdbem_handle {
     int device = 0;
-    EventPool ev_timed;                                   // MarchRun's step events
+    EventPool ev_timed;                                   // MarchRun's timed events
+    EventPool ev_step{{}, cudaEventDisableTiming};        // its steps' events
     EventPool ev_order{{}, cudaEventDisableTiming};       // ordering-only events (copy chunks, grouped march)
     cudaStream_t s0 = nullptr;    // default stream of the handle
     cudaStream_t hp = nullptr;    // high-priority stream of the per-step chain
@@ -482,7 +483,7 @@ struct tdbem_handle {
     DevBuf d_leaf_begin, d_leaf_count, d_leaf_off, d_row_leaf;
     DevBuf d_pmat, d_pmat_c, d_pinv, d_pinv_c, d_pinv32, d_minv;  // leaf blocks and inverses (LeafBlocks)
     GmresTiles tiles;                                             // A' for the GMRES clusters
-    DevBuf d_xring, d_wring, d_bulk, d_b, d_x, d_rv, d_aw, d_u, d_V, d_givens, d_status, d_flags, d_audit;
+    DevBuf d_xring, d_wring, d_bulk, d_b, d_x, d_rv, d_aw, d_u, d_V, d_givens, d_status, d_flags, d_audit, d_stamps;
     DevBuf d_known, d_out_lu, d_out_lt, d_rec_rhs, d_rec_x, d_xold;
     std::unique_ptr<AdjointState> adjoint;
 
@@ -1489,11 +1490,11 @@ FILE* open_diagnostic_csv(const std::string& path, const char* header)
 struct MarchRun {
     tdbem_handle* h = nullptr;
     MarchData d{};
-    std::vector<cudaEvent_t> ev;
+    std::vector<cudaEvent_t> ev, order;  // start, first launch, end; the steps' (StepEvents)
     bool overlap = false;
     // TDBEM_OVERLAP=0: the history part k >= 3 runs on the chain stream
-    // after each step's GMRES instead of beside it (same results; its
-    // events then time the history kernel alone, for measurement)
+    // after each step's GMRES instead of beside it (same results; the
+    // history time is then that of the kernel alone, for measurement)
     bool serial_history = false;
     bool grouped = false;             // stepped by the several-models launches (no per-phase times)
     cudaStream_t us = nullptr, s = nullptr;
@@ -1503,7 +1504,7 @@ struct MarchRun {
     MarchRun() = default;
     MarchRun(const MarchRun&) = delete;
     MarchRun& operator=(const MarchRun&) = delete;
-    cudaEvent_t E7(int step, int j) const { return ev[3 + 7 * (size_t)(step - 1) + j]; }
+    cudaEvent_t E2(int step, int j) const { return order[2 * (size_t)(step - 1) + j]; }
 
     tdbem_status begin(tdbem_handle* hh, const double* d_known_lu, double* d_out_lu, double* d_out_lt, void* stream)
     {
@@ -1518,8 +1519,11 @@ struct MarchRun {
         R = h->R;
         h->saved_forward = false;
         h->diag_ready = false;
-        CUDA_TRY(h->d_flags.alloc(sizeof(int) * 3 * std::max(N, 1) * R));
-        CUDA_TRY(h->d_audit.alloc(sizeof(double) * 2 * std::max(N, 1)));
+        // kept from march to march: sized by the handle
+        auto keep = [](DevBuf& b, size_t n) { return b.p && b.bytes == n ? cudaSuccess : b.alloc(n); };
+        CUDA_TRY(keep(h->d_flags, sizeof(int) * 3 * std::max(N, 1) * R));
+        CUDA_TRY(keep(h->d_audit, sizeof(double) * 2 * std::max(N, 1)));
+        CUDA_TRY(keep(h->d_stamps, sizeof(unsigned long long) * 5 * ((size_t)N + 4)));
         if (h->record) {
             CUDA_TRY(h->d_rec_rhs.alloc(sizeof(double) * 3 * E * std::max(N, 1)));
             CUDA_TRY(h->d_rec_x.alloc(sizeof(double) * 3 * E * std::max(N, 1)));
@@ -1603,6 +1607,7 @@ struct MarchRun {
         d.status = h->d_status.as<int>();
         d.step_flags = h->d_flags.as<int>();
         d.audit = h->d_audit.as<double>();
+        d.stamps = h->d_stamps.as<unsigned long long>();
         d.known_lu = d_known_lu;
         d.out_lu = d_out_lu;
         d.out_lt = d_out_lt;
@@ -1619,7 +1624,8 @@ struct MarchRun {
         // the chain runs on the handle's high-priority stream, ordered after
         // the caller's stream and followed by it
         const int NS = std::max(N, 1);
-        CUDA_TRY(h->ev_timed.take(7 * (size_t)NS + 3, ev));
+        CUDA_TRY(h->ev_timed.take(3, ev));
+        CUDA_TRY(h->ev_step.take(2 * (size_t)NS, order));
         CUDA_TRY(cudaEventRecord(ev[0], us));
         CUDA_TRY(cudaStreamWaitEvent(s, ev[0], 0));
         CUDA_TRY(cudaStreamWaitEvent(h->side, ev[0], 0));
@@ -1627,6 +1633,7 @@ struct MarchRun {
         CUDA_TRY(cudaMemsetAsync(d_out_lu, 0, sizeof(double) * R * (N + 1) * E * 3, s));
         CUDA_TRY(cudaMemsetAsync(d_out_lt, 0, sizeof(double) * R * (N + 1) * E * 3, s));
         CUDA_TRY(cudaMemsetAsync(h->d_flags.p, 0, h->d_flags.bytes, s));
+        CUDA_TRY(cudaMemsetAsync(h->d_stamps.p, 0, h->d_stamps.bytes, s));
         CUDA_TRY(march_prepare(d, s));
         return TDBEM_OK;
     }
@@ -1635,8 +1642,8 @@ struct MarchRun {
     {
         CUDA_TRY(cudaSetDevice(h->device));
         const int T = h->run_k >= 5 ? (h->run_k - 1) / 2 : 2;  // steps per history pass
-        StepEvents se{E7(k, 0), E7(k, 1), E7(k, 2), E7(k, 3), E7(k, 4), E7(k, 5), E7(k, 6),
-                      k == 1 ? ev[1] : E7(k - 1, 3), k > T ? E7(R == 1 ? k - 1 : k - T, 6) : nullptr};
+        StepEvents se{E2(k, 0), E2(k, 1), k == 1 ? ev[1] : E2(k - 1, 0),
+                      k > T ? E2(R == 1 ? k - 1 : k - T, 1) : nullptr};
         CUDA_TRY(march_step(d, k, s, serial_history ? s : h->side, se, overlap));
         return TDBEM_OK;
     }
@@ -1660,16 +1667,20 @@ struct MarchRun {
         tdbem_report rep{};
         float ms = 0.0f;
         double ms_rhs = 0.0, ms_gm = 0.0, ms_hist = 0.0;
-        for (int step = 1; step <= N && !grouped; ++step) {
-            float a = 0.0f, b = 0.0f, c = 0.0f;
-            cudaEventElapsedTime(&a, E7(step, 0), E7(step, 1));
-            cudaEventElapsedTime(&b, E7(step, 2), E7(step, 3));
-            if (overlap && step < N) cudaEventElapsedTime(&c, E7(step, 4), E7(step, 5));
-            ms_rhs += a + c;
-            ms_gm += b;
-            ms_hist += c;
+        if (!grouped) {
+            std::vector<unsigned long long> t(h->d_stamps.bytes / 8);
+            CUDA_TRY(cudaMemcpy(t.data(), h->d_stamps.p, h->d_stamps.bytes, cudaMemcpyDeviceToHost));
+            auto span = [&](int step, int a, int b) {
+                const unsigned long long t0 = t[5 * (size_t)step + a], t1 = t[5 * (size_t)step + b];
+                return t0 && t1 > t0 ? 1e-6 * (double)(t1 - t0) : 0.0;
+            };
+            for (int step = 1; step <= N; ++step) {
+                ms_rhs += span(step, 0, 1);
+                ms_gm += span(step, 1, 2);
+            }
+            for (size_t row = 0; row < t.size() / 5; ++row) ms_hist += span((int)row, 3, 4);
+            ms_rhs += ms_hist;
         }
-
         cudaEventElapsedTime(&ms, ev[1], ev[2]);
         rep.ms_total = ms;
         rep.gmres_cluster = h->cluster;

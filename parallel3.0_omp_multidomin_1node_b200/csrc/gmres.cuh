@@ -29,6 +29,13 @@
 namespace cg = cooperative_groups;
 
 namespace tdbem {
+
+__device__ __forceinline__ unsigned long long device_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
 namespace {
 
 constexpr int kGmresThreads = 512;  // at most (gmres_threads)
@@ -850,7 +857,7 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
     };
     auto V = [&](int k) -> double* { return k < vcap ? vs + k * vs_len : vg + (int64_t)k * n; };
     auto pi = [&](int t) { return kLocal ? mirror_index<R>(t) : t; };
-    auto rhs = [&](int t) { return __ldg(d.b + (3LL * lo + t / R) * RT + roff + tr); };
+    auto rhs = [&](int t) { return __ldcg(d.b + (3LL * lo + t / R) * RT + roff + tr); };
     auto off = [&](const double* p) { return (int)(p - dsm); };
     const int2* const slices = d.g_sp + __ldg(d.g_cs + rank);
     const int32_t* const srows = d.g_rows + 4 * __ldg(d.g_cs + rank);
@@ -887,6 +894,11 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
         const int64_t end = (int64_t)(((uint64_t)(uint32_t)fl.y << 32) | (uint32_t)fl.x) + (int64_t)fl.w * fl.w;
         for (int i = threadIdx.x; rows > 0 && i < (int)(end - off0); i += NT) pc[i] = __ldg(pinv + off0 + i);
     }
+
+    // all above read what setup laid out; the head pass, beside which this launch may
+    // have started, is complete below
+    cudaGridDependencySynchronize();
+    if (d.stamps && blockIdx.x == 0 && threadIdx.x == 0) d.stamps[5 * (int64_t)step + 1] = device_ns();
 
     // start vector and residual (in us).  Mixed mode starts from the previous
     // steps' solutions extrapolated linearly (x_{s-1} at step 2); the FP64 path

@@ -42,6 +42,16 @@ struct Lanes {
     static constexpr int BPW = 32 / TPB;        // blocks per warp iteration
 };
 
+// Device clock readings of the launches (MarchData::stamps)
+__device__ __forceinline__ void stamp_start(const MarchData& d, int row, int which)
+{
+    if (d.stamps && blockIdx.x == 0 && threadIdx.x == 0) d.stamps[5 * (int64_t)row + which] = device_ns();
+}
+__device__ __forceinline__ void stamp_end(const MarchData& d, int row, int which)
+{
+    if (d.stamps && threadIdx.x == 0) atomicMax(d.stamps + 5 * (int64_t)row + which, device_ns());
+}
+
 // CPT consecutive values (16-byte aligned when CPT = 4 and R % 4 == 0)
 template <int CPT>
 __device__ __forceinline__ void load_cases(const float* p, float* v)
@@ -262,7 +272,10 @@ __device__ __forceinline__ void rhs_row(const MarchData& d, const int p, const i
 template <int R, bool kMixed, bool kBulk, int kCpt>
 __global__ void __launch_bounds__(kRhsThreads, R >= 8 ? 2 : 3) rhs_kernel(MarchData d, int step, int add_bulk)
 {
+    if constexpr (!kBulk) cudaTriggerProgrammaticLaunchCompletion();  // GMRES sets up beside it
+    stamp_start(d, step, kBulk ? 3 : 0);
     rhs_row<R, kMixed, kBulk, kCpt>(d, blockIdx.x, step, add_bulk, d.k_lo, d.k_hi);
+    if constexpr (kBulk) stamp_end(d, step, 4);
 }
 
 // The head pass of one load case over its packed blocks (MarchData hd_*): a row
@@ -284,7 +297,9 @@ __global__ void __launch_bounds__(kRhsThreads, 3) head_rows_kernel(MarchData d, 
     constexpr int NW = kRhsThreads / 32, wpr = kHeadWarps, kUnroll = 4;
     constexpr size_t kTile = head_tile_bytes(kMixed);
     __shared__ double red[NW][3];
-    if (*(volatile int*)d.status) return;  // set by GMRES before this launch only
+    cudaTriggerProgrammaticLaunchCompletion();  // GMRES sets up beside it
+    if (*(volatile int*)d.status) return;       // set by GMRES before this launch only
+    stamp_start(d, step, 0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, part = w % wpr;
     const int p = blockIdx.x * (NW / wpr) + w / wpr;
     const bool on = p < d.E;
@@ -373,6 +388,7 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
     constexpr int CPT = L::CPT, TPB = L::TPB, BPW = L::BPW;
     constexpr int NW = kRhsThreads / 32, NG = NW * BPW;
     __shared__ double red[NW][T][3][R];
+    stamp_start(d, t0, 3);
     // runs beside GMRES launches that may set the status word: thread 0's
     // reading is OR-ed across the CTA by the barrier
     if (__syncthreads_or(threadIdx.x == 0 && *(volatile int*)d.status)) return;
@@ -511,6 +527,7 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
         for (int q = 0; q < NW; ++q) s += red[q][h][c][r];
         d.bulk[(int64_t)((t0 + h) & 7) * E3R + (int64_t)(3 * blockIdx.x + c) * R + r] = s;
     }
+    stamp_end(d, t0, 4);
 }
 
 // The same part of the right-hand sides for one load case, over the step-major
@@ -526,11 +543,12 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
 // GMRES launch of the T has a T-th of the rows beside it (launched as one, a pass
 // held up the next head and GMRES for an SM: 218 -> 206 us with the head above).
 template <bool kMixed, int T>
-__global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0, int p0)
+__global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0, int p0, int part)
 {
     constexpr int NW = kRhsThreads / 32, kUnroll = 3;
     extern __shared__ int slot_of_k[];  // slot of W_{t0-k}
     __shared__ double red[NW][T][3];
+    stamp_start(d, t0 + part, 3);
     const int p = p0 + blockIdx.x, row = d.row_of[p], K = d.K, SW = d.SW;
     for (int k = threadIdx.x; k <= K; k += blockDim.x) slot_of_k[k] = (((t0 - k) % SW) + SW) % SW;
     // runs beside GMRES launches that may set the status word: thread 0's
@@ -540,8 +558,8 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, 
     const int64_t nnz = d.h_nnz, *kp = d.h_kptr + (int64_t)row * (K + 1);
     const int64_t slot_len = 6LL * d.nh;
     double a[T][3] = {};
-    // part(h0): blocks [beg, end) for the steps t0 + h, h >= h0
-    auto part = [&](auto first, int64_t beg, int64_t end) {
+    // apply(h0): blocks [beg, end) for the steps t0 + h, h >= h0
+    auto apply = [&](auto first, int64_t beg, int64_t end) {
         constexpr int h0 = decltype(first)::value;
 #pragma unroll kUnroll
         for (int64_t i = beg + threadIdx.x; i < end; i += kRhsThreads) {
@@ -567,11 +585,11 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, 
         }
     };
     const int kb = t0 < K ? t0 : K;  // up to here every step has a stored vector
-    if (kb >= d.kr) part(std::integral_constant<int, 0>{}, kp[d.kr - 1], kp[kb]);
+    if (kb >= d.kr) apply(std::integral_constant<int, 0>{}, kp[d.kr - 1], kp[kb]);
     // W_{t0+h-k} of t0 < k exists for the later steps only (while t0 < K)
-    if (t0 < K && t0 + 1 >= d.kr) part(std::integral_constant<int, 1>{}, kp[t0], kp[t0 + 1]);
+    if (t0 < K && t0 + 1 >= d.kr) apply(std::integral_constant<int, 1>{}, kp[t0], kp[t0 + 1]);
     if constexpr (T > 2)
-        if (t0 + 1 < K && t0 + 2 >= d.kr) part(std::integral_constant<int, 2>{}, kp[t0 + 1], kp[t0 + 2]);
+        if (t0 + 1 < K && t0 + 2 >= d.kr) apply(std::integral_constant<int, 2>{}, kp[t0 + 1], kp[t0 + 2]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -594,12 +612,12 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, 
     __syncthreads();
     if (threadIdx.x < 3 * T) {
         const int h = threadIdx.x / 3, c = threadIdx.x % 3;
-        if (t0 + h > d.nstep) return;
         double s = 0.0;
 #pragma unroll
         for (int q = 0; q < NW; ++q) s += red[q][h][c];
-        d.bulk[(int64_t)((t0 + h) & 7) * 3 * d.E + 3 * p + c] = s;
+        if (t0 + h <= d.nstep) d.bulk[(int64_t)((t0 + h) & 7) * 3 * d.E + 3 * p + c] = s;
     }
+    stamp_end(d, t0 + part, 4);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,6 +675,7 @@ __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kern
     constexpr int NT = P::NT, NW = P::NW;
     const int group = (int)blockIdx.x / split, rank = (int)blockIdx.x % split;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    stamp_start(d, t0, 3);
     // runs beside GMRES launches that may set the status word: the cluster
     // takes rank 0's reading
     __shared__ int stop, stop_all;
@@ -844,6 +863,7 @@ __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kern
         d.bulk[(int64_t)((t0 + h) & 7) * E3R + (int64_t)(3 * p + m % 3) * R + r] = s;
     }
     if (split > 1) cluster_barrier();  // peers still read this CTA's sums
+    stamp_end(d, t0, 4);
 }
 
 // Copy one model's MarchData into shared memory (several models per launch).
@@ -951,6 +971,7 @@ template <int R, bool kMixed, bool kLocal>
 __global__ void __launch_bounds__(kGmresThreads, 1) gmres_cluster_kernel(const __grid_constant__ MarchData d, int step)
 {
     gmres_body<R, kMixed, kLocal>(d, step, (int)(blockIdx.x / cg::this_cluster().num_blocks()));
+    stamp_end(d, step, 2);
 }
 
 // Several models' GMRES of one step in one launch: cluster m solves model m
@@ -1047,13 +1068,15 @@ cudaError_t launch_gmres_form(const MarchData& d0, int step, cudaStream_t s)
     if (cfg.dynamicSmemBytes > (size_t)cap) return cudaErrorInvalidValue;
     // the rest of the shared memory goes to leaf inverses and basis vectors
     if (kLocal) cfg.dynamicSmemBytes += gmres_caches(d, (size_t)cap - cfg.dynamicSmemBytes, R, kMixed);
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = d.cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = d.after_head ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, gmres_cluster_kernel<R, kMixed, kLocal>, d, step);
 }
 
@@ -1163,8 +1186,8 @@ cudaError_t launch_bulk_steps(const MarchData& d, int t0, int part, cudaStream_t
         const size_t slots = sizeof(int) * (d.K + 1);
         const int T = d.kr >= 7 ? 3 : 2, p0 = (int)((int64_t)d.E * part / T), p1 = (int)((int64_t)d.E * (part + 1) / T);
         if (p1 == p0) return cudaSuccess;
-        if (T == 3) bulk_rows_kernel<kMixed, 3><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0);
-        else bulk_rows_kernel<kMixed, 2><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0);
+        if (T == 3) bulk_rows_kernel<kMixed, 3><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0, part);
+        else bulk_rows_kernel<kMixed, 2><<<p1 - p0, kRhsThreads, slots, s>>>(d, t0, p0, part);
     } else {
         if (d.kr >= 7) bulk_steps_kernel<R, kMixed, 2, 3><<<d.E, kRhsThreads, 0, s>>>(d, t0);
         else bulk_steps_kernel<R, kMixed, 2, 2><<<d.E, kRhsThreads, 0, s>>>(d, t0);
@@ -1188,7 +1211,6 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
     cudaError_t e;
     // the first step a pass covers waits for it
     if (pair && step >= 2 + T && (step - 2) % T == 0 && ev.prev_pass) cudaStreamWaitEvent(s, ev.prev_pass, 0);
-    cudaEventRecord(ev.head0, s);
     if (!overlap) {
         d.k_lo = 1;
         d.k_hi = kcap;
@@ -1209,8 +1231,10 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
         e = d.mixed ? launch_rhs<R, true>(d, step, false, add, s) : launch_rhs<R, false>(d, step, false, add, s);
     }
     if (e != cudaSuccess) return e;
-    cudaEventRecord(ev.head1, s);
-    cudaEventRecord(ev.gm0, s);
+    // GMRES is scheduled while the head runs: without it a history pass takes the
+    // SMs that the head leaves.  Steps of one load case: 120-element rod 57.2 ->
+    // 55.0 us, 1,728-element bar 132 -> 117, 2,058 elements 179 -> 158.
+    d.after_head = 1;
     switch (d.R / d.groups) {
     case 1: e = d.mixed ? launch_gmres<1, true>(d, step, s) : launch_gmres<1, false>(d, step, s); break;
     case 2: e = d.mixed ? launch_gmres<2, true>(d, step, s) : launch_gmres<2, false>(d, step, s); break;
@@ -1221,26 +1245,23 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
     default: e = cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    cudaEventRecord(ev.gm1, s);
+    cudaEventRecord(ev.gm, s);
     if (pair) {
         // part k >= kr of steps step+T .. step+2T-1 needs the states up to
         // step-1 only: it runs beside the GMRES of this step and the T - 1
         // after it
         if (ev.prev_gm) cudaStreamWaitEvent(side, ev.prev_gm, 0);
-        cudaEventRecord(ev.bulk0, side);
         const int t0 = step - part + T;
         if (launches && t0 <= d.nstep) {
             e = d.mixed ? launch_bulk_steps<R, true>(d0, t0, part, side) : launch_bulk_steps<R, false>(d0, t0, part, side);
             if (e != cudaSuccess) return e;
         }
-        cudaEventRecord(ev.bulk1, side);
         cudaEventRecord(ev.sync, side);
     } else if (overlap && step + 1 <= d.nstep) {
         // bulk of step+1 (k >= 3) needs the states up to step-1 only: run it on
         // the side stream while this step's GMRES runs; the next head waits.
         const int kc1 = step + 1 < d.K ? step + 1 : d.K;
         if (ev.prev_gm) cudaStreamWaitEvent(side, ev.prev_gm, 0);
-        cudaEventRecord(ev.bulk0, side);
         if (kc1 >= 3) {
             MarchData db = d0;
             db.k_lo = 3;
@@ -1249,7 +1270,6 @@ cudaError_t step_r(const MarchData& d0, int step, cudaStream_t s, cudaStream_t s
                         : launch_rhs<R, false>(db, step + 1, true, 0, side);
             if (e != cudaSuccess) return e;
         }
-        cudaEventRecord(ev.bulk1, side);
         cudaEventRecord(ev.sync, side);
         cudaStreamWaitEvent(s, ev.sync, 0);
     }

@@ -44,3 +44,23 @@ def test_rows_pass_equals_one_step(n, nstep, beta, steps, precision, mark):
         assert a[2].history_launches < b[2].history_launches
     for x, y in zip(a[:2], b[:2]):
         assert np.max(np.abs(x - y)) <= mark * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("overlap", ["1", "0"])
+def test_phase_times_add_up(overlap):
+    """Head, GMRES and history times come from the device clock: on the chain, head
+    and GMRES do not overlap (1 us of clock granularity a step and phase allowed)."""
+    from tdbem import cases
+    from tdbem.api import MultiDomainSolver
+    c = cases.config_bar8(nstep=30, n=3)
+    s = MultiDomainSolver(c)
+    s.assemble()
+    os.environ["TDBEM_OVERLAP"] = overlap
+    try:
+        rep = s.march(c.known[0])[2]
+    finally:
+        os.environ.pop("TDBEM_OVERLAP")
+    head = rep.ms_rhs - rep.ms_history
+    assert rep.ms_gmres > 0 and head > 0 and rep.ms_history > 0
+    chain = rep.ms_gmres + head + (rep.ms_history if overlap == "0" else 0.0)
+    assert chain <= rep.ms_total + 3e-3 * c.nstep
