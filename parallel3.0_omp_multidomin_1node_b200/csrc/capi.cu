@@ -857,7 +857,7 @@ void bisect_rows(const std::vector<double>& node, int32_t* b, int32_t* e, int G)
 // size on, the L2's: what fits there the one-step pass reads fast enough to hide
 // beside GMRES, and the longer head costs more than it saves.  Steps of bars
 // with one load case, one-step -> T = 2: 0.02 GB 86.9 -> 88.2 us, 0.19 GB 129.6 ->
-// 126.8, 0.44 GB 145.4 -> 139.0, 0.82 GB 197.8 -> 185, 1.68 GB 339 -> 200.
+// 126.8, 0.44 GB 145.4 -> 139.0, 0.82 GB 197.8 -> 185, 1.68 GB 339 -> 200 (169 now).
 constexpr double kRowsPassBytes = 126e6;
 double history_bytes(const tdbem_handle* h)
 {

@@ -538,14 +538,15 @@ __global__ void __launch_bounds__(kRhsThreads, 2) bulk_steps_kernel(MarchData d,
 // of blocks, the one-step pass took 270 us a step, more than the GMRES it runs
 // beside (223 us), and a step 339 us; with T = 2 a step takes 218 us (mixed
 // precision: 201 -> 168).  T = 3 is slower (230), as the head then reads 14% of
-// the blocks on the chain instead of 6%.  Of 256 to 1,024 threads with 1 to 3
-// blocks in flight each, 256 with 3 at two CTAs per SM was fastest in both.  Each
+// the blocks on the chain instead of 6%.  Of 128 to 1,024 threads with 1 to 8
+// blocks in flight each, 256 with 4 (3 FP32) at two CTAs per SM was fastest: beside
+// GMRES scheduled with the head, a step takes 169 us, 195 with 3. Each
 // GMRES launch of the T has a T-th of the rows beside it (launched as one, a pass
 // held up the next head and GMRES for an SM: 218 -> 206 us with the head above).
 template <bool kMixed, int T>
 __global__ void __launch_bounds__(kRhsThreads, 2) bulk_rows_kernel(MarchData d, int t0, int p0, int part)
 {
-    constexpr int NW = kRhsThreads / 32, kUnroll = 3;
+    constexpr int NW = kRhsThreads / 32, kUnroll = T > 2 || kMixed ? 3 : 4;
     extern __shared__ int slot_of_k[];  // slot of W_{t0-k}
     __shared__ double red[NW][T][3];
     stamp_start(d, t0 + part, 3);
