@@ -31,15 +31,16 @@ __global__ void hist_keys_kernel(int E, int K, int nh, const int64_t* kptr, cons
     }
 }
 
-// Gather rows and values (9 planes -> 9 consecutive doubles) in group order.
-__global__ void hist_gather_kernel(int64_t nnz, const uint32_t* order, const int32_t* rowof, const double* hval,
-                                   int32_t* trow, double* tval)
+// Gather rows and values in group order: k << 21 | row, and tiles of 32 blocks in
+// 9 planes.
+__global__ void hist_gather_kernel(int64_t nnz, int K, const uint32_t* key, const uint32_t* order, const int32_t* rowof,
+                                   const double* hval, uint32_t* trow, double* tval)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = order[i];
-        trow[i] = rowof[j];
+        trow[i] = (key[i] % (uint32_t)(K + 1)) << 21 | (uint32_t)rowof[j];
 #pragma unroll
-        for (int q = 0; q < 9; ++q) tval[9 * i + q] = hval[(int64_t)q * nnz + j];
+        for (int q = 0; q < 9; ++q) tval[(i >> 5) * 288 + 32 * q + (i & 31)] = hval[(int64_t)q * nnz + j];
     }
 }
 
@@ -61,10 +62,10 @@ struct Scratch {
 }  // namespace
 
 cudaError_t adjoint_history_groups(int E, int K, int nh, int64_t nnz, const int64_t* kptr, const uint32_t* hcol,
-                                   const double* hval, int64_t* tptr, int32_t* trow, double* tval, cudaStream_t s)
+                                   const double* hval, int64_t* tptr, uint32_t* trow, double* tval, cudaStream_t s)
 {
     const int64_t groups = 2LL * nh * (K + 1);
-    if (nnz >= (1LL << 31) || groups >= (1LL << 31)) return cudaErrorInvalidValue;
+    if (nnz >= (1LL << 31) || groups >= (1LL << 31) || E > (1 << 21)) return cudaErrorInvalidValue;
     int end_bit = 1;
     while (end_bit < 32 && (1LL << end_bit) < groups) ++end_bit;
     const size_t n = (size_t)std::max<int64_t>(nnz, 1);
@@ -95,7 +96,7 @@ cudaError_t adjoint_history_groups(int E, int K, int nh, int64_t nnz, const int6
     if (nnz > 0) {
         ADJ_TRY(cub::DeviceRadixSort::SortPairs(temp.p, sort_bytes, k1, k2, i1, i2, (int)nnz, 0, end_bit, s));
         const int grid = (int)std::min<int64_t>(ceil_div(nnz, 256), 8 * 148);
-        hist_gather_kernel<<<grid, 256, 0, s>>>(nnz, i2, static_cast<int32_t*>(rowof.p), hval, trow, tval);
+        hist_gather_kernel<<<grid, 256, 0, s>>>(nnz, K, k2, i2, static_cast<int32_t*>(rowof.p), hval, trow, tval);
         ADJ_TRY(cudaGetLastError());
     }
     // the scratch is released when this returns: wait for its last use
@@ -108,79 +109,95 @@ namespace tdbem {
 
 namespace {
 
-// Transposed write-back of reverse step n: the cotangents of the global-frame
-// outputs of step n plus the history adjoint go back through LocToAbs and the
-// GlobalDofMap references; prescribed entries add to gk, unknown entries are
-// left per (element, U/T) in contrib for adj_unknown_kernel.
-__global__ void adj_writeback_kernel(AdjWriteBack a, int n)
+// Cotangent of element i's displacement (which = 0) or traction (1) reference at
+// step n in its local frame: that of the global-frame output plus the history
+// adjoint, back through LocToAbs.
+__device__ __forceinline__ void reference_cotangent(const AdjWriteBack& a, int n, int64_t i, int which, double (&cl)[3])
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.E) return;
     const int64_t o = ((int64_t)n * a.E + i) * 3;
-    double cu[3], ct[3];
-    for (int c = 0; c < 3; ++c) {
-        cu[c] = a.cot_lu ? a.cot_lu[o + c] : 0.0;
-        ct[c] = a.cot_lt ? a.cot_lt[o + c] : 0.0;
-    }
+    const double* cot = which ? a.cot_lt : a.cot_lu;
+    double cg[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) cg[c] = cot ? cot[o + c] : 0.0;
     if (a.adj && a.hist_owner[i]) {
-        const int64_t hb = a.hist_block[i];
-        for (int c = 0; c < 3; ++c) {
-            cu[c] += a.hu_sign[i] * a.adj[3 * hb + c];
-            ct[c] += a.ht_sign[i] * a.adj[3 * (a.nh + hb) + c];
-        }
+        const double* adj = a.adj + 3 * ((which ? (int64_t)a.nh : 0) + a.hist_block[i]);
+        const double sg = which ? a.ht_sign[i] : a.hu_sign[i];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cg[c] += sg * adj[c];
     }
-    const double* F = a.trans + 9 * i;
-    const double* T = a.itf_trans + 9 * i;
-    for (int which = 0; which < 2; ++which) {
-        const double* cg = which ? ct : cu;
-        double cl[3];  // gu = F^T l  ->  dl = F dgu
-        for (int j = 0; j < 3; ++j) cl[j] = F[3 * j] * cg[0] + F[3 * j + 1] * cg[1] + F[3 * j + 2] * cg[2];
-        const bool known = which ? a.tref_known[i] : a.uref_known[i];
-        const double sg = which ? a.tref_sign[i] : a.uref_sign[i];
-        double* cv = a.contrib + (2 * i + which) * 3;
-        if (known) {
-            for (int c = 0; c < 3; ++c) a.gk[o + c] += sg * cl[c];
-            for (int c = 0; c < 3; ++c) cv[c] = 0.0;
-        } else {
-            for (int j = 0; j < 3; ++j) cv[j] = sg * (T[j] * cl[0] + T[3 + j] * cl[1] + T[6 + j] * cl[2]);
-        }
-    }
+    const double* F = a.trans + 9 * i;  // gu = F^T l  ->  dl = F dgu
+#pragma unroll
+    for (int j = 0; j < 3; ++j) cl[j] = F[3 * j] * cg[0] + F[3 * j + 1] * cg[1] + F[3 * j + 2] * cg[2];
 }
 
-// Right-hand side of the transposed solve in perm (A' column) order: unknown
-// u = unk_of[p] sums its (at most two) sources in element order.
-__global__ void adj_unknown_kernel(int E, const int32_t* unk_src, const int32_t* unk_of, const double* contrib,
-                                   double* gp)
+// Transposed write-back of reverse step n, a thread per element and perm (A'
+// column) row t: prescribed references of element t add to gk, and the unknown of
+// row t sums its (at most two) references in element order into the right-hand
+// side of the transposed solve.  The solve's status word is cleared here, and the
+// solve sets up beside this launch.
+__global__ void adj_writeback_kernel(AdjWriteBack a, int n, const int32_t* unk_src, const int32_t* unk_of, double* gp,
+                                     int* status)
 {
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= E) return;
-    const int64_t u = unk_of[p];
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) *status = 0;
+    if (t >= a.E) return;
+    for (int which = 0; which < 2; ++which) {
+        if (!(which ? a.tref_known[t] : a.uref_known[t])) continue;
+        double cl[3];
+        reference_cotangent(a, n, t, which, cl);
+        const double sg = which ? a.tref_sign[t] : a.uref_sign[t];
+        double* g = a.gk + ((int64_t)n * a.E + t) * 3;
+        for (int c = 0; c < 3; ++c) g[c] += sg * cl[c];
+    }
+    const int64_t u = unk_of[t];
     double g[3] = {0.0, 0.0, 0.0};
     for (int k = 0; k < 2; ++k) {
         const int src = unk_src[2 * u + k];
         if (src < 0) continue;
-        for (int c = 0; c < 3; ++c) g[c] += contrib[3 * (int64_t)src + c];
+        const int64_t i = src >> 1;
+        const int which = src & 1;
+        double cl[3];
+        reference_cotangent(a, n, i, which, cl);
+        const double sg = which ? a.tref_sign[i] : a.uref_sign[i];
+        const double* T = a.itf_trans + 9 * i;
+        for (int j = 0; j < 3; ++j) g[j] += sg * (T[j] * cl[0] + T[3 + j] * cl[1] + T[6 + j] * cl[2]);
     }
-    for (int c = 0; c < 3; ++c) gp[3 * p + c] = g[c];
+    for (int c = 0; c < 3; ++c) gp[3 * t + c] = g[c];
 }
 
-// KnownM^T lam_n into the prescribed-value gradient: known block kb sums its
-// column's blocks in row order.
-__global__ void adj_known_kernel(int n_known, const int32_t* kt_ptr, const int32_t* kt_row, const int32_t* kt_blk,
-                                 const double* k_val, const int32_t* known_elem, const double* known_sign,
-                                 const double* lam, double* gk)
+// After the solve of step n: lam_n (equation rows) from x (perm rows), the sums
+// com_m = lam_{m-1} + 2 lam_m + lam_{m+1} of what is known by now, and KnownM^T
+// lam_n into the prescribed-value gradient, a warp per known block.
+__global__ void __launch_bounds__(256) adj_finish_kernel(AdjFinish a, int n, int rows_ctas)
 {
-    const int kb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kb >= n_known) return;
+    const int64_t per = 3LL * a.E;
+    if ((int)blockIdx.x < rows_ctas) {
+        const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (t >= per) return;
+        const double l = a.x[3LL * a.perm_of_row[t / 3] + t % 3];
+        a.lam[n * per + t] = l;
+        a.com[n * per + t] = 2.0 * l + a.lam[(n + 1) * per + t];
+        a.com[(n + 1) * per + t] += l;
+        return;
+    }
+    const int kb = ((int)blockIdx.x - rows_ctas) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (kb >= a.n_known) return;
     double acc[3] = {0.0, 0.0, 0.0};
-    for (int j = kt_ptr[kb]; j < kt_ptr[kb + 1]; ++j) {
-        const double* B = k_val + 9 * (int64_t)kt_blk[j];
-        const double* l = lam + 3 * (int64_t)kt_row[j];
+    for (int j = a.kt_ptr[kb] + lane; j < a.kt_ptr[kb + 1]; j += 32) {
+        const double* B = a.k_val + 9 * (int64_t)a.kt_blk[j];
+        const double* l = a.x + 3LL * a.perm_of_row[a.kt_row[j]];
+#pragma unroll
         for (int c = 0; c < 3; ++c) acc[c] += B[c] * l[0] + B[3 + c] * l[1] + B[6 + c] * l[2];
     }
-    const double sg = known_sign[kb];
-    double* g = gk + 3 * (int64_t)known_elem[kb];
-    for (int c = 0; c < 3; ++c) g[c] += sg * acc[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (lane == 0) {
+        double* g = a.gk + ((int64_t)n * a.E + a.known_elem[kb]) * 3;
+        for (int c = 0; c < 3; ++c) g[c] += a.known_sign[kb] * acc[c];
+    }
 }
 
 // Step 0 of the gradient: bd[0] is the prescribed value converted to the
@@ -208,22 +225,16 @@ cudaError_t adjoint_step0(int E, const double* trans, const int32_t* bcid, const
 }
 
 cudaError_t adjoint_writeback(const AdjWriteBack& a, int n, const int32_t* unk_src, const int32_t* unk_of, double* gp,
-                              cudaStream_t s)
+                              int* status, cudaStream_t s)
 {
-    adj_writeback_kernel<<<ceil_div(a.E, 128), 128, 0, s>>>(a, n);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    adj_unknown_kernel<<<ceil_div(a.E, 128), 128, 0, s>>>(a.E, unk_src, unk_of, a.contrib, gp);
+    adj_writeback_kernel<<<ceil_div(a.E, 64), 64, 0, s>>>(a, n, unk_src, unk_of, gp, status);
     return cudaGetLastError();
 }
 
-cudaError_t adjoint_known(int n_known, const int32_t* kt_ptr, const int32_t* kt_row, const int32_t* kt_blk,
-                          const double* k_val, const int32_t* known_elem, const double* known_sign, const double* lam,
-                          double* gk, cudaStream_t s)
+cudaError_t adjoint_finish(const AdjFinish& a, int n, cudaStream_t s)
 {
-    if (n_known <= 0) return cudaSuccess;
-    adj_known_kernel<<<ceil_div(n_known, 128), 128, 0, s>>>(n_known, kt_ptr, kt_row, kt_blk, k_val, known_elem,
-                                                            known_sign, lam, gk);
+    const int rows = ceil_div(3LL * a.E, 256);
+    adj_finish_kernel<<<rows + ceil_div(a.n_known, 8), 256, 0, s>>>(a, n, rows);
     return cudaGetLastError();
 }
 

@@ -385,14 +385,14 @@ struct AdjointState {
     GmresTiles tiles;                               // A'^T for the GMRES cluster of cta_row
     std::vector<int32_t> cta_row;
     DevBuf tptr, trow, tval;                        // history blocks by (type, column), then k
-    DevBuf lam, adj, gp;                            // adjoint right-hand sides, state adjoint, solve rhs
+    DevBuf lam, com, adj, gp;                       // adjoint vectors and their sums, state adjoint, solve rhs
     DevBuf x, rv, aw, u, V, givens, status, flags;
     DevBuf unk_of, perm_of_row;
     DevBuf unk_src, kt_ptr, kt_row, kt_blk;         // write-back sources per unknown; KnownM by columns
-    DevBuf cot_u, cot_t, gk, contrib, flags_all;    // per-call cotangents, gradient, scratch, per-step flags
+    DevBuf cot_u, cot_t, gk, flags_all;             // per-call cotangents, gradient, per-step flags
 };
 
-// CUDA events a handle reuses from march to march (a march records seven
+// CUDA events a handle reuses from march to march (a march records two
 // per time step, the host-buffer march two per copy chunk): created on first
 // need, grown on demand, destroyed with the handle.
 struct EventPool {
@@ -3017,12 +3017,6 @@ tdbem_status tdbem_md_load_matrix_cache(tdbem_handle* h, const char* path, void*
 // The march is linear in the prescribed values, so no forward state is kept.
 namespace {
 
-__global__ void gather_blocks(int E, const int32_t* idx, const double* in, double* out)
-{
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 3LL * E; t += (int64_t)gridDim.x * blockDim.x)
-        out[t] = in[3LL * idx[t / 3] + t % 3];
-}
-
 tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
 {
     auto A = std::make_unique<AdjointState>();
@@ -3063,9 +3057,9 @@ tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
     const int64_t hn = std::max<int64_t>(h->h_nnz, 1);
     CUDA_TRY(A->tptr.alloc(sizeof(int64_t) * 2 * (size_t)nh * (K + 1)));
     CUDA_TRY(A->trow.alloc(sizeof(int32_t) * (size_t)hn));
-    CUDA_TRY(A->tval.alloc(sizeof(double) * 9 * (size_t)hn));
+    CUDA_TRY(A->tval.alloc(sizeof(double) * 288 * (size_t)((hn + 31) / 32)));
     CUDA_TRY(adjoint_history_groups((int)E, K, (int)nh, h->h_nnz, h->d_h_kptr.as<int64_t>(), h->d_h_col.as<uint32_t>(),
-                                    h->d_h_val.as<double>(), A->tptr.as<int64_t>(), A->trow.as<int32_t>(),
+                                    h->d_h_val.as<double>(), A->tptr.as<int64_t>(), A->trow.as<uint32_t>(),
                                     A->tval.as<double>(), s));
     CUDA_TRY(up(A->unk_of, unk_of, s));
     CUDA_TRY(up(A->perm_of_row, perm_of_row, s));
@@ -3102,7 +3096,6 @@ tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
         CUDA_TRY(up(A->kt_blk, blk, s));
         const size_t per = 3 * (size_t)E;
         for (DevBuf* b : {&A->cot_u, &A->cot_t, &A->gk}) CUDA_TRY(b->alloc(sizeof(double) * per * (h->nstep + 1)));
-        CUDA_TRY(A->contrib.alloc(sizeof(double) * 2 * per));
         CUDA_TRY(A->flags_all.alloc(sizeof(int) * 3 * (size_t)std::max(h->nstep, 1)));
     }
     // GMRES storage for one load case
@@ -3114,6 +3107,7 @@ tdbem_status adjoint_setup(tdbem_handle* h, cudaStream_t s)
     CUDA_TRY(A->status.alloc(sizeof(int) * 4));
     CUDA_TRY(A->flags.alloc(sizeof(int) * 4));
     CUDA_TRY(A->lam.alloc(sizeof(double) * 3 * (size_t)E * (h->nstep + 2)));
+    CUDA_TRY(A->com.alloc(sizeof(double) * 3 * (size_t)E * (h->nstep + 2)));
     CUDA_TRY(A->adj.alloc(sizeof(double) * 6 * (size_t)nh));
     CUDA_TRY(cudaStreamSynchronize(s));
     h->adjoint = std::move(A);
@@ -3175,6 +3169,7 @@ tdbem_status tdbem_md_march_vjp(tdbem_handle* h, const double* cot_lu, const dou
     d.cluster = h->cluster;
     d.givens_stride = gmres_givens_doubles(h->restart);
     CUDA_TRY(cudaMemsetAsync(A.lam.p, 0, A.lam.bytes, s));
+    CUDA_TRY(cudaMemsetAsync(A.com.p, 0, A.com.bytes, s));
     // the reverse march runs on the device without host round trips:
     // cotangents in, transposed write-back, A'^T solve, KnownM^T, history
     // adjoint; GMRES flags per step are read once at the end
@@ -3199,27 +3194,25 @@ tdbem_status tdbem_md_march_vjp(tdbem_handle* h, const double* cot_lu, const dou
     wb.uref_known = h->d_uref_known.as<int32_t>();
     wb.tref_known = h->d_tref_known.as<int32_t>();
     wb.gk = A.gk.as<double>();
-    wb.contrib = A.contrib.as<double>();
+    const AdjFinish fin{(int)E, (int)h->n_known, A.x.as<double>(), A.perm_of_row.as<int32_t>(), A.lam.as<double>(),
+                        A.com.as<double>(), A.kt_ptr.as<int32_t>(), A.kt_row.as<int32_t>(), A.kt_blk.as<int32_t>(),
+                        h->d_k_val.as<double>(), h->d_known_elem.as<int32_t>(), h->d_known_sign.as<double>(),
+                        A.gk.as<double>()};
+    d.after_head = 1;  // the solve sets up beside the write-back
     tdbem_report rep{};
-    const int grid = (int)std::min<int64_t>(ceil_div(3 * E, 256), 4 * 148);
     for (int n = N; n >= 1; --n) {
         wb.adj = nullptr;
         if (n < N && nh > 0) {
-            CUDA_TRY(adj_history(N, n, K, (int)nh, (int)E, A.tptr.as<int64_t>(), A.trow.as<int32_t>(),
-                                 A.tval.as<double>(), A.lam.as<double>(), A.adj.as<double>(), s));
+            CUDA_TRY(adj_history(N, n, K, (int)nh, (int)E, A.tptr.as<int64_t>(), A.trow.as<uint32_t>(),
+                                 A.tval.as<double>(), A.com.as<double>(), A.adj.as<double>(), s));
             wb.adj = A.adj.as<double>();
         }
         // lam_n = A^-T g: write-back transposed into A'^T rows, solve, equation rows
-        CUDA_TRY(adjoint_writeback(wb, n, A.unk_src.as<int32_t>(), A.unk_of.as<int32_t>(), A.gp.as<double>(), s));
-        CUDA_TRY(cudaMemsetAsync(A.status.p, 0, A.status.bytes, s));
+        CUDA_TRY(adjoint_writeback(wb, n, A.unk_src.as<int32_t>(), A.unk_of.as<int32_t>(), A.gp.as<double>(),
+                                   A.status.as<int>(), s));
         d.step_flags = A.flags_all.as<int>() + 3 * (size_t)(n - 1);
         CUDA_TRY(gmres_solve_single(d, s));
-        double* lam_n = A.lam.as<double>() + (size_t)n * per;
-        gather_blocks<<<grid, 256, 0, s>>>((int)E, A.perm_of_row.as<int32_t>(), A.x.as<double>(), lam_n);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(adjoint_known((int)h->n_known, A.kt_ptr.as<int32_t>(), A.kt_row.as<int32_t>(),
-                               A.kt_blk.as<int32_t>(), h->d_k_val.as<double>(), h->d_known_elem.as<int32_t>(),
-                               h->d_known_sign.as<double>(), lam_n, A.gk.as<double>() + (size_t)n * per, s));
+        CUDA_TRY(adjoint_finish(fin, n, s));
     }
     // step 0: bd[0] converted to the global frame (lu for BCID 123, lt for 456)
     CUDA_TRY(adjoint_step0((int)E, h->g_trans.as<double>(), h->g_bcid.as<int32_t>(), wb.cot_lu, wb.cot_lt,

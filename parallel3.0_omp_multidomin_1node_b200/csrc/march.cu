@@ -913,37 +913,33 @@ __global__ void __launch_bounds__(kRhsThreads, R >= 8 ? 2 : 3) rhs_models_kernel
 //   Omega_{n,k} = lam_{n+k-1} (k >= 2) + 2 lam_{n+k} + lam_{n+k+1}, steps <= N,
 // the transpose of the forward sum over k of B . (X_{s-k+1} + 2 X_{s-k} +
 // X_{s-k-1}) (DBEM1/multidomain.cpp:3201-3225, 3843-3866) with B the stacked
-// blocks (MTS negated).  Column-major view: one warp per (type, column), its
-// blocks ordered by k.
-__global__ void __launch_bounds__(256) adj_history_kernel(int N, int n, int K, int nh, int E, const int64_t* tptr,
-                                                          const int32_t* trow, const double* tval, const double* lam,
-                                                          double* adj)
+// blocks (MTS negated).  Omega_{n,k} is row n + k of com, which adjoint_finish
+// keeps so.  What bounds it: latency, then L2 bandwidth (76 bytes and one vector a
+// block).  Four warps take a (type, column) pair's blocks of all k as one list; a
+// warp that went through k by k, with three vectors a block, took 97 us a step of
+// 480 elements (509,000 blocks) with cold caches, 15 now.
+__global__ void __launch_bounds__(256, 3) adj_history_kernel(int N, int n, int K, int nh, int E, const int64_t* tptr,
+                                                             const uint32_t* trow, const double* tval, const double* com,
+                                                             double* adj)
 {
-    const int64_t seg = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (seg >= 2LL * nh) return;
+    constexpr int kWarps = 4;  // per pair
+    __shared__ double red[8][3];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, part = w % kWarps;
+    const int64_t seg = (int64_t)blockIdx.x * (8 / kWarps) + w / kWarps;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int k = 1; k <= K; ++k) {
-        const int64_t b = tptr[seg * (K + 1) + k - 1], e = tptr[seg * (K + 1) + k];
-        if (b == e) continue;
-        const int m0 = n + k - 1, m1 = n + k, m2 = n + k + 1;
-        const double c0 = (k >= 2 && m0 <= N) ? 1.0 : 0.0, c1 = m1 <= N ? 2.0 : 0.0, c2 = m2 <= N ? 1.0 : 0.0;
-        if (c0 == 0.0 && c1 == 0.0 && c2 == 0.0) continue;
-        for (int64_t j = b + lane; j < e; j += 32) {
-            const int64_t r = trow[j];
-            double w[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double v = 0.0;
-                if (c0 != 0.0) v += lam[((int64_t)m0 * E + r) * 3 + c];
-                if (c1 != 0.0) v += c1 * lam[((int64_t)m1 * E + r) * 3 + c];
-                if (c2 != 0.0) v += lam[((int64_t)m2 * E + r) * 3 + c];
-                w[c] = v;
-            }
-            const double* B = tval + 9 * j;  // row-major B; B^T w
-            a0 += B[0] * w[0] + B[3] * w[1] + B[6] * w[2];
-            a1 += B[1] * w[0] + B[4] * w[1] + B[7] * w[2];
-            a2 += B[2] * w[0] + B[5] * w[1] + B[8] * w[2];
+    if (seg < 2LL * nh) {
+        const int kmax = K < N + 1 - n ? K : N + 1 - n;  // later rows of com are zero
+        const int64_t b = tptr[seg * (K + 1)], e = tptr[seg * (K + 1) + kmax];
+        const double* w0 = com + 3LL * n * E;
+#pragma unroll 4
+        for (int64_t j = b + part * 32 + lane; j < e; j += 32 * kWarps) {
+            const uint32_t kr = __ldg(trow + j);  // k << 21 | row
+            const double* x = w0 + 3 * ((int64_t)(kr >> 21) * E + (kr & 0x1FFFFFu));
+            const double* B = tval + (j >> 5) * 288 + (j & 31);  // row-major B in planes; B^T x
+            const double x0 = x[0], x1 = x[1], x2 = x[2];
+            a0 += __ldg(B) * x0 + __ldg(B + 96) * x1 + __ldg(B + 192) * x2;
+            a1 += __ldg(B + 32) * x0 + __ldg(B + 128) * x1 + __ldg(B + 224) * x2;
+            a2 += __ldg(B + 64) * x0 + __ldg(B + 160) * x1 + __ldg(B + 256) * x2;
         }
     }
 #pragma unroll
@@ -953,17 +949,24 @@ __global__ void __launch_bounds__(256) adj_history_kernel(int N, int n, int K, i
         a2 += __shfl_xor_sync(0xffffffffu, a2, o);
     }
     if (lane == 0) {
-        adj[3 * seg] = a0;
-        adj[3 * seg + 1] = a1;
-        adj[3 * seg + 2] = a2;
+        red[w][0] = a0;
+        red[w][1] = a1;
+        red[w][2] = a2;
+    }
+    __syncthreads();
+    if (part == 0 && lane < 3 && seg < 2LL * nh) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < kWarps; ++q) s += red[w + q][lane];
+        adj[3 * seg + lane] = s;
     }
 }
 
-cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr, const int32_t* trow,
-                        const double* tval, const double* lam, double* adj, cudaStream_t s)
+cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr, const uint32_t* trow,
+                        const double* tval, const double* com, double* adj, cudaStream_t s)
 {
     const int64_t segs = 2LL * nh;
-    adj_history_kernel<<<(int)((segs + 7) / 8), 256, 0, s>>>(N, n, K, nh, E, tptr, trow, tval, lam, adj);
+    adj_history_kernel<<<(int)((segs + 1) / 2), 256, 0, s>>>(N, n, K, nh, E, tptr, trow, tval, com, adj);
     return cudaGetLastError();
 }
 

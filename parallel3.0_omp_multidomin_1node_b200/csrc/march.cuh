@@ -297,9 +297,10 @@ cudaError_t rhs_split(const RhsSplitArgs& a, cudaStream_t s);
 
 // The stacked history blocks regrouped for adj_history: tptr [2 nh (K+1)]
 // group ends, group (type * nh + column) * (K + 1) + k in ascending row order;
-// trow, tval [nnz] and [nnz][9].  Synchronises the stream.
+// trow [nnz] k << 21 | row, tval tiles of 32 blocks in 9 planes.  Synchronises the
+// stream.
 cudaError_t adjoint_history_groups(int E, int K, int nh, int64_t nnz, const int64_t* kptr, const uint32_t* hcol,
-                                   const double* hval, int64_t* tptr, int32_t* trow, double* tval, cudaStream_t s);
+                                   const double* hval, int64_t* tptr, uint32_t* trow, double* tval, cudaStream_t s);
 // Transposed write-back of one reverse step (adjoint march), device arrays.
 struct AdjWriteBack {
     int E, nh;
@@ -317,24 +318,34 @@ struct AdjWriteBack {
     const int32_t* uref_known;
     const int32_t* tref_known;
     double* gk;                // [N+1][E][3] prescribed-value gradient (added to)
-    double* contrib;           // [E][2][3] scratch
 };
-// Write-back of step n, then the transposed solve's right-hand side gp in
-// perm order (unk_src: [E][2] (element * 2 + U/T) sources of each unknown,
-// -1 for none; unk_of: unknown of each perm row).
+// Write-back of step n to the transposed solve's right-hand side gp in perm order
+// (unk_src: [E][2] (element * 2 + U/T) sources of each unknown, -1 for none;
+// unk_of: unknown of each perm row); clears *status.
 cudaError_t adjoint_writeback(const AdjWriteBack& a, int n, const int32_t* unk_src, const int32_t* unk_of, double* gp,
-                              cudaStream_t s);
+                              int* status, cudaStream_t s);
+// What follows the transposed solve of a reverse step, device arrays.
+struct AdjFinish {
+    int E, n_known;
+    const double* x;             // [E][3] solution, perm rows
+    const int32_t* perm_of_row;
+    double* lam;                 // [N+2][E][3] by equation rows; rows past the last step zero
+    double* com;                 // [N+2][E][3] lam_{m-1} + 2 lam_m + lam_{m+1}, so far
+    const int32_t* kt_ptr;       // [n_known+1] KnownM by columns, in row order: kt_row, kt_blk (block
+    const int32_t* kt_row;       // of k_val, 9 doubles row-major)
+    const int32_t* kt_blk;
+    const double* k_val;
+    const int32_t* known_elem;
+    const double* known_sign;
+    double* gk;                  // [N+1][E][3] prescribed-value gradient (added to)
+};
+cudaError_t adjoint_finish(const AdjFinish& a, int n, cudaStream_t s);
 // gk (step 0) += the cotangent of bd[0] through the local frame (lu for BCID
 // 123, lt for 456); cot_* are the device cotangents of step 0 (or null).
 cudaError_t adjoint_step0(int E, const double* trans, const int32_t* bcid, const double* cot_lu, const double* cot_lt,
                           double* gk, cudaStream_t s);
-// gk (one step) += KnownM^T lam by columns: kt_ptr [n_known+1], kt_row and
-// kt_blk (block index into k_val, 9 doubles row-major) in row order.
-cudaError_t adjoint_known(int n_known, const int32_t* kt_ptr, const int32_t* kt_row, const int32_t* kt_blk,
-                          const double* k_val, const int32_t* known_elem, const double* known_sign, const double* lam,
-                          double* gk, cudaStream_t s);
-cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr, const int32_t* trow,
-                        const double* tval, const double* lam, double* adj, cudaStream_t s);
+cudaError_t adj_history(int N, int n, int K, int nh, int E, const int64_t* tptr, const uint32_t* trow,
+                        const double* tval, const double* com, double* adj, cudaStream_t s);
 // Shared memory of the GMRES kernel for Rg load cases per cluster, a row
 // capacity of `rows` (0: the global-memory form) and `halo` rows from other
 // CTAs, without cached leaf inverses and basis vectors; and whether that fits
