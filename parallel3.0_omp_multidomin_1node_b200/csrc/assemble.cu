@@ -25,14 +25,6 @@ namespace {
 
 __device__ __forceinline__ double ws(double v) { return qwarp_sum(v); }
 
-__device__ void load_rules(const QuadRules* g, QuadRules* s)
-{
-    const double* src = reinterpret_cast<const double*>(g);
-    double* dst = reinterpret_cast<double*>(s);
-    for (int i = threadIdx.x; i < (int)(sizeof(QuadRules) / sizeof(double)); i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
-}
-
 __device__ __forceinline__ void load_elem(const ElemGeom& g, int f, QElem& e)
 {
     e.cc = g.cc + 24 * (int64_t)f;
@@ -96,68 +88,62 @@ struct SelfBlocks {
     const S* t2;
 };
 
-// Step0 coefficient block with the effective BCID (RegularInt*Coef /
-// InElementInt*Coef with FlagDynaMethod 2); unknown = 1 for the kernel that
-// multiplies the unknown.  Warp-uniform; result valid on every lane.
+// Coefficients of steps 0 and 1 of a pair (RegularInt*Coef / InElementInt*Coef
+// with FlagDynaMethod 2), 4 (.)(0) + (.)(1), to k[0 .. 8] displacement and
+// k[9 .. 17] traction (T1 and, at step 0, T2); false: no wave reaches the element.
+// What bounds it: FP64 arithmetic.  Both come from one walk of pair_steps over the
+// two steps; evaluated one by one, up to six times per pair over every point, the
+// pairs of the 2,058-element bar took 14.9 ms, 1.7 now.
 template <class MT, class S = typename MT::Scalar>
-__device__ bool step0_block(const QuadRules& q, const MT& M, const QElem& e, const double* trans9, bool self,
-                            const SelfBlocks<S>& sb, const double* src, int bcid, int unknown, S* out)
+__device__ __forceinline__ bool step0_sums(const QuadRules& rules, const MT& M, const PairTable& tb, PairWarp<S>& pw,
+                                           const QElem& e, bool self, const SelfBlocks<S>& sb, const double* src, S* k)
+{
+    const int lane = threadIdx.x & 31, l = lane < 9 ? lane : 0;
+    S ku = 0.0, kt = 0.0;
+    if (self) {
+        S u[9], t[9];
+        w_int_u_pw(rules, M, e, src, 1.0, u);
+        w_int_t_pw(rules, M, e, 1, src, 1.0, t);
+        if (lane == 0)
+            for (int i = 0; i < 9; ++i) {
+                k[i] = 4.0 * sb.u1[i] + u[i];
+                k[9 + i] = 4.0 * sb.t1[i] + sb.t2[i] + t[i];
+            }
+        __syncwarp();
+        return true;
+    }
+    const PairClass cls(M, e.center, e.radius, src);
+    if (cls(0) == 0 && cls(1) == 0) return false;
+    pair_steps(M, tb, pw, e, src, false, 0, 1, [&](int step, int c2, int c1, const S* t2, const S* t1, const S* u) {
+        if (step == 0) {
+            if (c1) {
+                ku = 4.0 * u[sym6(l)];
+                kt = 4.0 * t1[l];
+            }
+        } else {
+            if (c2) kt += t2[l];
+            if (c1) {
+                ku += u[sym6(l)];
+                kt += t1[l];
+            }
+        }
+    });
+    if (lane < 9) {
+        k[lane] = ku;
+        k[9 + lane] = kt;
+    }
+    __syncwarp();
+    return true;
+}
+
+// Step0 coefficient block with the effective BCID; unknown = 1 for the kernel that
+// multiplies the unknown.  k: step0_sums.
+template <class S>
+__device__ __forceinline__ void step0_block(const S* k, const double* trans9, int bcid, int unknown, S* out)
 {
     const bool useU = unknown ? (bcid == 123) : (bcid == 456);
-    S K[9], t[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) K[i] = 0.0;
-    if (self) {
-        if (useU) {
-            for (int i = 0; i < 9; ++i) K[i] += 4.0 * sb.u1[i];
-            w_int_u_pw(q, M, e, src, 1.0, t);
-        } else {
-            for (int i = 0; i < 9; ++i) {
-                K[i] += 4.0 * sb.t1[i];
-                K[i] += sb.t2[i];
-            }
-            w_int_t_pw(q, M, e, 1, src, 1.0, t);
-        }
-#pragma unroll
-        for (int i = 0; i < 9; ++i) K[i] += t[i];
-    } else {
-        const int f0 = q_need_cal(M, e.center, e.radius, 1, 0.0, src);
-        int fsum = f0;
-        if (f0) {
-            if (useU) {
-                if (f0 == 1) w_int_u_pw(q, M, e, src, 0.0, t);
-                else w_int_u_regular(q, M, e, src, 0.0, t);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) K[i] += 4.0 * t[i];
-            } else {
-                if (f0 == 1) w_int_t_pw(q, M, e, 1, src, 0.0, t);
-                else w_int_t_regular(q, M, e, src, 0.0, t);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) K[i] += 4.0 * t[i];
-                if (f0 == 1) w_int_t_pw(q, M, e, 2, src, 1.0, t);
-                else w_int_t_regular(q, M, e, src, 1.0, t);
-#pragma unroll
-                for (int i = 0; i < 9; ++i) K[i] += t[i];
-            }
-        }
-        const int f1 = q_need_cal(M, e.center, e.radius, 1, 1.0, src);
-        fsum += f1;
-        if (f1) {
-            if (useU) {
-                if (f1 == 1) w_int_u_pw(q, M, e, src, 1.0, t);
-                else w_int_u_regular(q, M, e, src, 1.0, t);
-            } else {
-                if (f1 == 1) w_int_t_pw(q, M, e, 1, src, 1.0, t);
-                else w_int_t_regular(q, M, e, src, 1.0, t);
-            }
-#pragma unroll
-            for (int i = 0; i < 9; ++i) K[i] += t[i];
-        }
-        if (!fsum) return false;
-    }
     const double sign = unknown ? (bcid == 123 ? -1.0 : 1.0) : (bcid == 456 ? 1.0 : -1.0);
-    convert_block(K, trans9, sign, out);
-    return true;
+    convert_block(k + (useU ? 0 : 9), trans9, sign, out);
 }
 
 // The Step0 blocks of one (source s, field f) pair of a domain
@@ -165,9 +151,8 @@ __device__ bool step0_block(const QuadRules& q, const MT& M, const QElem& e, con
 // DBEM1/multidomain.cpp:2256-2327, 1594-1691): up to two A blocks (out0,
 // out1) and one KnownM block (out1 for outer elements), transposed and
 // signed; returns flags bit0 A0, bit1 A1, bit2 K.
-template <class MT, class S = typename MT::Scalar>
-__device__ uint8_t step0_pair(const QuadRules& q, const MT& M, const QElem& e, const ElemGeom& g, const DofRefs& dr,
-                              int f, bool self, const SelfBlocks<S>& sb, const double* src, S* out0, S* out1)
+template <class S>
+__device__ uint8_t step0_pair(const S* k, const ElemGeom& g, const DofRefs& dr, int f, S* out0, S* out1)
 {
     const double* tr = g.trans + 9 * (int64_t)f;
     S blk[9];
@@ -177,7 +162,8 @@ __device__ uint8_t step0_pair(const QuadRules& q, const MT& M, const QElem& e, c
         for (int pass = 0; pass < 2; ++pass) {
             const int bc = pass == 0 ? 456 : 123;
             const double sign = pass == 0 ? dr.uref_sign[f] : dr.tref_sign[f];
-            if (step0_block(q, M, e, tr, self, sb, src, bc, 1, blk)) {
+            step0_block(k, tr, bc, 1, blk);
+            {
                 // TransformColumnBlock9 then AddBlock's transpose
                 S tb[9];
                 for (int r = 0; r < 3; ++r)
@@ -196,7 +182,8 @@ __device__ uint8_t step0_pair(const QuadRules& q, const MT& M, const QElem& e, c
         }
     } else {
         const int bc = g.bcid[f];
-        if (step0_block(q, M, e, tr, self, sb, src, bc, 1, blk)) {
+        step0_block(k, tr, bc, 1, blk);
+        {
             const double sign = bc == 123 ? dr.tref_sign[f] : dr.uref_sign[f];
             if (sign != 0.0 && admit(blk)) {
                 for (int r = 0; r < 3; ++r)
@@ -204,7 +191,8 @@ __device__ uint8_t step0_pair(const QuadRules& q, const MT& M, const QElem& e, c
                 if (maxabs9(out0) > 1.0e-14) fl |= 1;
             }
         }
-        if (step0_block(q, M, e, tr, self, sb, src, bc, 0, blk)) {
+        step0_block(k, tr, bc, 0, blk);
+        {
             const double sign = bc == 123 ? dr.uref_sign[f] : dr.tref_sign[f];
             if (sign != 0.0 && admit(blk)) {
                 for (int r = 0; r < 3; ++r)
@@ -426,32 +414,68 @@ __global__ void __launch_bounds__(256) singular_kernel(int E, const QuadRules* r
     }
 }
 
+namespace {
+
+// CTA b's field element and sources: CTAs run over the domains' (chunk of
+// kPairSources sources, field element), fields fastest.
+__device__ __forceinline__ bool pair_cta(const PairSpace& ps, int64_t b, int& d, int& f, int& s0, int& s1)
+{
+    for (d = 0; d < ps.n_domains; ++d) {
+        const int nd = ps.dom_count[d];
+        const int64_t n = (int64_t)nd * ((nd + kPairSources - 1) / kPairSources);
+        if (b < n) {
+            f = ps.dom_begin[d] + (int)(b % nd);
+            s0 = (int)(b / nd) * kPairSources;
+            s1 = min(s0 + kPairSources, nd);
+            s0 += ps.dom_begin[d];
+            s1 += ps.dom_begin[d];
+            return true;
+        }
+        b -= n;
+    }
+    return false;
+}
+
+}  // namespace
+
 // ---------------------------------------------------------------------------
 // Step0 blocks, one warp per (source row, field element) pair of a domain:
 // up to two A blocks (slot 0, 1) and one KnownM block (slot 1 for outer
 // elements), already transposed and signed; flags bit0 A0, bit1 A1, bit2 K.
-__global__ void __launch_bounds__(128) step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr,
-                                                    double* blocks, uint8_t* flags)
+__global__ void __launch_bounds__(32 * kPairWarps, 2) step0_kernel(PairSpace ps, const QuadRules* rules,
+                                                                  const DynaMat* mats, ElemGeom g, DofRefs dr,
+                                                                  double* blocks, uint8_t* flags)
 {
-    __shared__ QuadRules q;
-    load_rules(rules, &q);
-    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (p >= ps.n_pairs) return;
-    const int lane = threadIdx.x & 31;
-    int d, s, f;
-    decode_pair(ps, p, d, s, f);
-    const DynaMat& M = c_mats[d];
+    extern __shared__ __align__(16) unsigned char pair_sm[];
+    __shared__ DynaMat M;
+    PairTable& tb = *reinterpret_cast<PairTable*>(pair_sm);
+    PairWarp<double>& pw = reinterpret_cast<PairWarp<double>*>(pair_sm + sizeof(PairTable))[threadIdx.x >> 5];
+    int d, f, s0, s1;
+    if (!pair_cta(ps, blockIdx.x, d, f, s0, s1)) return;
     QElem e;
     load_elem(g, f, e);
-    const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+    fill_table(tb, *rules, e.cc);
+    if (threadIdx.x == 0) M = mats[d];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nd = ps.dom_count[d], b = ps.dom_begin[d];
     const SelfBlocks<double> sb{g.on_u1 + 9 * (int64_t)f, g.on_t1 + 9 * (int64_t)f, g.on_t2 + 9 * (int64_t)f};
-    double out0[9], out1[9];
-    const uint8_t fl = step0_pair(q, M, e, g, dr, f, s == f, sb, src, out0, out1);
-    if (lane < 9) {
-        blocks[(p * 2 + 0) * 9 + lane] = (fl & 1) ? out0[lane] : 0.0;
-        blocks[(p * 2 + 1) * 9 + lane] = (fl & 6) ? out1[lane] : 0.0;
+    for (int s = s0 + (threadIdx.x >> 5); s < s1; s += kPairWarps) {
+        const int64_t p = ps.pair_off[d] + (int64_t)(s - b) * nd + (f - b);
+        const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+        uint8_t fl = 0;
+        if (step0_sums(*rules, M, tb, pw, e, s == f, sb, src, pw.out)) {
+            double out0[9], out1[9];
+            fl = step0_pair<double>(pw.out, g, dr, f, out0, out1);
+            if (lane == 0)
+#pragma unroll
+                for (int c = 0; c < 9; ++c) {
+                    if (fl & 1) blocks[(p * 2 + 0) * 9 + c] = out0[c];
+                    if (fl & 6) blocks[(p * 2 + 1) * 9 + c] = out1[c];
+                }
+            __syncwarp();
+        }
+        if (lane == 0) flags[p] = fl;
     }
-    if (lane == 0) flags[p] = fl;
 }
 
 // Steps k >= 1 in which a pair's history blocks can be nonzero (its T2 part is
@@ -484,30 +508,6 @@ __global__ void history_range_kernel(PairSpace ps, const DynaMat* mats, ElemGeom
     range[p] = ((uint32_t)first << 16) | (uint32_t)n;
     slots[p] = n;
 }
-
-namespace {
-
-// CTA b's field element and sources: CTAs run over the domains' (chunk of
-// kPairSources sources, field element), fields fastest.
-__device__ __forceinline__ bool pair_cta(const PairSpace& ps, int64_t b, int& d, int& f, int& s0, int& s1)
-{
-    for (d = 0; d < ps.n_domains; ++d) {
-        const int nd = ps.dom_count[d];
-        const int64_t n = (int64_t)nd * ((nd + kPairSources - 1) / kPairSources);
-        if (b < n) {
-            f = ps.dom_begin[d] + (int)(b % nd);
-            s0 = (int)(b / nd) * kPairSources;
-            s1 = min(s0 + kPairSources, nd);
-            s0 += ps.dom_begin[d];
-            s1 += ps.dom_begin[d];
-            return true;
-        }
-        b -= n;
-    }
-    return false;
-}
-
-}  // namespace
 
 int64_t pair_ctas(const PairSpace& ps, const int32_t* dom_count)
 {
@@ -982,46 +982,55 @@ __device__ __forceinline__ void contract_add(const QDual* B, const double* l, co
 // kernel blocks: an interface element's T column (slot 1), an outer
 // element's unknown column when its BCID is 123 and its known column when
 // it is 456.  part[2p], part[2p+1] = the pair's gE and gU.
-__global__ void __launch_bounds__(128) grad_step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr,
-                                                         const QDual* self_d, GradState gs, double* part)
+__global__ void __launch_bounds__(32 * kPairWarps) grad_step0_kernel(PairSpace ps, const QuadRules* rules,
+                                                                     const DynaMatD* mats, ElemGeom g, DofRefs dr,
+                                                                     const QDual* self_d, GradState gs, double* part)
 {
-    __shared__ QuadRules q;
-    load_rules(rules, &q);
-    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (p >= ps.n_pairs) return;
-    const int lane = threadIdx.x & 31;
-    int d, s, f;
-    decode_pair(ps, p, d, s, f);
-    const DynaMatD& M = c_dmats[d];
+    extern __shared__ __align__(16) unsigned char pair_sm[];
+    __shared__ DynaMatD M;
+    PairTable& tb = *reinterpret_cast<PairTable*>(pair_sm);
+    PairWarp<QDual>& pw = reinterpret_cast<PairWarp<QDual>*>(pair_sm + sizeof(PairTable))[threadIdx.x >> 5];
+    int d, f, s0, s1;
+    if (!pair_cta(ps, blockIdx.x, d, f, s0, s1)) return;
     QElem e;
     load_elem(g, f, e);
-    const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+    fill_table(tb, *rules, e.cc);
+    if (threadIdx.x == 0) M = mats[d];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nd = ps.dom_count[d], b = ps.dom_begin[d];
     const QDual* sd = self_d + 27 * (int64_t)f;
     const SelfBlocks<QDual> sb{sd, sd + 9, sd + 18};
-    QDual out0[9], out1[9];
-    const uint8_t fl = step0_pair(q, M, e, g, dr, f, s == f, sb, src, out0, out1);
     const bool surf = g.surface[f] != 0;
     const bool u0 = !surf && g.bcid[f] == 123, uk = !surf && g.bcid[f] == 456;
-    double ge = 0.0, gu = 0.0;
-    if (fl) {
-        const int64_t E3 = 3 * (int64_t)gs.E;
-        for (int n = 1 + lane; n <= gs.N; n += 32) {
-            const double* l = gs.lam + n * E3 + 3 * (int64_t)s;
-            const double* xn = gs.x + (int64_t)(n - 1) * E3;
-            if (fl & 1) contract_add(out0, l, xn + 3 * gs.col_a0[f], -1.0, u0, ge, gu);
-            if (fl & 2) contract_add(out1, l, xn + 3 * gs.col_a1[f], -1.0, true, ge, gu);
-            if (fl & 4) {
-                const int64_t kb = gs.col_k[f];
-                const double* kv = gs.known + ((int64_t)n * gs.E + gs.known_elem[kb]) * 3;
-                contract_add(out1, l, kv, gs.known_sign[kb], uk, ge, gu);
+    for (int s = s0 + (threadIdx.x >> 5); s < s1; s += kPairWarps) {
+        const int64_t p = ps.pair_off[d] + (int64_t)(s - b) * nd + (f - b);
+        const double src[3] = {g.node[3 * s], g.node[3 * s + 1], g.node[3 * s + 2]};
+        double ge = 0.0, gu = 0.0;
+        if (step0_sums(*rules, M, tb, pw, e, s == f, sb, src, pw.out)) {
+            QDual out0[9], out1[9];
+            const uint8_t fl = step0_pair<QDual>(pw.out, g, dr, f, out0, out1);
+            if (fl) {
+                const int64_t E3 = 3 * (int64_t)gs.E;
+                for (int n = 1 + lane; n <= gs.N; n += 32) {
+                    const double* l = gs.lam + n * E3 + 3 * (int64_t)s;
+                    const double* xn = gs.x + (int64_t)(n - 1) * E3;
+                    if (fl & 1) contract_add(out0, l, xn + 3 * gs.col_a0[f], -1.0, u0, ge, gu);
+                    if (fl & 2) contract_add(out1, l, xn + 3 * gs.col_a1[f], -1.0, true, ge, gu);
+                    if (fl & 4) {
+                        const int64_t kb = gs.col_k[f];
+                        const double* kv = gs.known + ((int64_t)n * gs.E + gs.known_elem[kb]) * 3;
+                        contract_add(out1, l, kv, gs.known_sign[kb], uk, ge, gu);
+                    }
+                }
             }
+            __syncwarp();
         }
-    }
-    ge = qwarp_sum(ge);
-    gu = qwarp_sum(gu);
-    if (lane == 0) {
-        part[2 * p] = ge;
-        part[2 * p + 1] = gu;
+        ge = qwarp_sum(ge);
+        gu = qwarp_sum(gu);
+        if (lane == 0) {
+            part[2 * p] = ge;
+            part[2 * p + 1] = gu;
+        }
     }
 }
 

@@ -73,8 +73,8 @@ __global__ void geometry_kernel(int E, const double* points, const int64_t* elem
                                 ElemGeom g);
 __global__ void singular_kernel(int E, const QuadRules* rules, const double* secpw_pos, const double* secpw_val,
                                 ElemGeom g);
-__global__ void step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr, double* blocks,
-                             uint8_t* flags);
+__global__ void step0_kernel(PairSpace ps, const QuadRules* rules, const DynaMat* mats, ElemGeom g, DofRefs dr,
+                             double* blocks, uint8_t* flags);
 __global__ void history_range_kernel(PairSpace ps, const DynaMat* mats, ElemGeom g, int maxn, uint32_t* range,
                                      int64_t* slots);
 __global__ void history_pairs_kernel(PairSpace ps, const QuadRules* rules, const DynaMat* mats, ElemGeom g, DofRefs dr,
@@ -99,8 +99,8 @@ __global__ void singular_grad_kernel(int E, const double* secpw_pos, const doubl
 __global__ void history_states_kernel(int N, int E, int nh, const int32_t* hist_owner, const int64_t* hist_block,
                                       const double* hu_sign, const double* ht_sign, const double* out_lu,
                                       const double* out_lt, double* xh);
-__global__ void grad_step0_kernel(PairSpace ps, const QuadRules* rules, ElemGeom g, DofRefs dr, const QDual* self_d,
-                                  GradState gs, double* part);
+__global__ void grad_step0_kernel(PairSpace ps, const QuadRules* rules, const DynaMatD* mats, ElemGeom g, DofRefs dr,
+                                  const QDual* self_d, GradState gs, double* part);
 __global__ void grad_history_kernel(PairSpace ps, const QuadRules* rules, const DynaMatD* mats, ElemGeom g, DofRefs dr,
                                     const uint32_t* range, const QDual* self_d, GradState gs, double* part);
 __global__ void to_float_kernel(const double* in, float* out, int64_t n);

@@ -1801,9 +1801,9 @@ tdbem_status tdbem_md_assemble(tdbem_handle* h, void* stream)
     CUDA_TRY(blocks.alloc(sizeof(double) * 18 * ps.n_pairs));
     CUDA_TRY(flags.alloc(ps.n_pairs));
     ElemGeom g = h->geom();
-    const int warps_per_cta = 4;
-    step0_kernel<<<ceil_div(ps.n_pairs, warps_per_cta), 32 * warps_per_cta, 0, s>>>(
-        ps, h->d_rules.as<QuadRules>(), g, dr, blocks.as<double>(), flags.as<uint8_t>());
+    CUDA_TRY(cudaFuncSetAttribute(step0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(false)));
+    step0_kernel<<<(unsigned)pair_ctas(ps, h->dom_count.data()), 256, pair_smem(false), s>>>(
+        ps, h->d_rules.as<QuadRules>(), h->d_mats.as<DynaMat>(), g, dr, blocks.as<double>(), flags.as<uint8_t>());
     CUDA_TRY(cudaGetLastError());
     {
         ScatterCols sa{{0, 1, 1}, {P.col_a0.as<int64_t>(), P.col_a1.as<int64_t>(), P.col_k.as<int64_t>()}};
@@ -3295,12 +3295,13 @@ tdbem_status material_gradient(tdbem_handle* h, cudaStream_t s, double* grad)
                                                                range.as<uint32_t>(), slots.as<int64_t>());
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaFuncSetAttribute(grad_history_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(true)));
+    CUDA_TRY(cudaFuncSetAttribute(grad_step0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(true)));
     std::vector<double> pv;
-    const int warps = 4;
     for (int pass = 0; pass < 2 && np > 0; ++pass) {
         if (pass == 0)
-            grad_step0_kernel<<<ceil_div(np, warps), 32 * warps, 0, s>>>(P.ps, h->d_rules.as<QuadRules>(), g, P.dr,
-                                                                         self_d.as<QDual>(), gs, part.as<double>());
+            grad_step0_kernel<<<(unsigned)pair_ctas(P.ps, h->dom_count.data()), 256, pair_smem(true), s>>>(
+                P.ps, h->d_rules.as<QuadRules>(), d_dm.as<DynaMatD>(), g, P.dr, self_d.as<QDual>(), gs,
+                part.as<double>());
         else
             grad_history_kernel<<<(unsigned)pair_ctas(P.ps, h->dom_count.data()), 256, pair_smem(true), s>>>(
                 P.ps, h->d_rules.as<QuadRules>(), d_dm.as<DynaMatD>(), g, P.dr, range.as<uint32_t>(), self_d.as<QDual>(),

@@ -78,7 +78,9 @@ __device__ __forceinline__ int front_step(double t, double dt)
     return n;
 }
 
-// Wave-front classification of q_need_cal with its distances taken once.
+// Wave-front classification of (field element, source point) for time index m: 0
+// skip, 1 patch-wise rule, 2 regular rule (NeedCal,
+// DBEM1/dsquareelement.cpp:1156-1201), with its distances taken once.
 struct PairClass {
     double a1, a2, b1, b2, dt;
     template <class MT>

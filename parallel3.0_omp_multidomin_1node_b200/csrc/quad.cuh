@@ -302,28 +302,6 @@ __device__ __forceinline__ void q_static_t(const MT& M, double* T, const double*
     T[8] = t9 + t10 * R[3] * R[3];
 }
 
-// Wave-front classification of (field element, source point) for time
-// index n: 0 skip, 1 patch-wise rule, 2 regular rule (NeedCal,
-// DBEM1/dsquareelement.cpp:1156-1201).
-template <class MT>
-__device__ __forceinline__ int q_need_cal(const MT& M, const double* center, double radius, int type, double n,
-                                          const double* o)
-{
-    const double nn = type == 2 ? n - 1 : n;
-    const double ndt = nn * M.Dt, np1dt = (nn + 1) * M.Dt;
-    const double r = q_dist(center, o);
-    const double Rmax = r + radius;
-    double Rmin = r - radius;
-    if (Rmin < 0.0) Rmin = 0.0;
-    const double a1 = Rmax / qv(M.C1), a2 = Rmax / qv(M.C2), b1 = Rmin / qv(M.C1), b2 = Rmin / qv(M.C2);
-    if (ndt >= a2 || np1dt <= b1) return 0;
-    if (ndt <= b1 && (np1dt >= a1 && np1dt <= b2)) return 2;
-    if (ndt <= b1 && np1dt >= a2) return 2;
-    if (ndt >= a1 && np1dt <= b2) return 2;
-    if ((ndt >= a1 && ndt <= b2) && np1dt >= a2) return 2;
-    return 1;
-}
-
 template <class MT>
 __device__ __forceinline__ bool q_pw_need_cal(const MT& M, double rpw, int type, double n, const double* pc,
                                               const double* o)
@@ -343,59 +321,6 @@ struct QElem {
 };
 
 // ---- warp-cooperative element integrals (result in out[9] on every lane) ----
-
-// regular 4x4 rule for U(n) (IntDynaUij, DBEM1/dsquareelement.cpp:1955-2009)
-template <class MT, class S = typename MT::Scalar>
-__device__ __forceinline__ void w_int_u_regular(const QuadRules& q, const MT& M, const QElem& e,
-                                                const double* src, double n, S* out)
-{
-    const int lane = threadIdx.x & 31;
-    S c[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    if (lane < 16) {
-        double pt[3];
-        S U[9];
-        QR r;
-        q_from_local(e.cc, q.rp[lane][0], q.rp[lane][1], pt);
-        q_get_r(src, pt, r);
-        if (q_dyna_u(M, U, n, r)) {
-            const double t = q.nrgv0[lane] * q_jacobi(e.cc, q.rp[lane][0], q.rp[lane][1]);
-            c[0] = U[0] * t; c[1] = U[1] * t; c[2] = U[2] * t; c[3] = U[4] * t; c[4] = U[5] * t; c[5] = U[8] * t;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) c[i] = qwarp_sum(c[i]);
-    out[0] = c[0]; out[1] = c[1]; out[2] = c[2]; out[3] = c[1]; out[4] = c[3]; out[5] = c[4];
-    out[6] = c[2]; out[7] = c[4]; out[8] = c[5];
-}
-
-// regular rule for T: T1(n) + T2(n) at every point, whatever the requested
-// type (IntDynaTij(typeT, ..., T_ID), DBEM1/dsquareelement.cpp:2233-2290)
-template <class MT, class S = typename MT::Scalar>
-__device__ __forceinline__ void w_int_t_regular(const QuadRules& q, const MT& M, const QElem& e,
-                                                const double* src, double n, S* out)
-{
-    const int lane = threadIdx.x & 31;
-    S c[9];
-#pragma unroll
-    for (int i = 0; i < 9; ++i) c[i] = 0.0;
-    if (lane < 16) {
-        double pt[3], nor[3], jac;
-        S T1[9], T2[9];
-        QR r;
-        q_from_local(e.cc, q.rp[lane][0], q.rp[lane][1], pt);
-        q_get_r(src, pt, r);
-        q_normal_jacobi(e.cc, q.rp[lane][0], q.rp[lane][1], nor, &jac);
-        int flag = q_dyna_t(M, 1, T1, n, r, nor);
-        flag += q_dyna_t(M, 2, T2, n, r, nor);
-        if (flag) {
-            const double t = q.nrgv0[lane] * jac;
-#pragma unroll
-            for (int i = 0; i < 9; ++i) c[i] = (T1[i] + T2[i]) * t;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 9; ++i) out[i] = qwarp_sum(c[i]);
-}
 
 // patch-wise 6x6 x 3x3 rule for U(n) (IntDynaUijPW, DBEM1/dsquareelementdyna.cpp:794-848)
 template <class MT, class S = typename MT::Scalar>
