@@ -216,8 +216,8 @@ def measured_hbm_peak():
 def profile_traffic_ratio():
     """DRAM bytes per algorithmic byte of the 32-load two-step history pass,
     from the committed ncu summary (line 'dram_to_algorithmic=' in
-    profiles/bulk_steps_kernel_bar8_32loads_mixed.txt); None when absent."""
-    p = os.path.join(REPO, "profiles", "bulk_steps_kernel_bar8_32loads_mixed.txt")
+    profiles/bulk_groups_kernel_bar8_32loads_mixed.txt); None when absent."""
+    p = os.path.join(REPO, "profiles", "bulk_groups_kernel_bar8_32loads_mixed.txt")
     try:
         for ln in open(p):
             if ln.startswith("dram_to_algorithmic="):
@@ -430,8 +430,10 @@ def ours_arm(args):
         "gmres_cluster_ms_per_march": hd["ms_gmres"] / args.steps,
         "assembly_s": hd["asm"],
         "roofline": {"bound": "hbm",
-                     "kernel": ("bulk_steps_kernel (history steps k >= %d of %d time steps, %d loads)"
-                                % (2 * steps_per_pass + 1, steps_per_pass, R) if steps_per_pass > 1
+                     "kernel": ("%s (history steps k >= %d of %d time steps, %d loads)"
+                                % ("bulk_groups_kernel" if R >= 8 else "bulk_steps_kernel" if R > 1
+                                   else "bulk_rows_kernel", 2 * steps_per_pass + 1, steps_per_pass, R)
+                                if steps_per_pass > 1
                                 else "rhs_kernel (history steps k >= 3 of one time step, %d loads)" % R),
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind,
@@ -441,7 +443,7 @@ def ours_arm(args):
                      "ms_per_launch": serial["ms"] / launches_hist,
                      "launches_per_march": launches_hist,
                      "timing": "one extra march with the history passes run after each step's GMRES instead of "
-                               "beside it; CUDA events around those launches only",
+                               "beside it; device clock from those launches' first to last CTA",
                      "l2_state": {"achieved": l2_achieved, "peak": l2_peak, "unit": "GB/s",
                                   "frac": l2_achieved / l2_peak,
                                   "peak_kind": "ncu sustained peak of L2 tex-sector throughput (hardware counter "

@@ -1,5 +1,5 @@
-"""History matrices assembled over all steps of a pair at once, against the C
-oracle's step-by-step assembly (B200): domains of one element a face, of 96
+"""History and step-0 matrices assembled over all steps of a pair at once, against
+the C oracle's step-by-step assembly (B200): domains of one element a face, of 96
 elements (more sources than a CTA's 64, not a multiple), several materials, and
 time steps short and long against the element size (waves that stay many steps in
 an element, or cross it within one), with the workspace limit cutting the rows
@@ -69,6 +69,23 @@ def test_history_matrices_equal_the_oracle(domains, n, beta):
             zero = np.zeros(9)
             for key in a.keys() | b.keys():
                 assert np.max(np.abs(a.get(key, zero) - b.get(key, zero))) <= mark, (name, k, key)
+
+
+@pytest.mark.parametrize("domains,n,beta", SHAPES)
+def test_step0_matrices_equal_the_oracle(domains, n, beta):
+    from tdbem.api import MultiDomainSolver
+    from oracle_lib import Oracle
+    c = _case(domains, n, beta, 4)
+    o = Oracle(c)
+    o.assemble()
+    s = MultiDomainSolver(c)
+    s.assemble()
+    for name in ("A", "KnownM"):
+        a, b = _blocks(s.export_matrix(name)), _blocks(o.matrix(name))
+        mark = max(1e-12 * max(np.max(np.abs(v)) for v in b.values()), 2e-14)
+        zero = np.zeros(9)
+        for key in a.keys() | b.keys():
+            assert np.max(np.abs(a.get(key, zero) - b.get(key, zero))) <= mark, (name, key)
 
 
 @pytest.mark.parametrize("domains,n,beta", SHAPES)
