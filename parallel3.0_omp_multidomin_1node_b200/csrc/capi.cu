@@ -21,6 +21,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 #include <limits>
 
@@ -1638,13 +1639,19 @@ struct MarchRun {
         return TDBEM_OK;
     }
 
+    // The stream of the history passes, and how many steps ahead of step k the
+    // prescribed values (KnownM . known) reach that the pass launched at k reads:
+    // T-step passes cover the steps up to k + 2T - 1, the one-step pass k + 1.
+    cudaStream_t pass_stream() const { return serial_history ? s : h->side; }
+    int pass_lead() const { return !overlap ? 0 : h->run_k >= 5 ? h->run_k - 2 : 1; }
+
     tdbem_status step(int k)
     {
         CUDA_TRY(cudaSetDevice(h->device));
         const int T = h->run_k >= 5 ? (h->run_k - 1) / 2 : 2;  // steps per history pass
         StepEvents se{E2(k, 0), E2(k, 1), k == 1 ? ev[1] : E2(k - 1, 0),
                       k > T ? E2(R == 1 ? k - 1 : k - T, 1) : nullptr};
-        CUDA_TRY(march_step(d, k, s, serial_history ? s : h->side, se, overlap));
+        CUDA_TRY(march_step(d, k, s, pass_stream(), se, overlap));
         return TDBEM_OK;
     }
 
@@ -2174,7 +2181,8 @@ tdbem_status tdbem_md_march(tdbem_handle* h, const double* known_lu, double* out
     // Pinned host buffers: the copies run beside the march by chunks of
     // steps.  Chunk 0's inputs go ahead of the set-up on the caller's stream,
     // the later chunks' on the input stream, each waited for by the first
-    // step that reads it; each chunk's boundary values go back on the output
+    // step that reads it and, on their own stream, by the first history pass
+    // that does; each chunk's boundary values go back on the output
     // stream once its last step's GMRES (which writes them) is done.
     const int chunks = std::max(1, std::min(N + 1, 32));
     std::vector<int> bound((size_t)chunks + 1);
@@ -2206,7 +2214,15 @@ tdbem_status tdbem_md_march(tdbem_handle* h, const double* known_lu, double* out
     CUDA_TRY(copy_chunk(0, true, s));
     CUDA_TRY(cudaEventRecord(ev[2 * chunks], s));  // the input stream follows the caller's stream
     CUDA_TRY(cudaStreamWaitEvent(h->cin, ev[2 * chunks], 0));
+    // TDBEM_INPUT_DELAY: microseconds every later chunk's copy is held back, for
+    // tests of what waits for it
+    const char* held = std::getenv("TDBEM_INPUT_DELAY");
+    const intptr_t delay_us = held ? std::atoi(held) : 0;
     for (int c = 1; c < chunks; ++c) {
+        if (delay_us > 0)
+            CUDA_TRY(cudaLaunchHostFunc(
+                h->cin, [](void* us) { std::this_thread::sleep_for(std::chrono::microseconds((intptr_t)us)); },
+                reinterpret_cast<void*>(delay_us)));
         CUDA_TRY(copy_chunk(c, true, h->cin));
         CUDA_TRY(cudaEventRecord(in_done[c], h->cin));
     }
@@ -2216,8 +2232,11 @@ tdbem_status tdbem_md_march(tdbem_handle* h, const double* known_lu, double* out
         cudaStreamSynchronize(h->cin);
         return st;
     }
-    int c = 0;
+    int c = 0, ahead = 0;
     for (int step = 1; step <= N && st == TDBEM_OK; ++step) {
+        while (ahead + 1 < chunks && step + run.pass_lead() >= bound[ahead + 1] && st == TDBEM_OK)
+            if (cudaStreamWaitEvent(run.pass_stream(), in_done[++ahead], 0) != cudaSuccess)
+                st = fail(TDBEM_CUDA_ERROR, "input wait");
         while (c + 1 < chunks && step >= bound[c + 1]) {
             // chunk c's boundary values are complete: steps < bound[c + 1] are done
             if (cudaEventRecord(out_ready[c], run.s) != cudaSuccess ||
