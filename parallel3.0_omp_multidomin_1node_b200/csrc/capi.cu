@@ -354,7 +354,9 @@ struct GmresTiles {
     cudaError_t build(const std::vector<int32_t>& rows, int64_t leaf_values, const std::vector<int32_t>& rp,
                       const std::vector<int32_t>& mcol, const double* d_val9, bool mixed, cudaStream_t s);
     // for Rg load cases per cluster.  TDBEM_GMRES_DSM=0 forces the kernel's
-    // global-memory form, for tuning.
+    // global-memory form, for tuning; TDBEM_GMRES_WAIT is another limit of the
+    // cluster's waits, the exponent of a power of two in cycles, for tests (zero or
+    // less: the last CTA gives up its first wait, and the exponent is the magnitude).
     void fill(MarchData& d, int Rg, bool mixed) const
     {
         d.cta_row = cta_row.as<int32_t>();
@@ -371,6 +373,8 @@ struct GmresTiles {
         const int cap = gmres_row_capacity(own_rows);
         const char* off = std::getenv("TDBEM_GMRES_DSM");
         const bool fits = gmres_dsm_fits(cap, halo_rows, Rg, mixed) && !(off && std::atoi(off) == 0);
+        const char* wait = std::getenv("TDBEM_GMRES_WAIT");
+        d.wait_log2 = wait ? std::max(-62, std::min(62, std::atoi(wait))) : kGmresWaitLog2;
         d.own_rows = own_rows;
         d.leaf_max = leaf_max;
         d.dsm_rows = fits ? cap : 0;

@@ -41,9 +41,9 @@ namespace {
 constexpr int kGmresThreads = 512;  // at most (gmres_threads)
 constexpr int kGmresWarps = kGmresThreads / 32;
 static_assert(kGmresWarps == 16 && kGmresClusterMax == 16, "reductions use 16 lanes per value");
-// cycles (about two seconds) after which a wait gives up and the step fails; a
-// wait takes microseconds
-constexpr long long kWaitCycles = 4000000000ll;
+// cycles a CTA whose wait ran out stays after its peers have stopped, for their
+// pushes still on the way to it (they take some 600)
+constexpr long long kDrainCycles = 200000;
 
 // basis vectors per cluster reduction, and Krylov columns whose small arrays
 // (rotations, Hessenberg columns) are kept in shared memory: as many as the
@@ -72,7 +72,7 @@ struct GShared {
     double h1[R], phibar[R], n2b[R];
     int run[R], flag[R], inner[R], cycles[R], stag[R], check[R], jend[R];
     int any_run, any_cand, any_check;
-    unsigned long long red_bar[2], vec_bar;         // mbarriers: partial sums of the two slots, vector halos
+    unsigned long long red_bar[2], vec_bar;         // mbarriers: partial sums of the two slots, vectors
     // the cluster and the vectors of this CTA
     int rank, C, nown, vcap, vs_off, vs_len, gl;    // basis vectors k < vcap at dsm + vs_off, vs_len apart
     int rl_off, pc_off;                             // cached leaf inverses: row table, values (doubles into dsm)
@@ -114,34 +114,53 @@ __device__ __forceinline__ void push16(uint32_t addr, unsigned long long v, unsi
                  "l"(w), "r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ void bar_init(unsigned long long* bar)
+__device__ __forceinline__ void bar_init(unsigned long long* bar, uint32_t arrivals)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(bar)) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(bar)), "r"(arrivals) : "memory");
 }
 // one thread per CTA and phase: the phase ends when `bytes` have arrived
 __device__ __forceinline__ void bar_expect(unsigned long long* bar, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(bar)), "r"(bytes) : "memory");
 }
-// The bytes counted lie in this CTA's shared memory, so the wait acquires at CTA
-// scope: a cluster-scope acquire also drops the SM's L1, and reading a 21-column
-// leaf inverse after it took 3,700 cycles instead of 860 (measured).
-// Waits for a phase, at most kWaitCycles; then `dead` is set and this and later
-// waits pass, so that the kernel ends and the step fails.
-__device__ __forceinline__ void bar_wait(unsigned long long* bar, uint32_t parity, bool& dead)
+// State of a thread's exchanges: bit 0 slot of the next reduction, bits 1, 2 parity
+// of the slots' current phases, bit 3 that of vec_bar, all the same in a CTA; bit 4
+// a wait of this thread ran out, bit 5 its waits do so at once (a test's); from bit
+// 8 on the limit of a wait, as a power of two in cycles.
+constexpr uint32_t kDead = 16, kGiveUp = 32;
+constexpr int kLimitShift = 8;
+
+// Waits for a phase, at most about its limit.  When it runs out, this wait and the
+// thread's later ones pass, and the thread arms no barrier and pushes nothing any
+// more: a phase that did not end is never armed again, the waits of the CTA's other
+// threads and of the peers that miss its share run out in turn, and every CTA comes
+// to the barrier at the solve's end, where the step fails.
+// kCluster: what other CTAs wrote to global memory is read next.  Otherwise the
+// bytes counted lie in this CTA's shared memory and the wait acquires at CTA scope:
+// a cluster-scope acquire also drops the SM's L1, and reading a 21-column leaf
+// inverse after it took 3,700 cycles instead of 860 (measured).
+template <bool kCluster = false>
+__device__ __forceinline__ uint32_t bar_wait(unsigned long long* bar, uint32_t parity, uint32_t st)
 {
     const uint32_t a = shared_addr(bar);
     long long start = 0;
+    bool dead = (st & (kDead | kGiveUp)) != 0;
     while (!dead) {
         uint32_t done;
-        asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2; "
-                     "selp.u32 %0, 1, 0, p;}"
-                     : "=r"(done) : "r"(a), "r"(parity) : "memory");
-        if (done) return;
+        if constexpr (kCluster)
+            asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; "
+                         "selp.u32 %0, 1, 0, p;}"
+                         : "=r"(done) : "r"(a), "r"(parity) : "memory");
+        else
+            asm volatile("{.reg .pred p; mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2; "
+                         "selp.u32 %0, 1, 0, p;}"
+                         : "=r"(done) : "r"(a), "r"(parity) : "memory");
+        if (done) return 0;
         const long long now = clock64();
         if (start == 0) start = now;
-        else if (now - start > kWaitCycles) dead = true;
+        else if ((now - start) >> (st >> kLimitShift) != 0) dead = true;
     }
+    return kDead;
 }
 
 // the CPT cases of the three components of one row of a shared-memory vector
@@ -217,11 +236,6 @@ __device__ __forceinline__ GShared<R>& gshared()
     return *reinterpret_cast<GShared<R>*>(dsm);
 }
 
-// State of a CTA's exchanges, the same in all its threads: bit 0 slot of the
-// next reduction, bits 1, 2 parity of the slots' current phases, bit 3 that of
-// the vector halos, bit 4 a wait ran out.
-constexpr uint32_t kDead = 16;
-
 // Sums of m values per case over the cluster, in dst[q * R + case] (shared
 // memory) of every CTA.  Each CTA pushes its partial sums into every peer's
 // shared memory, all reads are local and every CTA adds the same partials in
@@ -234,19 +248,19 @@ __device__ __noinline__ uint32_t red_finish(int m, int dst, uint32_t st)
     GShared<R>& s = gshared<R>();
     const int l = threadIdx.x & 15, g = threadIdx.x >> 4, per = blockDim.x >> 4, nw = blockDim.x >> 5;
     const int items = m * R, slot = st & 1u, C = s.C;
+    const bool live = !(st & kDead);
     unsigned long long* bar = &s.red_bar[slot];
     __syncthreads();
-    if (threadIdx.x == 0) bar_expect(bar, (uint32_t)(sizeof(double) * items * C));
+    if (threadIdx.x == 0 && live) bar_expect(bar, (uint32_t)(sizeof(double) * items * C));
     const uint32_t peer = (uint32_t)(l < C ? l : s.rank);
     const uint32_t to = peer_addr(shared_addr(&s.part[slot][s.rank][0]), peer), to_bar = peer_addr(shared_addr(bar), peer);
 #pragma unroll 1
     for (int i0 = 0; i0 < items; i0 += per) {
         const int i = i0 + g;
         const double v = sum16(i < items && l < nw ? s.wred[l][i] : 0.0);
-        if (i < items && l < C) push8(to + 8 * i, (unsigned long long)__double_as_longlong(v), to_bar);
+        if (i < items && l < C && live) push8(to + 8 * i, (unsigned long long)__double_as_longlong(v), to_bar);
     }
-    bool dead = (st & kDead) != 0;
-    bar_wait(bar, (st >> (1 + slot)) & 1u, dead);
+    st |= bar_wait(bar, (st >> (1 + slot)) & 1u, st);
 #pragma unroll 1
     for (int i0 = 0; i0 < items; i0 += per) {
         const int i = i0 + g;
@@ -254,7 +268,7 @@ __device__ __noinline__ uint32_t red_finish(int m, int dst, uint32_t st)
         if (i < items && l == 0) dsm[dst + i] = v;
     }
     __syncthreads();
-    return (st ^ 1u ^ (2u << slot)) | (dead ? kDead : 0u);
+    return st ^ 1u ^ (2u << slot);
 }
 
 // Dot products of the work vector u (shared-memory offset, or a global pointer)
@@ -270,10 +284,11 @@ __device__ __noinline__ uint32_t gram_dots(int q0, int nq, bool norm, const doub
     GShared<R>& s = gshared<R>();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, C = s.C, slot = st & 1u;
     const int m = nq + norm, parts = R <= 4 || m >= nw ? 1 : nw / m, nown = s.nown;
+    const int to_all = st & kDead ? 0 : C;  // peers to push to
     unsigned long long* bar = &s.red_bar[slot];
     const uint32_t to = shared_addr(&s.part[slot][s.rank][0]), to_bar = shared_addr(bar);
     __syncthreads();
-    if (threadIdx.x == 0) bar_expect(bar, (uint32_t)(sizeof(double) * m * R * C));
+    if (threadIdx.x == 0 && to_all) bar_expect(bar, (uint32_t)(sizeof(double) * m * R * C));
 #pragma unroll 1
     for (int i = w; i < m * parts; i += nw) {
         const int k = i % m, part = i / m, kv = q0 + k, step = 32 * parts;
@@ -300,7 +315,7 @@ __device__ __noinline__ uint32_t gram_dots(int q0, int nq, bool norm, const doub
 #pragma unroll
             for (int j = 0; j < (R + 1) / 2; ++j) {
                 const int peer = lane / R + j * (32 / R);
-                if (peer < C)
+                if (peer < to_all)
                     push8(peer_addr(to + 8 * (k * R + lane % R), (uint32_t)peer),
                           (unsigned long long)__double_as_longlong(a0), peer_addr(to_bar, (uint32_t)peer));
             }
@@ -315,13 +330,12 @@ __device__ __noinline__ uint32_t gram_dots(int q0, int nq, bool norm, const doub
         for (int i0 = 0; i0 < items; i0 += per) {
             const int i = i0 + g;
             const double v = sum16(i < items && l < parts ? s.wred[l][i] : 0.0);
-            if (i < items && l < C)
+            if (i < items && l < to_all)
                 push8(peer_addr(to + 8 * i, (uint32_t)l), (unsigned long long)__double_as_longlong(v),
                       peer_addr(to_bar, (uint32_t)l));
         }
     }
-    bool dead = (st & kDead) != 0;
-    bar_wait(bar, (st >> (1 + slot)) & 1u, dead);
+    st |= bar_wait(bar, (st >> (1 + slot)) & 1u, st);
 #pragma unroll 1
     for (int i0 = 0; i0 < items; i0 += per) {
         const int i = i0 + g;
@@ -329,7 +343,7 @@ __device__ __noinline__ uint32_t gram_dots(int q0, int nq, bool norm, const doub
         if (i < items && l == 0) dsm[dst + i] = v;
     }
     __syncthreads();
-    return (st ^ 1u ^ (2u << slot)) | (dead ? kDead : 0u);
+    return st ^ 1u ^ (2u << slot);
 }
 
 // Publishes the owned rows of the product's source vector v (shared memory; row
@@ -343,8 +357,9 @@ __device__ __noinline__ uint32_t publish(const int2* __restrict__ send, int n_se
     constexpr int kChunks = kRowBytes / kChunk;
     GShared<R>& s = gshared<R>();
     const char* v = reinterpret_cast<const char*>(dsm + v_off);
+    if (st & kDead) n_send = 0;
     __syncthreads();
-    if (threadIdx.x == 0) bar_expect(&s.vec_bar, (uint32_t)(halo * kRowBytes));
+    if (threadIdx.x == 0 && !(st & kDead)) bar_expect(&s.vec_bar, (uint32_t)(halo * kRowBytes));
     const uint32_t base = shared_addr(v), bar = shared_addr(&s.vec_bar);
 #pragma unroll 1
     for (int i = threadIdx.x; i < n_send * kChunks; i += blockDim.x) {
@@ -359,9 +374,24 @@ __device__ __noinline__ uint32_t publish(const int2* __restrict__ send, int n_se
             push8(to, *reinterpret_cast<const unsigned long long*>(src), peer_addr(bar, peer));
         }
     }
-    bool dead = (st & kDead) != 0;
-    bar_wait(&s.vec_bar, (st >> 3) & 1u, dead);
-    return (st ^ 8u) | (dead ? kDead : 0u);
+    return (st | bar_wait(&s.vec_bar, (st >> 3) & 1u, st)) ^ 8u;
+}
+
+// The global-memory form's counterpart: this CTA's rows of a vector in global
+// memory are complete, and every other CTA's are after it.  An arrival at each
+// peer's vec_bar, with the limit of the other waits: the cluster barrier has none,
+// and a CTA that gave up would have to keep count of its peers'.  A peer arrives
+// for the next vector only after a reduction between, so after this CTA's wait.
+template <int R>
+__device__ __noinline__ uint32_t vectors_complete(uint32_t st)
+{
+    GShared<R>& s = gshared<R>();
+    __syncthreads();
+    if ((int)threadIdx.x < s.C && !(st & kDead))
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(
+                         peer_addr(shared_addr(&s.vec_bar), threadIdx.x))
+                     : "memory");
+    return (st | bar_wait<true>(&s.vec_bar, (st >> 3) & 1u, st)) ^ 8u;
 }
 
 // ---- products ------------------------------------------------------------
@@ -798,7 +828,10 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
         rank = (int)cgc.block_rank();
         C = (int)cgc.num_blocks();
     }
-    uint32_t st = 0;  // state of the exchanges
+    // state of the exchanges; a limit of zero or less makes the last thread of the
+    // last CTA give up its first wait
+    uint32_t st = (uint32_t)abs(d.wait_log2) << kLimitShift;
+    if (d.wait_log2 <= 0 && rank == C - 1 && threadIdx.x == blockDim.x - 1) st |= kGiveUp;
     const int NT = (int)blockDim.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int RT = d.R, roff = grp * R;  // total cases, first case of this group
     const int E = d.E, rs = d.restart;
@@ -826,9 +859,9 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
     double* const vg = d.V + (int64_t)grp * (rs + 1) * n + ob;
     const int vcap = kLocal ? d.vcap : 0, vs_len = 3 * d.dsm_rows * R;
     if (threadIdx.x == 0) {
-        bar_init(&s.red_bar[0]);
-        bar_init(&s.red_bar[1]);
-        bar_init(&s.vec_bar);
+        bar_init(&s.red_bar[0], 1);
+        bar_init(&s.red_bar[1], 1);
+        bar_init(&s.vec_bar, kLocal ? 1 : C);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s.rank = rank;
         s.C = C;
@@ -869,7 +902,7 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
             st = publish<R, double>(d.g_send + e0, n_send, halo, pv_off, st);
             spmm_tiles<R, true, double, double, double>(slices, srows, d.g_col, d.g_val, nullptr, pv_off, rows, y);
         } else {
-            cluster_barrier();
+            st = vectors_complete<R>(st);
             spmm_tiles<R, false, double, double, double>(slices, srows, d.g_colg, d.g_val, pv - ob, 0, rows, y);
         }
     };
@@ -1031,7 +1064,7 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
                 else
                     spmm_tiles<R, true, double, double, double>(slices, srows, d.g_col, d.g_val, nullptr, pv_off, rows, aw);
             } else {
-                cluster_barrier();  // V_j complete in every CTA
+                st = vectors_complete<R>(st);
                 if constexpr (kMixed)
                     spmm_tiles<R, false, float, double, double>(slices, srows, d.g_colg, d.g_val32, V(j) - ob, 0, rows, aw);
                 else
@@ -1258,8 +1291,8 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
             __syncthreads();
         }
     }
-    const bool dead = (st & kDead) != 0;
-    int failed = __syncthreads_or(dead) ? 1 : 0;  // the flags are the same in every CTA
+    const bool dead = __syncthreads_or(st & kDead) != 0;  // a wait ran out in this CTA: the step has failed
+    int failed = dead;  // the flags are the same in every CTA otherwise
     for (int r = 0; r < R; ++r) failed |= s.flag[r] != 0;
     int* const fl = d.step_flags + ((int64_t)(step - 1) * RT + roff + tr) * 3;
     if (threadIdx.x < R && rank == 0 && !aborted) {
@@ -1269,9 +1302,14 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
         if (s.flag[tr] != 0) atomicExch(d.status, 1);
     }
     cluster_barrier();  // x complete; no peer is accessed below
-    if (threadIdx.x < R && dead) {  // a wait ran out in this CTA: the step has failed
-        fl[0] = 1;
-        atomicExch(d.status, 1);
+    if (dead) {
+        if (threadIdx.x < R) {
+            fl[0] = 1;
+            atomicExch(d.status, 1);
+        }
+        // all peers have stopped; what they had pushed may still be on its way here
+        const long long t0 = clock64();
+        while (clock64() - t0 < kDrainCycles) {}
     }
     if (failed || aborted || d.solve_only) return;
     write_back<R>(d, step, roff, d.x + (int64_t)grp * n, rank * NT + (int)threadIdx.x, C * NT);

@@ -149,6 +149,7 @@ struct MarchData {
     int cluster;             // CTAs in the GMRES cluster
     int rhs_cpt;             // history pass: load cases per thread (0 = default: min(R, 4))
     int64_t givens_stride;   // doubles per (CTA, case) in givens
+    int wait_log2;           // limit of the GMRES clusters' waits for one another, 2^wait_log2 cycles
     int after_head;          // 1: the GMRES launch follows the step's head pass in its stream and may
                              // start beside it (its caches of leaf inverses fill meanwhile)
     int solve_only;          // 1: GMRES alone, no write-back, history update or audit (bare solve)
@@ -164,6 +165,9 @@ constexpr int64_t gmres_givens_doubles(int restart)
     return (int64_t)kGivensArrays * (restart + 2) + (int64_t)(restart + 1) * (restart + 2) / 2;
 }
 constexpr int kGmresClusterMax = 16;
+// 2^32 cycles (about two seconds) after which a wait of a GMRES cluster gives up and
+// the step fails; a wait takes microseconds.
+constexpr int kGmresWaitLog2 = 32;
 
 // A' in the tile form of MarchData::g_*, built on the host as block indices and
 // gathered on the device (gather_tiles): src[tile][32] is the block of the
