@@ -739,6 +739,7 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
     double* Wa = d.wring + ((step - 1) % d.SW) * per_slot;
     double* Wb = d.wring + (step % d.SW) * per_slot;
     double worst[2] = {0.0, 0.0};  // displacement jump, traction balance
+    double zero = 0.0;             // not any more once a combined vector is not finite
 #pragma unroll 1
     for (int t = gtid; t < E * R; t += gstride) {
         const int i = t / R, r = t % R, rg = roff + r;
@@ -768,9 +769,11 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
                 const double xs = (c < 3 ? su : st) * g[c];
                 const int64_t p = o + (c < 3 ? 0 : per_type) + (c % 3) * RT;
                 const double xm1 = X1[p], xm2 = X2[p];
+                const double wa = (xs + 2.0 * xm1) + xm2, wb = 2.0 * xs + xm1;
                 X[p] = xs;
-                Wa[p] = (xs + 2.0 * xm1) + xm2;
-                Wb[p] = 2.0 * xs + xm1;
+                Wa[p] = wa;
+                Wb[p] = wb;
+                zero += 0.0 * wa + 0.0 * wb;
             }
         }
         if (e >= 0) {
@@ -782,6 +785,7 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
             }
         }
     }
+    if (zero != 0.0) d.status[1] = 1;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
 #pragma unroll

@@ -668,6 +668,42 @@ struct GroupPass {
     static constexpr size_t kBytes = kRing > kRed ? kRing : kRed;
 };
 
+// One row's sum of one step by a warp, from the step-major matrices: only the
+// products of stored blocks.  For histories with vectors that are not finite, which
+// the group layout's zeros must not meet.
+template <int R, class V>
+__device__ __noinline__ void group_row_plain(const MarchData& d, int p, int step, int lane)
+{
+    constexpr int kLists = 32 / R;
+    const int row = d.row_of[p], r = lane % R, K = d.K, SW = d.SW;
+    const int64_t* kp = d.h_kptr + (int64_t)row * (K + 1);
+    const int64_t slot_len = 2LL * d.nh * 3 * R, nnz = d.h_nnz;
+    double acc[3];
+    known_share<R>(d, row, step, 0, 1, lane, acc);
+    const int64_t end = kp[step < K ? step : K];
+#pragma unroll 1
+    for (int64_t i = kp[d.kr - 1] + lane / R; i < end; i += kLists) {
+        const uint32_t cp = d.h_col[i];
+        const double* x = d.wring + ((step - (int)(cp >> 21)) % SW) * slot_len +
+                          ((int64_t)((cp >> 20) & 1u) * d.nh + (cp & 0xFFFFFu)) * 3 * R + r;
+        const V* v;
+        if constexpr (sizeof(V) == 4) v = d.h_val32 + i;
+        else v = d.h_val + i;
+        const double x0 = x[0], x1 = x[R], x2 = x[2 * R];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            acc[c] += (double)v[3 * c * nnz] * x0 + (double)v[(3 * c + 1) * nnz] * x1 + (double)v[(3 * c + 2) * nnz] * x2;
+    }
+#pragma unroll
+    for (int o = 16; o >= R; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (lane < R)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            d.bulk[(int64_t)(step & 7) * 3 * d.E * R + (int64_t)(3 * p + c) * R + lane] = acc[c];
+}
+
 template <int R, int T, class V>
 __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kernel(const __grid_constant__ MarchData d,
                                                                                    int t0, int split)
@@ -677,10 +713,11 @@ __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kern
     const int group = (int)blockIdx.x / split, rank = (int)blockIdx.x % split;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     stamp_start(d, t0, 3);
-    // runs beside GMRES launches that may set the status word: the cluster
-    // takes rank 0's reading
+    // runs beside GMRES launches that may set the status words: the cluster
+    // takes rank 0's reading.  A word that is set meanwhile for vectors that are
+    // not finite is set for later ones than this pass reads.
     __shared__ int stop, stop_all;
-    if (threadIdx.x == 0) stop = *(volatile int*)d.status;
+    if (threadIdx.x == 0) stop = ((volatile int*)d.status)[0] ? 1 : ((volatile int*)d.status)[1] ? 2 : 0;
     unsigned char* const ring = reinterpret_cast<unsigned char*>(dsm) + w * P::kStages * P::kStage;
     for (int i = lane; i < P::kStages * P::kStage / 8; i += 32) reinterpret_cast<double*>(ring)[i] = 0.0;
     __syncthreads();
@@ -688,8 +725,16 @@ __global__ void __launch_bounds__(GroupPass<R, T, V>::kThreads) bulk_groups_kern
         cluster_barrier();
         if (threadIdx.x == 0) stop_all = *cg::this_cluster().map_shared_rank(&stop, 0);
         cluster_barrier();
-        if (stop_all) return;
-    } else if (stop) {
+    } else {
+        if (threadIdx.x == 0) stop_all = stop;
+        __syncthreads();
+    }
+    if (stop_all) {
+        if (stop_all == 2)
+            for (int i = rank * NW + w; i < 8 * T; i += NW * split) {
+                const int p = __ldg(d.hg_rows + (int64_t)group * 8 + i % 8), step = t0 + i / 8;
+                if (p >= 0 && step <= d.nstep) group_row_plain<R, V>(d, p, step, lane);
+            }
         return;
     }
     const int SW = d.SW, klast = t0 + T - 1 < d.K ? t0 + T - 1 : d.K;  // last step of the last sum
