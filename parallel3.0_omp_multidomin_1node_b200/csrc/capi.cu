@@ -945,8 +945,8 @@ tdbem_status build_runs(tdbem_handle* h, cudaStream_t s)
             h->run_k = hg.kr;
             return TDBEM_OK;
         }
-        // out of device memory part way, or too little in common between
-        // neighbouring rows: the run layout
+        // out of device memory part way, too little in common between neighbouring
+        // rows, or values that are not finite: the run layout
         for (DevBuf* b : {&h->d_hg_ptr, &h->d_hg_meta, &h->d_hg_off, &h->d_hg_val}) b->release();
         if (e != cudaErrorMemoryAllocation) CUDA_TRY(e);
         cudaGetLastError();
@@ -1293,7 +1293,7 @@ tdbem_status gmres_layout(tdbem_handle* h, int G, int C, cudaStream_t s)
 }
 
 // Packed blocks of the head pass of one load case (MarchData hd_*); where they do
-// not fit, the head reads the step-major matrices.
+// not fit or are not all finite, the head reads the step-major matrices.
 tdbem_status build_head(tdbem_handle* h, cudaStream_t s)
 {
     h->d_hd_ptr.release();
@@ -1310,7 +1310,9 @@ tdbem_status build_head(tdbem_handle* h, cudaStream_t s)
         if (tiles > INT32_MAX) return TDBEM_OK;
         ptr[p + 1] = (int32_t)tiles;
     }
-    cudaError_t e = h->d_hd_tile.alloc(head_tile_bytes(mixed) * std::max<int64_t>(tiles, 1));
+    // a word behind the tiles tells whether a value is not finite
+    const size_t bytes = head_tile_bytes(mixed) * std::max<int64_t>(tiles, 1);
+    cudaError_t e = h->d_hd_tile.alloc(bytes + sizeof(int));
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         h->d_hd_tile.release();
@@ -1318,10 +1320,18 @@ tdbem_status build_head(tdbem_handle* h, cudaStream_t s)
     }
     CUDA_TRY(e);
     CUDA_TRY(up(h->d_hd_ptr, ptr, s));
+    int* d_infinite = reinterpret_cast<int*>(h->d_hd_tile.as<unsigned char>() + bytes);
+    int infinite = 0;
+    CUDA_TRY(cudaMemsetAsync(d_infinite, 0, sizeof(int), s));
     CUDA_TRY(pack_head((int)E, h->K, head_k, h->d_row_of.as<int32_t>(), h->d_h_kptr.as<int64_t>(),
                        h->d_h_col.as<uint32_t>(), mixed ? h->d_h_val32.p : h->d_h_val.p, mixed, h->h_nnz,
-                       h->d_hd_ptr.as<int32_t>(), h->d_hd_tile.as<unsigned char>(), s));
+                       h->d_hd_ptr.as<int32_t>(), h->d_hd_tile.as<unsigned char>(), d_infinite, s));
+    CUDA_TRY(cudaMemcpyAsync(&infinite, d_infinite, sizeof(int), cudaMemcpyDeviceToHost, s));
     CUDA_TRY(cudaStreamSynchronize(s));
+    if (infinite) {
+        h->d_hd_ptr.release();
+        h->d_hd_tile.release();
+    }
     return TDBEM_OK;
 }
 

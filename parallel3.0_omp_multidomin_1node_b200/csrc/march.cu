@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kRhsThreads, 3) head_rows_kernel(MarchData d, 
 // Packs the blocks k <= head_k of each perm row into tiles of 32, zero-padded.
 template <class V>
 __global__ void pack_head_kernel(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
-                                 const V* val, int64_t nnz, const int32_t* ptr, unsigned char* tiles)
+                                 const V* val, int64_t nnz, const int32_t* ptr, unsigned char* tiles, int* infinite)
 {
     const int p = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (p >= E) return;
@@ -364,7 +364,11 @@ __global__ void pack_head_kernel(int E, int K, int head_k, const int32_t* row_of
         unsigned char* tile = tiles + t * head_tile_bytes(sizeof(V) == 4);
         reinterpret_cast<uint32_t*>(tile)[lane] = i < e ? col[i] : 0u;
         V* v = reinterpret_cast<V*>(tile + 128) + lane;
-        for (int c = 0; c < 9; ++c) v[32 * c] = i < e ? val[c * nnz + i] : V(0);
+        for (int c = 0; c < 9; ++c) {
+            const V x = i < e ? val[c * nnz + i] : V(0);
+            v[32 * c] = x;
+            if (!isfinite(x)) *infinite = 1;
+        }
     }
 }
 
@@ -1457,14 +1461,15 @@ __global__ void gather_tiles_kernel(int64_t n, const int32_t* src, const double*
 }
 
 cudaError_t pack_head(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
-                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, cudaStream_t s)
+                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, int* infinite,
+                      cudaStream_t s)
 {
     if (mixed)
         pack_head_kernel<<<(E + 7) / 8, 256, 0, s>>>(E, K, head_k, row_of, kptr, col, static_cast<const float*>(val), nnz,
-                                                     ptr, tiles);
+                                                     ptr, tiles, infinite);
     else
         pack_head_kernel<<<(E + 7) / 8, 256, 0, s>>>(E, K, head_k, row_of, kptr, col, static_cast<const double*>(val), nnz,
-                                                     ptr, tiles);
+                                                     ptr, tiles, infinite);
     return cudaGetLastError();
 }
 

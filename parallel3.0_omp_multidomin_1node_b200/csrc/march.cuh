@@ -204,8 +204,9 @@ cudaError_t build_history_runs(int E, int K, int kr, const std::vector<int64_t>&
 size_t history_runs_bytes(int64_t nb, bool mixed);
 
 // Group layout of the same blocks (MarchData hg_*): place[row] = group * 8 + slot
-// of every equation row.  Left empty (kr = 0) when the sizes exceed the sort's
-// indices or the blocks fill less than kGroupFillMin of the matrices.
+// of every equation row.  Left out (kr = 0) when the sizes exceed the sort's
+// indices, the blocks fill less than kGroupFillMin of the matrices, or a value is
+// not finite (a fragment also meets the zero vectors of steps not yet reached).
 struct HistoryGroups {
     int64_t* ptr = nullptr;   // [groups+1]
     uint2* meta = nullptr;    // [segments]
@@ -221,10 +222,13 @@ cudaError_t build_history_groups(int E, int K, int kr, const std::vector<int32_t
                                  const void* d_val, int64_t nnz, bool mixed, HistoryGroups& out, cudaStream_t s);
 size_t history_groups_bytes(int64_t nb, bool mixed);
 
-// Blocks of steps 1 .. head_k of each perm row to tiles (MarchData hd_*).
+// Blocks of steps 1 .. head_k of each perm row to tiles (MarchData hd_*); sets
+// *infinite when a value is not finite (the head multiplies blocks of steps not yet
+// reached by zero).
 constexpr size_t head_tile_bytes(bool mixed) { return 128 + 9 * 32 * (mixed ? 4 : 8); }
 cudaError_t pack_head(int E, int K, int head_k, const int32_t* row_of, const int64_t* kptr, const uint32_t* col,
-                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, cudaStream_t s);
+                      const void* val, bool mixed, int64_t nnz, const int32_t* ptr, unsigned char* tiles, int* infinite,
+                      cudaStream_t s);
 
 // Sizes of the R template instantiations.
 bool march_supported_loads(int R);

@@ -182,13 +182,14 @@ __global__ void group_steps_kernel(int n_segs, const unsigned long long* __restr
 
 // one warp per segment (in final order): header, then its blocks to their
 // places in the fragments (which start at zero): entry (3 slot + i, 3 (k - k0) +
-// j) of the segment's matrix
+// j) of the segment's matrix.  *infinite is set when a value is not finite.
 template <class V>
 __global__ void group_scatter_kernel(int n_segs, int64_t nb, int64_t nnz, const int* __restrict__ order,
                                      const int* __restrict__ start, const unsigned long long* __restrict__ okey,
                                      const int64_t* __restrict__ off, const unsigned long long* __restrict__ key,
                                      const uint32_t* __restrict__ idx, const V* __restrict__ val,
-                                     uint2* __restrict__ meta, int64_t* __restrict__ s_off, V* __restrict__ out)
+                                     uint2* __restrict__ meta, int64_t* __restrict__ s_off, V* __restrict__ out,
+                                     int* __restrict__ infinite)
 {
     const int i = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= n_segs) return;
@@ -208,7 +209,9 @@ __global__ void group_scatter_kernel(int n_segs, int64_t nb, int64_t nnz, const 
 #pragma unroll
         for (int c = 0; c < 9; ++c) {
             const int m = 3 * slot + c / 3, kk = 3 * step + c % 3;
-            out[((o + kk / 4) * 3 + m / 8) * 32 + (m % 8) * 4 + kk % 4] = val[c * nnz + src];
+            const V v = val[c * nnz + src];
+            out[((o + kk / 4) * 3 + m / 8) * 32 + (m % 8) * 4 + kk % 4] = v;
+            if (!isfinite(v)) *infinite = 1;
         }
     }
 }
@@ -517,20 +520,25 @@ cudaError_t build_history_groups(int E, int K, int kr, const std::vector<int32_t
     RUN_TRY(cudaMalloc(&out.val, val_bytes));
     RUN_TRY(cudaMemsetAsync(out.val, 0, val_bytes, s));
     const int gb = (int)(((int64_t)n_segs * 32 + 255) / 256);
+    int infinite = 0;
+    int* d_infinite = gcnt.as<int>();  // free again
+    RUN_TRY(cudaMemsetAsync(d_infinite, 0, sizeof(int), s));
     if (mixed)
         group_scatter_kernel<float><<<gb, 256, 0, s>>>(n_segs, nb, nnz, ov2.as<int>(), start.as<int>(),
                                                        okey2.as<unsigned long long>(), offs.as<int64_t>(),
                                                        k2.as<unsigned long long>(), i2.as<uint32_t>(),
                                                        static_cast<const float*>(d_val), out.meta, out.off,
-                                                       static_cast<float*>(out.val));
+                                                       static_cast<float*>(out.val), d_infinite);
     else
         group_scatter_kernel<double><<<gb, 256, 0, s>>>(n_segs, nb, nnz, ov2.as<int>(), start.as<int>(),
                                                         okey2.as<unsigned long long>(), offs.as<int64_t>(),
                                                         k2.as<unsigned long long>(), i2.as<uint32_t>(),
                                                         static_cast<const double*>(d_val), out.meta, out.off,
-                                                        static_cast<double*>(out.val));
+                                                        static_cast<double*>(out.val), d_infinite);
     RUN_TRY(cudaGetLastError());
+    RUN_TRY(cudaMemcpyAsync(&infinite, d_infinite, sizeof(int), cudaMemcpyDeviceToHost, s));
     RUN_TRY(cudaStreamSynchronize(s));
+    if (infinite) return cudaSuccess;
     out.steps = steps;
     out.segments = n_segs;
     out.kr = kr;

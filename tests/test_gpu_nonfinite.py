@@ -94,3 +94,24 @@ def test_infinite_history_vector(loads, K, nstep, precision):
                 assert np.max(np.abs(a - b)) <= mark * np.max(np.abs(b)), (r, q)
             else:
                 assert np.array_equal(np.isfinite(a), np.isfinite(b))
+
+
+@pytest.mark.parametrize("loads,precision,at,nstep,value,env", [
+    (1, "fp64", 2, 1, np.inf, {}),                                 # packed head of the one-step pass
+    (1, "mixed", 2, 1, 1e300, {}),                                 # infinite as FP32
+    (1, "fp64", 4, 3, np.nan, {"TDBEM_RUNS": "2"}),                # packed head of the two-step pass
+    (8, "fp64", 14, 13, np.inf, {}), (8, "mixed", 14, 13, 1e300, {}),  # fragments past the last sum's step
+])
+def test_block_that_is_not_finite(loads, precision, at, nstep, value, env):
+    c = _case(loads, nstep, 1e-12 if precision == "mixed" else 1e-13)
+    m = _matrices(c.n_elements, 14, 0.5)
+    ref = _march(c, loads, precision, m, **env)
+    assert ref[2].failed_step == 0 and ref[2].steps_solved == nstep
+    assert loads == 1 or ref[2].history_vector_loads < ref[2].history_block_steps / 2  # groups
+    for hist in m[2:]:
+        hist[at - 1][2][7::11] = value
+    got = _march(c, loads, precision, m, **env)
+    assert got[2].failed_step == 0 and got[2].steps_solved == nstep
+    mark = 1e-8 if precision == "mixed" else 1e-12
+    for q in range(2):
+        assert np.max(np.abs(got[q] - ref[q])) <= mark * np.max(np.abs(ref[q])), q
