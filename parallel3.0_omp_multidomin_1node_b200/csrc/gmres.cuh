@@ -739,7 +739,7 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
     double* Wa = d.wring + ((step - 1) % d.SW) * per_slot;
     double* Wb = d.wring + (step % d.SW) * per_slot;
     double worst[2] = {0.0, 0.0};  // displacement jump, traction balance
-    double zero = 0.0;             // not any more once a combined vector is not finite
+    double zero = 0.0;             // not any more once a combined vector is not finite (for the group pass)
 #pragma unroll 1
     for (int t = gtid; t < E * R; t += gstride) {
         const int i = t / R, r = t % R, rg = roff + r;
@@ -773,7 +773,7 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
                 X[p] = xs;
                 Wa[p] = wa;
                 Wb[p] = wb;
-                zero += 0.0 * wa + 0.0 * wb;
+                if (d.hg_n > 0) zero += 0.0 * wa + 0.0 * wb;
             }
         }
         if (e >= 0) {
@@ -1055,8 +1055,9 @@ __device__ __forceinline__ void gmres_body(const MarchData& d, const int step, c
         }
         __syncthreads();
         if (!s.any_run) break;
-        // V_1 = z / |z|
-        combine<R, MT>(kH, 0, 0, V(0), 0.0, s.run[tr] ? 1.0 / s.h1[tr] : 0.0, V(0), kLocal ? pv_off : -1);
+        // V_1 = z / |z|; zero for a case that does not run, whose z need not be finite
+        combine<R, MT>(kH, 0, 0, R == 1 || s.run[tr] ? V(0) : nullptr, 0.0, s.run[tr] ? 1.0 / s.h1[tr] : 0.0, V(0),
+                       kLocal ? pv_off : -1);
         int jn = 0;  // columns done
 #pragma unroll 1
         for (int j = 0; j < rs; ++j) {

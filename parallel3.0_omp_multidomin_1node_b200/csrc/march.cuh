@@ -133,7 +133,7 @@ struct MarchData {
     double* aw;       // [groups][3E][Rg]
     double* u;        // [groups][3E][Rg]
     double* givens;   // [groups][C][Rg] small arrays of gmres_givens_doubles(restart) each
-    int* status;      // [0] abort, [1] a combined history vector is not finite
+    int* status;      // [0] abort, [1] a combined history vector is not finite (with groups)
     // [nstep+4][5] device clock (ns): start of the step's head pass, start and end of
     // its GMRES, start and end of the history pass launch kept under it; or null
     unsigned long long* stamps;

@@ -115,3 +115,26 @@ def test_block_that_is_not_finite(loads, precision, at, nstep, value, env):
     mark = 1e-8 if precision == "mixed" else 1e-12
     for q in range(2):
         assert np.max(np.abs(got[q] - ref[q])) <= mark * np.max(np.abs(ref[q])), q
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("loads", [2, 4, 8, 32])
+def test_infinite_right_hand_side_beside_others(loads, precision):
+    """Load cases that share a GMRES cluster with one whose right-hand side is
+    infinite, against every case in its own cluster."""
+    nstep = 20
+    c = _case(loads, nstep, 1e-12 if precision == "mixed" else 1e-13)
+    lone = int(np.nonzero(c.bcid == 123)[0][0])
+    m = _matrices(c.n_elements, 11, 0.5, 6, lone)
+    c.known[1, 2, lone, 0] = 1.7e308
+    got = _march(c, loads, precision, m, TDBEM_GMRES_GROUPS="1", TDBEM_RUNS="0")
+    ref = _march(c, loads, precision, m, TDBEM_GMRES_GROUPS=str(loads), TDBEM_RUNS="0")
+    assert (got[2].gmres_groups, ref[2].gmres_groups) == (1, loads)
+    for out in (got, ref):
+        assert out[2].failed_step == 0 and out[2].steps_solved == nstep and np.isfinite(out[1]).all()
+    mark = 1e-8 if precision == "mixed" else 1e-12
+    for r in range(loads):
+        for q in range(2):
+            s = slice(None) if r != 1 else slice(0, 7)  # case 1: up to the infinite sums
+            a, b = got[q][r, s], ref[q][r, s]
+            assert np.max(np.abs(a - b)) <= mark * np.max(np.abs(b)), (r, q)
