@@ -2053,18 +2053,17 @@ tdbem_status tdbem_md_march_many(tdbem_handle* const* handles, int32_t n, const 
         cudaStream_t gs = h0->hp;
         std::vector<MarchData> ds((size_t)n);
         std::vector<int32_t> row_off((size_t)n + 1, 0);
-        size_t dsm = 0;
+        ModelForms forms{};
         int max_K = 0;
-        bool local = true;  // one form of the kernel for all models
-        for (int i = 0; i < n; ++i) local = local && runs[i].d.dsm_rows > 0;
         for (int i = 0; i < n; ++i) {
             ds[i] = runs[i].d;
-            if (!local) ds[i].dsm_rows = ds[i].halo_rows = 0;
             ds[i].k_lo = 1;
             ds[i].k_hi = 0;
             row_off[i + 1] = row_off[i] + runs[i].d.E;
-            dsm = std::max(dsm, gmres_dsm_bytes(ds[i].dsm_rows, ds[i].halo_rows, h0->R,
-                                                h0->precision == TDBEM_PRECISION_MIXED));
+            (ds[i].dsm_rows > 0 ? forms.local : forms.global) = true;
+            if (ds[i].dsm_rows > 0)
+                forms.dsm = std::max(forms.dsm, gmres_dsm_bytes(ds[i].dsm_rows, ds[i].halo_rows, h0->R,
+                                                                h0->precision == TDBEM_PRECISION_MIXED));
             max_K = std::max(max_K, runs[i].d.K);
         }
         DevBuf d_ds, d_off;
@@ -2077,9 +2076,12 @@ tdbem_status tdbem_md_march_many(tdbem_handle* const* handles, int32_t n, const 
         cudaStream_t bs = h0->side;
         const bool overlap = max_K >= 3;
         std::vector<cudaEvent_t> ev;
-        CUDA_TRY(h0->ev_order.take((size_t)n + 2 + 2 * ((size_t)steps + 2), ev));
+        CUDA_TRY(h0->ev_order.take((size_t)n + 4 + 2 * ((size_t)steps + 2), ev));
         cudaEvent_t* gm = &ev[(size_t)n + 1];
         cudaEvent_t* bk = gm + (steps + 2);
+        forms.fork = ev[ev.size() - 3];
+        forms.join = ev[ev.size() - 2];
+        forms.other = runs[1].s;  // its own set-up is behind ev[1]
         for (int i = 0; i < n; ++i) {
             CUDA_TRY(cudaEventRecord(ev[i], runs[i].s));
             CUDA_TRY(cudaStreamWaitEvent(gs, ev[i], 0));
@@ -2089,7 +2091,7 @@ tdbem_status tdbem_md_march_many(tdbem_handle* const* handles, int32_t n, const 
         tdbem_status st = TDBEM_OK;
         auto launch = [&](int step, int phase, cudaStream_t on) {
             const cudaError_t e = march_models_step(d_ds.as<MarchData>(), d_off.as<int32_t>(), n, row_off[n], h0->R,
-                                                    mixed, gC, dsm, local, max_K, step, phase, on);
+                                                    mixed, gC, forms, max_K, step, phase, on);
             if (e != cudaSuccess && st == TDBEM_OK)
                 st = fail(TDBEM_CUDA_ERROR, std::string("grouped march: ") + cudaGetErrorString(e));
         };

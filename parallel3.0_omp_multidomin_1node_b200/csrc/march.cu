@@ -1027,15 +1027,15 @@ __global__ void __launch_bounds__(kGmresThreads, 1) gmres_cluster_kernel(const _
     stamp_end(d, step, 2);
 }
 
-// Several models' GMRES of one step in one launch: cluster m solves model m
-// (one group of R load cases each; every model laid out for the launch's
-// cluster size); models whose march is shorter skip.
+// Several models' GMRES of one step in one launch per form: cluster m solves
+// model m (one group of R load cases each; every model laid out for the launch's
+// cluster size); models of the other form and models whose march is shorter skip.
 template <int R, bool kMixed, bool kLocal>
 __global__ void __launch_bounds__(kGmresThreads, 1) gmres_models_kernel(const MarchData* ds, int step)
 {
     __shared__ MarchData sd;
     load_model(ds, (int)(blockIdx.x / cg::this_cluster().num_blocks()), sd);
-    if (step > sd.nstep) return;
+    if (step > sd.nstep || (sd.dsm_rows > 0) != kLocal) return;
     gmres_body<R, kMixed, kLocal>(sd, step, 0);
 }
 
@@ -1484,25 +1484,13 @@ cudaError_t gather_tiles(int64_t tiles, const int32_t* src, const double* val9, 
 
 namespace {
 
-// One step of several models (one launch per phase): the right-hand sides of
-// every model, then one GMRES cluster of C CTAs per model.
-template <int R, bool kMixed>
-cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models, int total_rows, int cluster,
-                          size_t gmres_dsm, bool local, int max_K, int step, int phase, cudaStream_t s)
+template <int R, bool kMixed, bool kLocal>
+cudaError_t launch_gmres_models(const MarchData* ds, int n_models, int cluster, size_t gmres_dsm, int step,
+                                cudaStream_t s)
 {
-    constexpr int kC = R >= 4 ? 4 : R;
-    const size_t smem = sizeof(int) * (size_t)(max_K + 1);
-    if (phase == 2) {
-        rhs_models_kernel<R, kMixed, true, kC><<<total_rows, kRhsThreads, smem, s>>>(ds, row_off, n_models, step, 1);
-        return cudaGetLastError();
-    }
-    rhs_models_kernel<R, kMixed, false, kC><<<total_rows, kRhsThreads, smem, s>>>(ds, row_off, n_models, step, phase);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    static std::atomic<int> dyn_max[2][kMaxDevices];
+    static std::atomic<int> dyn_max[kMaxDevices];
     int cap = 0;
-    e = local ? kernel_attributes(gmres_models_kernel<R, kMixed, true>, dyn_max[1], cap)
-              : kernel_attributes(gmres_models_kernel<R, kMixed, false>, dyn_max[0], cap);
+    const cudaError_t e = kernel_attributes(gmres_models_kernel<R, kMixed, kLocal>, dyn_max, cap);
     if (e != cudaSuccess) return e;
     if (gmres_dsm > (size_t)cap) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
@@ -1517,22 +1505,53 @@ cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return local ? cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed, true>, ds, step)
-                 : cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed, false>, ds, step);
+    return cudaLaunchKernelEx(&cfg, gmres_models_kernel<R, kMixed, kLocal>, ds, step);
+}
+
+// One step of several models: the right-hand sides of every model in one launch,
+// then one GMRES cluster of C CTAs per model, the models of the two forms side by
+// side.
+template <int R, bool kMixed>
+cudaError_t models_step_r(const MarchData* ds, const int* row_off, int n_models, int total_rows, int cluster,
+                          const ModelForms& forms, int max_K, int step, int phase, cudaStream_t s)
+{
+    constexpr int kC = R >= 4 ? 4 : R;
+    const size_t smem = sizeof(int) * (size_t)(max_K + 1);
+    if (phase == 2) {
+        rhs_models_kernel<R, kMixed, true, kC><<<total_rows, kRhsThreads, smem, s>>>(ds, row_off, n_models, step, 1);
+        return cudaGetLastError();
+    }
+    rhs_models_kernel<R, kMixed, false, kC><<<total_rows, kRhsThreads, smem, s>>>(ds, row_off, n_models, step, phase);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const bool both = forms.local && forms.global;
+    cudaStream_t gs = both ? forms.other : s;
+    if (both && ((e = cudaEventRecord(forms.fork, s)) != cudaSuccess ||
+                 (e = cudaStreamWaitEvent(gs, forms.fork, 0)) != cudaSuccess))
+        return e;
+    if (forms.global)
+        if ((e = launch_gmres_models<R, kMixed, false>(ds, n_models, cluster, gmres_dsm_bytes(0, 0, R, kMixed), step,
+                                                       gs)) != cudaSuccess)
+            return e;
+    if (forms.local)
+        if ((e = launch_gmres_models<R, kMixed, true>(ds, n_models, cluster, forms.dsm, step, s)) != cudaSuccess)
+            return e;
+    if (both && (e = cudaEventRecord(forms.join, gs)) == cudaSuccess) e = cudaStreamWaitEvent(s, forms.join, 0);
+    return e;
 }
 
 }  // namespace
 
 cudaError_t march_models_step(const MarchData* ds, const int* row_off, int n_models, int total_rows, int R,
-                              bool mixed, int cluster, size_t gmres_dsm, bool local, int max_K, int step, int phase,
+                              bool mixed, int cluster, const ModelForms& forms, int max_K, int step, int phase,
                               cudaStream_t s)
 {
 #define TDBEM_MODELS_CASE(RR)                                                                                      \
     case RR:                                                                                                       \
-        return mixed ? models_step_r<RR, true>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, local, max_K,    \
-                                               step, phase, s)                                                     \
-                     : models_step_r<RR, false>(ds, row_off, n_models, total_rows, cluster, gmres_dsm, local, max_K,   \
-                                                step, phase, s);
+        return mixed ? models_step_r<RR, true>(ds, row_off, n_models, total_rows, cluster, forms, max_K, step,     \
+                                               phase, s)                                                           \
+                     : models_step_r<RR, false>(ds, row_off, n_models, total_rows, cluster, forms, max_K, step,    \
+                                                phase, s);
     switch (R) {
         TDBEM_MODELS_CASE(1)
         TDBEM_MODELS_CASE(2)

@@ -253,18 +253,26 @@ struct StepEvents {
 cudaError_t march_step(const MarchData& d, int step, cudaStream_t s, cudaStream_t side, const StepEvents& ev,
                        bool overlap);
 int gmres_cluster_size(int device, int R, bool mixed);
+// The forms of GMRES that several models take: vectors in shared memory
+// (MarchData::dsm_rows > 0; dsm: the largest dynamic shared memory one needs) or in
+// global memory.  With both, the second form's launch goes to `other` between the
+// events.
+struct ModelForms {
+    bool local, global;
+    size_t dsm;
+    cudaStream_t other;
+    cudaEvent_t fork, join;
+};
 // Launches of one time step of several models of R load cases each (R in 1,
 // 2, 4, 8).  phase 0: every model's right-hand side over all history steps,
-// then one GMRES cluster of `cluster` CTAs per model; phase 1: the same with
+// then one GMRES cluster of `cluster` CTAs per model (a launch per form); phase 1: the same with
 // the head right-hand side (KnownM, k <= 2, plus the bulk computed ahead);
 // phase 2: only the bulk (history steps k >= 3) of `step` into the models'
 // bulk buffers.  ds: device array of the models' MarchData (each laid out for
 // `cluster`); row_off: [n_models + 1] prefix sums of their element counts;
-// gmres_dsm: the largest dynamic shared memory any model's GMRES needs; local:
-// every model's vectors are in shared memory (dsm_rows > 0), else none's are;
-// max_K: the largest history length.
+// forms: which forms of GMRES the models take; max_K: the largest history length.
 cudaError_t march_models_step(const MarchData* ds, const int* row_off, int n_models, int total_rows, int R,
-                              bool mixed, int cluster, size_t gmres_dsm, bool local, int max_K, int step, int phase,
+                              bool mixed, int cluster, const ModelForms& forms, int max_K, int step, int phase,
                               cudaStream_t s);
 // The FP64 single-load GMRES step kernel on caller-supplied storage: d.R = 1,
 // d.groups = 1, d.nstep = 1, step 1.  Every pointer it writes (b, x, rv,
