@@ -348,7 +348,11 @@ void tree_split(const std::vector<double>& node, const Cube& cb, std::vector<int
 // ---------------------------------------------------------------------------
 // A matrix in the tile form the GMRES clusters read, on the device.
 struct GmresTiles {
-    DevBuf cta_row, cs, sp, srows, halo, send_ptr, send, col, colg, val, val32;
+    DevBuf tables, val, val32;  // the index tables in one buffer: a handle's set-up is mostly allocations
+    enum { kCtaRow, kCs, kSp, kRows, kHalo, kSendPtr, kSend, kCol, kColg, kSrc, kTables };
+    size_t at[kTables] = {};    // first word of each
+    template <class T>
+    const T* table(int t) const { return reinterpret_cast<const T*>(tables.as<int32_t>() + at[t]); }
     int own_rows = 0, halo_rows = 0, leaf_max = 0;  // leaf_max: values of the largest CTA's leaf inverses
     // tiles of the matrix rp, col (host) with row-major blocks d_val9 (device)
     cudaError_t build(const std::vector<int32_t>& rows, int64_t leaf_values, const std::vector<int32_t>& rp,
@@ -359,15 +363,15 @@ struct GmresTiles {
     // less: the last CTA gives up its first wait, and the exponent is the magnitude).
     void fill(MarchData& d, int Rg, bool mixed) const
     {
-        d.cta_row = cta_row.as<int32_t>();
-        d.g_cs = cs.as<int32_t>();
-        d.g_sp = sp.as<int2>();
-        d.g_rows = srows.as<int32_t>();
-        d.g_halo = halo.as<int32_t>();
-        d.g_send_ptr = send_ptr.as<int32_t>();
-        d.g_send = send.as<int2>();
-        d.g_col = col.as<int32_t>();
-        d.g_colg = colg.as<int32_t>();
+        d.cta_row = table<int32_t>(kCtaRow);
+        d.g_cs = table<int32_t>(kCs);
+        d.g_sp = table<int2>(kSp);
+        d.g_rows = table<int32_t>(kRows);
+        d.g_halo = table<int32_t>(kHalo);
+        d.g_send_ptr = table<int32_t>(kSendPtr);
+        d.g_send = table<int2>(kSend);
+        d.g_col = table<int32_t>(kCol);
+        d.g_colg = table<int32_t>(kColg);
         d.g_val = val.as<double>();
         d.g_val32 = val32.as<float>();
         const int cap = gmres_row_capacity(own_rows);
@@ -486,7 +490,8 @@ struct tdbem_handle {
     DevBuf d_k_rp, d_k_col, d_k_val, d_k_elem, d_k_sgn;
     DevBuf d_a_rp, d_a_col, d_a_val, d_row_of, d_unk_of, d_perm_of_unk;
     DevBuf d_leaf_begin, d_leaf_count, d_leaf_off, d_row_leaf;
-    DevBuf d_pmat, d_pmat_c, d_pinv, d_pinv_c, d_pinv32, d_minv;  // leaf blocks and inverses (LeafBlocks)
+    DevBuf d_leaf, d_pinv32;  // leaf blocks and inverses
+    LeafBlocks leaf{};        // (in d_leaf)
     GmresTiles tiles;                                             // A' for the GMRES clusters
     DevBuf d_xring, d_wring, d_bulk, d_b, d_x, d_rv, d_aw, d_u, d_V, d_givens, d_status, d_flags, d_audit, d_stamps;
     DevBuf d_known, d_out_lu, d_out_lt, d_rec_rhs, d_rec_x, d_xold;
@@ -1227,23 +1232,29 @@ cudaError_t GmresTiles::build(const std::vector<int32_t>& rows, int64_t leaf_val
     for (size_t c = 0; c + 1 < rows.size(); ++c) own_rows = std::max(own_rows, rows[c + 1] - rows[c]);
     gmres_tile_index(rows, gmres_row_capacity(own_rows), rp, mcol, ix);
     halo_rows = ix.halo_max;
-    DevBuf src;
-    cudaError_t e = up(cta_row, rows, s);
-    if (e == cudaSuccess) e = up(cs, ix.cs, s);
-    if (e == cudaSuccess) e = up(sp, ix.sp, s);
-    if (e == cudaSuccess) e = up(srows, ix.rows, s);
-    if (e == cudaSuccess) e = up(halo, ix.halo, s);
-    if (e == cudaSuccess) e = up(send_ptr, ix.send_ptr, s);
-    if (e == cudaSuccess) e = up(send, ix.send, s);
-    if (e == cudaSuccess) e = up(col, ix.col, s);
-    if (e == cudaSuccess) e = up(colg, ix.colg, s);
-    if (e == cudaSuccess) e = up(src, ix.src, s);
+    std::vector<int32_t> words;
+    auto put = [&](int t, const auto& v) {
+        at[t] = (words.size() + 3) / 4 * 4;  // 16-byte aligned
+        words.resize(at[t] + v.size() * (sizeof(v[0]) / sizeof(int32_t)));
+        if (!v.empty()) std::memcpy(words.data() + at[t], v.data(), v.size() * sizeof(v[0]));
+    };
+    put(kCtaRow, rows);
+    put(kCs, ix.cs);
+    put(kSp, ix.sp);
+    put(kRows, ix.rows);
+    put(kHalo, ix.halo);
+    put(kSendPtr, ix.send_ptr);
+    put(kSend, ix.send);
+    put(kCol, ix.col);
+    put(kColg, ix.colg);
+    put(kSrc, ix.src);
+    cudaError_t e = up(tables, words, s);
     const int64_t tiles = (int64_t)(ix.col.size() / 32);
     if (e == cudaSuccess) e = val.alloc(sizeof(double) * 288 * (size_t)std::max<int64_t>(tiles, 1));
     if (e == cudaSuccess && mixed) e = val32.alloc(sizeof(float) * 288 * (size_t)std::max<int64_t>(tiles, 1));
     if (e == cudaSuccess)
-        e = gather_tiles(tiles, src.as<int32_t>(), d_val9, val.as<double>(), mixed ? val32.as<float>() : nullptr, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // src is freed here
+        e = gather_tiles(tiles, table<int32_t>(kSrc), d_val9, val.as<double>(), mixed ? val32.as<float>() : nullptr, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // words is freed here
     return e;
 }
 
@@ -1379,10 +1390,11 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
         for (int q = 0; q < lc[l]; ++q) lop[lb[l] + q] = RowLeaf{loff[l], lb[l], 3 * lc[l]};
     CUDA_TRY(up(h->d_row_leaf, lop, s));
     CUDA_TRY(up(h->d_leaf_off, loff, s));
-    for (DevBuf* b : {&h->d_pmat, &h->d_pmat_c, &h->d_pinv, &h->d_pinv_c})
-        CUDA_TRY(b->alloc(sizeof(double) * std::max<int64_t>(loff[nl], 1)));
-    CUDA_TRY(h->d_minv.alloc(sizeof(double)));
-    CUDA_TRY(cudaMemsetAsync(h->d_minv.p, 0, sizeof(double), s));
+    const int64_t lv = loff[nl];
+    CUDA_TRY(h->d_leaf.alloc(sizeof(double) * (4 * lv + 1)));
+    double* lp = h->d_leaf.as<double>();
+    h->leaf = LeafBlocks{lp, lp + lv, lp + 2 * lv, lp + 3 * lv, lp + 4 * lv};
+    CUDA_TRY(cudaMemsetAsync(h->leaf.norm, 0, sizeof(double), s));
     DevBuf sing;
     CUDA_TRY(sing.alloc(sizeof(int)));
     CUDA_TRY(cudaMemsetAsync(sing.p, 0, sizeof(int), s));
@@ -1392,10 +1404,7 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
     leaf_inverse_kernel<<<nl, 256, smem, s>>>(nl, h->d_leaf_begin.as<int32_t>(), h->d_leaf_count.as<int32_t>(),
                                              h->d_leaf_off.as<int64_t>(), h->d_a_rp.as<int32_t>(),
                                              h->d_a_col.as<int32_t>(), h->d_a_val.as<double>(),
-                                             LeafBlocks{h->d_pmat.as<double>(), h->d_pmat_c.as<double>(),
-                                                        h->d_pinv.as<double>(), h->d_pinv_c.as<double>(),
-                                                        h->d_minv.as<double>()},
-                                             sing.as<int>());
+                                             h->leaf, sing.as<int>());
     CUDA_TRY(cudaGetLastError());
     int singular = 0;
     CUDA_TRY(cudaMemcpyAsync(&singular, sing.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1405,7 +1414,7 @@ tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
                                               " has a pivot <= 1e-10");
     if (h->precision == TDBEM_PRECISION_MIXED) {
         CUDA_TRY(h->d_pinv32.alloc(sizeof(float) * std::max<int64_t>(loff[nl], 1)));
-        to_float_kernel<<<148, 256, 0, s>>>(h->d_pinv_c.as<double>(), h->d_pinv32.as<float>(), loff[nl]);
+        to_float_kernel<<<148, 256, 0, s>>>(h->leaf.inv_c, h->d_pinv32.as<float>(), loff[nl]);
         CUDA_TRY(cudaGetLastError());
     }
     // GMRES: `groups` clusters of C CTAs, each solving R / groups load cases;
@@ -1588,10 +1597,10 @@ struct MarchRun {
         d.row_of = h->d_row_of.as<int32_t>();
         d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
         d.row_leaf = h->d_row_leaf.as<RowLeaf>();
-        d.pinv = h->d_pinv_c.as<double>();
+        d.pinv = h->leaf.inv_c;
         d.pinv32 = h->d_pinv32.as<float>();
-        d.pmat = h->d_pmat_c.as<double>();
-        d.minv = h->d_minv.as<double>();
+        d.pmat = h->leaf.mat_c;
+        d.minv = h->leaf.norm;
         d.uref_block = h->d_uref_block.as<int64_t>();
         d.uref_sign = h->d_uref_sign.as<double>();
         d.uref_known = h->d_uref_known.as<int32_t>();
@@ -2518,9 +2527,9 @@ tdbem_status tdbem_md_solve_noalloc(tdbem_handle* h, const double* d_rhs, double
     d.row_of = h->d_row_of.as<int32_t>();
     d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
     d.row_leaf = h->d_row_leaf.as<RowLeaf>();
-    d.pinv = h->d_pinv_c.as<double>();
-    d.pmat = h->d_pmat_c.as<double>();
-    d.minv = h->d_minv.as<double>();
+    d.pinv = h->leaf.inv_c;
+    d.pmat = h->leaf.mat_c;
+    d.minv = h->leaf.norm;
     d.status = reinterpret_cast<int*>(base + L.head);
     d.step_flags = reinterpret_cast<int*>(base + L.head + 16);
     d.solve_only = 1;
@@ -3182,9 +3191,9 @@ tdbem_status tdbem_md_march_vjp(tdbem_handle* h, const double* cot_lu, const dou
     }
     A.tiles.fill(d, 1, false);
     // the transposed leaf blocks by columns are the row-major blocks
-    d.pinv = h->d_pinv.as<double>();
-    d.pmat = h->d_pmat.as<double>();
-    d.minv = h->d_minv.as<double>();
+    d.pinv = h->leaf.inv;
+    d.pmat = h->leaf.mat;
+    d.minv = h->leaf.norm;
     d.row_of = h->d_row_of.as<int32_t>();
     d.perm_of_unk = h->d_perm_of_unk.as<int32_t>();
     d.row_leaf = h->d_row_leaf.as<RowLeaf>();
