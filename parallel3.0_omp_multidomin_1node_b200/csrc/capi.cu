@@ -1349,6 +1349,7 @@ tdbem_status build_head(tdbem_handle* h, cudaStream_t s)
 tdbem_status finish_setup(tdbem_handle* h, cudaStream_t s)
 {
     const int64_t E = h->E;
+    h->adjoint.reset();  // transposed operators of the matrices before
     std::vector<int32_t> row_of(E), unk_of(E), perm_of_unk(E);
     for (int64_t p = 0; p < E; ++p) {
         row_of[p] = (int32_t)h->repid[p];
