@@ -1898,6 +1898,7 @@ tdbem_status tdbem_md_assemble(tdbem_handle* h, void* stream)
     }
     blocks.release();
     flags.release();
+    h->assembled = false;  // until the set-up is complete
     tdbem_status st = assemble_history(h, P, std::min(maxn, kHistoryStepsMax), s);
     if (st != TDBEM_OK) return st;
     if ((st = build_runs(h, s)) != TDBEM_OK) return st;
@@ -1918,17 +1919,10 @@ tdbem_status tdbem_md_load_matrices(tdbem_handle* h, const int32_t* a_rowptr, co
     CUDA_TRY(cudaSetDevice(h->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : h->s0;
     const int E = (int)h->E;
-    h->a_rp.assign(a_rowptr, a_rowptr + E + 1);
-    h->a_col.assign(a_col, a_col + h->a_rp[E]);
-    h->a_val.assign(a_val, a_val + 9 * (int64_t)h->a_rp[E]);
-    h->k_rp.assign(k_rowptr, k_rowptr + E + 1);
-    h->k_col.assign(k_col, k_col + h->k_rp[E]);
-    h->k_val.assign(k_val, k_val + 9 * (int64_t)h->k_rp[E]);
-    for (int64_t j = 0; j < h->a_rp[E]; ++j)
-        if (h->a_col[j] < 0 || h->a_col[j] >= h->n_unknown) return fail(TDBEM_INVALID_INPUT, "A column out of range");
-    for (int64_t j = 0; j < h->k_rp[E]; ++j)
-        if (h->k_col[j] < 0 || h->k_col[j] >= h->n_known) return fail(TDBEM_INVALID_INPUT, "KnownM column out of range");
-    h->K = n_hist;
+    for (int64_t j = 0; j < a_rowptr[E]; ++j)
+        if (a_col[j] < 0 || a_col[j] >= h->n_unknown) return fail(TDBEM_INVALID_INPUT, "A column out of range");
+    for (int64_t j = 0; j < k_rowptr[E]; ++j)
+        if (k_col[j] < 0 || k_col[j] >= h->n_known) return fail(TDBEM_INVALID_INPUT, "KnownM column out of range");
     std::vector<std::vector<int64_t>> mts_rp(n_hist), mgs_rp(n_hist);
     std::vector<HistK> hk(n_hist);
     std::vector<std::unique_ptr<DevBuf>> keep;
@@ -1959,6 +1953,14 @@ tdbem_status tdbem_md_load_matrices(tdbem_handle* h, const int32_t* a_rowptr, co
         ot += nt;
         og += ng;
     }
+    h->assembled = false;  // until the set-up is complete
+    h->a_rp.assign(a_rowptr, a_rowptr + E + 1);
+    h->a_col.assign(a_col, a_col + h->a_rp[E]);
+    h->a_val.assign(a_val, a_val + 9 * (int64_t)h->a_rp[E]);
+    h->k_rp.assign(k_rowptr, k_rowptr + E + 1);
+    h->k_col.assign(k_col, k_col + h->k_rp[E]);
+    h->k_val.assign(k_val, k_val + 9 * (int64_t)h->k_rp[E]);
+    h->K = n_hist;
     tdbem_status st = stack_history(h, mts_rp, mgs_rp, hk, s);
     if (st != TDBEM_OK) return st;
     keep.clear();  // the per-step matrices, before the run layout takes its memory

@@ -36,3 +36,29 @@ def test_adjoint_follows_the_matrices():
         out.append((lu, lt, g))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_failed_load():
+    """A load refused for its input leaves the handle with the matrices it had; one
+    that fails later leaves it without any, until the next one succeeds."""
+    from tdbem.api import MultiDomainSolver, TdbemError
+    c = _case(8, NSTEP)
+    good, other = _seeded(c.n_elements, 5, 1), _seeded(c.n_elements, 9, 2)
+    s = MultiDomainSolver(c, n_loads=8)
+    s.load_matrices(*good)
+    ref = s.march(c.known)[:2]
+    bad = [*other[:2], [(r, np.where(k == 8, j + c.n_elements * 2, j), v) for k, (r, j, v) in enumerate(other[2])],
+           other[3]]
+    with pytest.raises(TdbemError, match="MTS column out of range"):
+        s.load_matrices(*bad)
+    for a, b in zip(s.march(c.known)[:2], ref):
+        assert np.array_equal(a, b)
+    singular = [(other[0][0], other[0][1], 0.0 * other[0][2]), *other[1:]]
+    with pytest.raises(TdbemError, match="SINGULAR_BLOCK"):
+        s.load_matrices(*singular)
+    with pytest.raises(TdbemError, match="NOT_ASSEMBLED"):
+        s.march(c.known)
+    s.load_matrices(*good)
+    for a, b in zip(s.march(c.known)[:2], ref):
+        assert np.array_equal(a, b)
+    s.close()
