@@ -450,8 +450,10 @@ def ours_arm(args):
                                                "peak, not a measured copy)",
                                   "bytes_per_launch": l2_bytes / launches_hist},
                      "fp64_tflops": fp64_tflops,
-                     "limiter": "L2 gather of the FP64 history vectors (3 x R values per load) and FP64 issue; "
-                                "the HBM fraction is low by construction at 32 load cases"},
+                     "limiter": ("FP64 tensor pipe (m8n8k4), part of it zero padding of the groups of rows; "
+                                 "the HBM fraction is low by construction at 32 load cases" if R >= 8 else
+                                 "L2 gather of the FP64 history vectors (3 x R values per load) and FP64 issue"
+                                 if R > 1 else "HBM reads of the blocks")},
         "e2e": {"value": world * args.steps * N * R / (ms_e2e / 1e3), "unit": "timesteps/s",
                 "h2d_bytes_per_step": int(kh.numel() * 8), "d2h_bytes_per_step": int(2 * kh.numel() * 8)},
         "gpu_launches": args.steps * (2 * N + 1 + launches_hist),

@@ -341,10 +341,11 @@ void tdbem_case_destroy(tdbem_case* c);
  *        once the work is enqueued, and a solve that does not converge is
  *        not reported (x then holds GMRES's last iterate): a caller that
  *        cannot wait must check the solution itself.
- * Limit: the solve needs 8 * ((15 + 9 * (restart + 1)) * E
- * + 5 * C * (restart + 2) + 32) bytes plus alignment (C = the handle's GMRES
- * cluster size), about 14,000 elements at restart 30.  Larger problems are
- * rejected with TDBEM_INVALID_INPUT and a message giving the bytes needed.
+ * Limit: the array's size, for which a system counts
+ * 8 * ((15 + 9 * (restart + 1)) * E + 5 * C * (restart + 2) + 32) bytes plus
+ * alignment (C = the handle's GMRES cluster size; the solve uses less), about
+ * 14,000 elements at restart 30.  Larger problems are rejected with
+ * TDBEM_INVALID_INPUT and a message giving that count.
  * The first call on each device sets up, with that device current, the
  * array's address and the cluster size the kernel can be scheduled with;
  * make that first call before any stream capture begins.  One array serves

@@ -525,7 +525,9 @@ size_t pair_smem(bool dual)
 // (type 1 = MGS) of the blocks kept.  A CTA takes a field element, its warps the
 // sources; only those of rows [r0, r1).  Slots run by rows, from slot0 here; no
 // values are kept without blocks, no counts without counts.  The 2,058-element
-// bar (36 steps): 707 ms -> 27.7 ms.
+// bar (36 steps): 707 ms -> 27.7 ms.  Two CTAs an SM leave 128 registers, too few
+// for the 24 sums beside the factors: 380 bytes of spill stores, 440 of loads (step0
+// 1,008 and 1,168); issue slots 50% busy on the 1,728-element bar.
 __global__ void __launch_bounds__(32 * kPairWarps, 2) history_pairs_kernel(PairSpace ps, const QuadRules* rules,
                                                                           const DynaMat* mats, ElemGeom g, DofRefs dr,
                                                                           const uint32_t* range, const int64_t* slot,
@@ -1038,7 +1040,8 @@ __global__ void __launch_bounds__(32 * kPairWarps) grad_step0_kernel(PairSpace p
 // (traction kernel) and MGS_k (displacement kernel) blocks add
 // lam_n^T (-dMTS_k W0 + dMGS_k W1) with the convolution vector the march
 // used at step n >= 2, W_m = [m+1 < n] X_{m+1} + 2 X_m + X_{m-1},
-// m = n - k (X_0 = X_-1 = 0).  480 elements, 200 steps: about 92 ms with the
+// m = n - k (X_0 = X_-1 = 0).  Dual numbers take all 255 registers and spill (152
+// bytes of stores, grad_step0_kernel 1,008).  480 elements, 200 steps: about 92 ms with the
 // blocks computed step by step, 10.3 ms.
 __global__ void __launch_bounds__(32 * kPairWarps) grad_history_kernel(PairSpace ps, const QuadRules* rules,
                                                                        const DynaMatD* mats, ElemGeom g, DofRefs dr,

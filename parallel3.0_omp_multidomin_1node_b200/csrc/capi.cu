@@ -2400,12 +2400,14 @@ tdbem_status tdbem_md_precond_layout(tdbem_handle* h, int64_t* repid, int64_t* l
 // and (optionally) a copy of three flags.
 namespace {
 
-// Capacity of the static scratch, and what a solve is charged for, in doubles:
+// Capacity of the static scratch.  The limit of a solve is stated in what it
+// counts for, in doubles:
 //   (15 + 9 (restart + 1)) E + 5 C (restart + 2) + 32
 // plus 256-byte alignment of each region (C = GMRES cluster CTAs): at
-// restart 30 about 2.35 KB per element, so roughly 14,000 elements.  The
-// solve uses less: its basis, 3 (restart + 1) E, and at most 16 x 115,921
-// doubles of small arrays (restart 480), which fit whenever the charge does.
+// restart 30 about 2.35 KB per element, so roughly 14,000 elements.  It is the
+// storage of a solver with three bases and stays the interface's limit.  The solve
+// uses less: five vectors, its basis, 3 (restart + 1) E, and at most 16 x 118,331
+// doubles of small arrays (restart 480), which fit whenever the count does.
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -2511,10 +2513,10 @@ tdbem_status tdbem_md_solve_noalloc(tdbem_handle* h, const double* d_rhs, double
                                              " the single-load solver can be scheduled with");
     const NoAllocLayout L = noalloc_layout(E, rs, C);
     if (std::max(L.charge, L.used) > kNoAllocScratchBytes)
-        return fail(TDBEM_INVALID_INPUT, "tdbem_md_solve_noalloc needs " + std::to_string(std::max(L.charge, L.used)) +
-                                             " bytes of scratch for " + std::to_string(E) +
-                                             " elements at restart " + std::to_string(rs) +
-                                             "; its static scratch holds " +
+        return fail(TDBEM_INVALID_INPUT, "tdbem_md_solve_noalloc: " + std::to_string(E) + " elements at restart " +
+                                             std::to_string(rs) + " count for " +
+                                             std::to_string(std::max(L.charge, L.used)) +
+                                             " bytes; the limit, the size of its static scratch, is " +
                                              std::to_string(kNoAllocScratchBytes) + " bytes");
     cudaStream_t s = stream ? (cudaStream_t)stream : h->s0;
     unsigned char* base = nd->scratch;

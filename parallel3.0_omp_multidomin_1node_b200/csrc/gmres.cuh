@@ -10,6 +10,8 @@
 //   asynchronous remote stores that complete on the receiver's mbarrier (about
 //   550 cycles), partial sums to every peer and basis vector values to the
 //   CTAs whose rows use them, which then read only their own shared memory.
+//   (Rows that do not fit shared memory: vectors in global memory, and a remote
+//   arrival per peer instead of the values.)
 // - A step runs straight through the code once, so its instructions have to
 //   stay in the instruction cache: with every product, leaf application and
 //   reduction inlined the kernel was 180 KB and each phase waited for its
@@ -814,8 +816,8 @@ __device__ __noinline__ void write_back(const MarchData& d, int step, int roff, 
 // The residual of each step comes without forming x: with z_j the
 // preconditioned residual, z_j = V t with t built from the rotations, and
 // r_j = M z_j with M the leaf blocks.  |r_j| >= |z_j| / |M^-1|, |z_j| =
-// |phibar|, so steps whose phibar is above 2 |M^-1| tol |b| cannot have
-// converged and skip it.  x = x0 + V y is formed once, when the residual meets
+// |phibar|, so steps whose phibar is above 1.01 |M^-1| tol |b| cannot have
+// converged and skip it (the hundredth is for rounding).  x = x0 + V y is formed once, when the residual meets
 // the tolerance.  (Carrying W_j = V_j R^-1 and A W_j through every step, as
 // the reference's recurrence does, read and wrote 4 j + 6 vectors per step.)
 template <int R, bool kMixed, bool kLocal>

@@ -5,19 +5,29 @@
 //                       history block is read from HBM once and applied to
 //                       all R combined history vectors (block SpMM),
 //                       DBEM1/multidomain.cpp:3843-3866; the head pass on
-//                       the GMRES chain and the one-step pass beside it
+//                       the GMRES chain for two or more load cases and the
+//                       one-step pass beside it
+//   head_rows_kernel    the head pass of one load case over packed blocks
 //   bulk_steps_kernel   the history steps k >= 2T + 1 of T time steps in
-//                       one pass over the run layout (two or more load
-//                       cases): each block read once for the T steps, each
-//                       history vector of a run once, kept in registers
+//                       one pass over the run layout (two or four load
+//                       cases, or rows that share too little): each block
+//                       read once for the T steps, each history vector of a
+//                       run once, kept in registers
+//   bulk_rows_kernel    the same for one load case over the step-major
+//                       matrices
+//   bulk_groups_kernel  the same for 8 or more load cases over groups of 8
+//                       rows, on the FP64 tensor path
+//   adj_history_kernel  the transposed history convolution of the adjoint
+//                       march
 //   gmres_cluster_kernel left-preconditioned GMRES(restart) for the R load
-//                       cases in lockstep on one thread-block cluster:
-//                       hardware cluster barriers, reductions through
-//                       distributed shared memory, one SpMM of A' per
-//                       Arnoldi step shared by all cases,
-//                       DBEM1/pre_gmres.cpp:1369-1605; then the boundary
-//                       write-back and history-state update,
-//                       DBEM1/multidomain.cpp:3086-3225
+//                       cases in lockstep on one thread-block cluster
+//                       (gmres.cuh): asynchronous remote stores completing
+//                       on mbarriers, one SpMM of A' per Arnoldi step
+//                       shared by all cases, DBEM1/pre_gmres.cpp:1369-1605;
+//                       then the boundary write-back and history-state
+//                       update, DBEM1/multidomain.cpp:3086-3225
+//   rhs_models_kernel, gmres_models_kernel  the same for several models per
+//                       launch
 #include "march.cuh"
 
 #include <algorithm>
@@ -1199,12 +1209,7 @@ cudaError_t launch_rhs(const MarchData& d, int step, bool bulk, int add_bulk, cu
     }
 }
 
-// T-step history pass (T = (kr - 1) / 2, 2 or 3): two load cases per thread
-// (the registers hold the T steps' sums and the window of T history
-// vectors); one load case reads the step-major matrices.  Measured against the two-step form on the 32-load
-// bar and kept out: staging the history vectors and block values through
-// shared memory with cp.async (72% more instructions, 1.5x slower) and L1
-// prefetches of the coming vectors (slower at every distance tried).
+// Group form of the T-step history pass: a cluster of hg_split CTAs per group.
 template <int R, int T, class V>
 cudaError_t launch_bulk_groups(const MarchData& d, int t0, cudaStream_t s)
 {
@@ -1228,6 +1233,14 @@ cudaError_t launch_bulk_groups(const MarchData& d, int t0, cudaStream_t s)
     return cudaLaunchKernelEx(&cfg, bulk_groups_kernel<R, T, V>, d, t0, d.hg_split);
 }
 
+// T-step history pass (T = (kr - 1) / 2, 2 or 3): groups where there are any, the
+// step-major matrices for one load case, else the run layout with two load cases
+// per thread (the registers hold the T steps' sums and the window of T history
+// vectors).  Measured against the run form and kept out of it: staging its history
+// vectors and block values through shared memory with cp.async (72% more
+// instructions, 1.5x slower; what pays for the staging in the group form is that
+// eight rows use a vector) and L1 prefetches of the coming vectors (slower at every
+// distance tried).
 template <int R, bool kMixed>
 cudaError_t launch_bulk_steps(const MarchData& d, int t0, int part, cudaStream_t s)
 {
